@@ -115,7 +115,7 @@ enum Scalar : int {
   kSegGridOn = 18,     // 1 when connection tests read segments from the segment grid
   kSegBig = 19,        // contour segments too large for the grid's cells
   kHeavyPolygons = 20, // polygons queued for warp-wide noding
-  kFrontierNext = 8,   // next frontier patch a subdivision warp takes
+  kFrontierNext = 8,   // next frontier patch a subdivision warp takes (or piece a clipping warp)
   // Iterative clipping (DevicePeeler): live pieces of this round, pieces
   // appended for the next round, hidden pieces of this layer, the current
   // work pool, and the clipping-round loop's condition.
@@ -155,7 +155,7 @@ struct Dev {
   unsigned long long *pred_counts;
   // Tuning knobs (edp_tuning): subdivision walk steps per patch and round,
   // subdivision blocks per SM, candidate x edge tests above which a polygon
-  // is noded by a warp, clipping candidate tests per piece and round.  None
+  // is noded by a warp, clipping walk steps per piece and round.  None
   // changes a result, only how the work is spread.
   int step_budget, subdivide_blocks, heavy_noding_work, clip_budget;
   Caps cap;

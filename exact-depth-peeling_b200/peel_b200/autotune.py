@@ -9,7 +9,7 @@ rounds, blocks and warps, never which regions or triangles come out:
   width of the persistent subdivision grid);
 * ``heavy_noding_work``: candidate x edge tests above which a polygon is
   noded by a warp instead of one thread;
-* ``clip_budget``: DevicePeeler candidate tests per piece and clipping round.
+* ``clip_budget``: DevicePeeler hierarchy walk steps per piece and clipping round.
 
 ``tune`` runs a coordinate search: starting from the defaults, each knob in
 turn takes each of its values with the others fixed, and the value with the
