@@ -344,7 +344,8 @@ __device__ inline int cut_piece(const Dev &d, const PiecePool &queue, const Piec
                                 int source, int target, int cursor,
                                 bool tested, V2 *left, V2 *right, V2 *held, int *held_n,
                                 Tally &t) {
-  const int lane = threadIdx.x & 31;
+  const Group<32> g;
+  const int lane = g.lane;
   if (!tested && warp_separated<F>(p, q, n, c, t)) return kKept;
   const bool mine = lane < n;
   const Plane so = d.scores[c.source];
@@ -367,7 +368,7 @@ __device__ inline int cut_piece(const Dev &d, const PiecePool &queue, const Piec
   if (!positive) return kKept;
   V2 behind = p, nearer = p;
   int behind_n = n, nearer_n = 0;
-  if (negative && !warp_split<F>(p, q, n, behind_by, sign, left, right, behind, behind_n, nearer,
+  if (negative && !group_split<F>(g, p, q, n, behind_by, sign, left, right, behind, behind_n, nearer,
                                  nearer_n)) {
     if (lane == 0) set_error(d.status, kErrPolygon);
     return kFailed;
@@ -397,10 +398,10 @@ __device__ inline int cut_piece(const Dev &d, const PiecePool &queue, const Piec
         if (lane < in_n) t.add(stage);
       // Nothing lies outside this edge: the part is inside as it is.
       if (!__ballot_sync(kFull, lane < in_n && s < 0)) continue;
-      const V2 in_next = shfl(in, lane + 1 < in_n ? lane + 1 : 0);
+      const V2 in_next = g.shfl(in, lane + 1 < in_n ? lane + 1 : 0);
       V2 inside, out;
       int inside_n, out_n;
-      if (!warp_split<F>(in, in_next, in_n, off, s, left, right, inside, inside_n, out, out_n)) {
+      if (!group_split<F>(g, in, in_next, in_n, off, s, left, right, inside, inside_n, out, out_n)) {
         if (lane == 0) set_error(d.status, kErrPolygon);
         return kFailed;
       }
@@ -435,7 +436,7 @@ __device__ inline int cut_piece(const Dev &d, const PiecePool &queue, const Piec
   }
   p = keep;
   n = keep_n;
-  q = shfl(p, lane + 1 < n ? lane + 1 : 0);
+  q = g.shfl(p, lane + 1 < n ? lane + 1 : 0);
   return kCut;
 }
 
@@ -513,7 +514,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_clip_round(Dev d) {
     const int target = d.work_target[wpar][i];
     const int start = d.work_cursor[wpar][i];
     V2 p = lane < n ? piece_at(d.work_v[wpar], i)[lane] : v2(0.0, 0.0);
-    V2 q = shfl(p, lane + 1 < n ? lane + 1 : 0);
+    V2 q = Group<32>().shfl(p, lane + 1 < n ? lane + 1 : 0);
     const int source = d.res_src[rpar][target];
     const Plane st = d.scores[source];
     // At least the steps from the root to a leaf group, so that every round
@@ -524,7 +525,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_clip_round(Dev d) {
       const Tree &t = tree == 0 ? d.source_tree : d.residual_tree;
       const int leaves = tree == 0 ? source_leaves : residual_leaves;
       const int cursor = tree == start >> kCursorTree ? start & kCursorLeaf : 0;
-      Box box = warp_bounds(p, n, st);
+      Box box = group_bounds<32>(p, n, st);
       box.lo.z = -1.0e30f;
       WarpWalk w;
       walk_begin(w, t, leaves, box.lo, box.hi, cursor);
@@ -571,7 +572,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_clip_round(Dev d) {
           done = result == kFailed || n == 0;
           if (done) break;
           whole = false;
-          box = warp_bounds(p, n, st);
+          box = group_bounds<32>(p, n, st);
           box.lo.z = -1.0e30f;
         }
       }

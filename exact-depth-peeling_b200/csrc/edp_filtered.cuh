@@ -43,6 +43,11 @@ struct Tally {
     s64 += stage == pred::kBinary64;
     sx += stage == pred::kExact;
   }
+  __device__ void add(const Tally &t) {
+    s32 += t.s32;
+    s64 += t.s64;
+    sx += t.sx;
+  }
   // Adds the tallies of the calling warp's active lanes to class `cls`, one
   // atomic per counter and warp.
   __device__ void flush(const Dev &d, int cls) const {

@@ -1,5 +1,6 @@
-// Contour-guided convex subdivision: one round of the device-controlled loop
-// (warp_peel/frontier.py:81-245, event_kernels.py:12-25).
+// Contour-guided convex subdivision: per-source candidate lists, then rounds
+// of the device-controlled loop (warp_peel/frontier.py:15-245,
+// event_kernels.py:12-25).
 #include "edp_filtered.cuh"
 #include "edp_internal.h"
 #include "edp_warp.cuh"
@@ -8,24 +9,7 @@ namespace edp {
 namespace {
 
 constexpr int kBlock = 128;
-
 constexpr int kWarps = kBlock / 32;
-// Dev::step_budget: group tests one patch may spend per round before it
-// carries over.  The budget decides only how the work is spread over rounds,
-// never which cut a patch takes: every patch meets its candidates in leaf
-// order in any case.
-
-// Does segment a->b cut the patch?  Its line has patch vertices strictly on
-// both sides, and the part of the segment inside the patch lies strictly in
-// front of it somewhere: the segment's parameter range clipped by each patch
-// edge and by the depth half-plane stays open (frontier.py:81-103).  za, zb
-// are patch depth minus segment depth at the ends (positive: segment nearer).
-//
-// The warp takes a batch's candidates one by one in leaf order with a lane per
-// patch edge (p -> q): ballots decide the sides and the closed edges, and warp
-// maxima / minima give the clip range, which is a max / min of the same
-// quotients as the sequential clip and so is order-free.  Each lane first
-// loads one candidate of the batch, so the loop itself reads no memory.
 
 // The contour segments: hierarchy leaf ids, end points and depth at the ends.
 struct Segments {
@@ -36,7 +20,14 @@ struct Segments {
   const Plane *scores;
   const int2 *vid;       // the welded mesh vertex at each end, or -1
   const int *faces, *canonical, *clipped, *src_n;
+  const float4 *lo, *hi;
 };
+
+__device__ inline Segments segments_of(const Dev &d) {
+  return Segments{d.seg_tree.ids, d.seg_a, d.seg_b, d.seg_near, d.seg_near_src,
+                  d.seg_near_mag, d.scores, d.seg_vid, d.faces, d.canonical, d.clipped,
+                  d.src_n, d.seg_lo, d.seg_hi};
+}
 
 // Source `s` is an unclipped triangle with welded vertex `v`.
 __device__ inline bool has_vertex(const Segments &g, int s, int v) {
@@ -45,174 +36,360 @@ __device__ inline bool has_vertex(const Segments &g, int s, int v) {
   return g.canonical[f[0]] == v || g.canonical[f[1]] == v || g.canonical[f[2]] == v;
 }
 
-// Predicate tallies of one subdivision warp (counted form only).
+// Depth order of a source and a segment at the segment's two ends, each +1
+// where the segment is nearer: 3 (sa + 1) + (sb + 1), or kDepthOpen when the
+// filter-only form (F = 4) leaves a sign undecided.
+constexpr int kDepthOpen = 9;
+
+// Neither end of the segment is nearer.
+__device__ inline bool behind(int code) { return code / 3 <= 1 && code % 3 <= 1; }
+
+// The plane `sc` of `source` against the plane of the source that gives
+// segment c its near depth, at the segment's ends a and b.  The plain form
+// compares the rounded depths.  The filtered forms: each binary64 evaluation
+// is within 3.01 u of its terms' magnitudes (two products, two sums), so a
+// difference above 4 u of both magnitudes has its sign.  Otherwise: zero when
+// the end is a mesh vertex of both triangles (both planes pass through it: the
+// projected mesh's exact depths tie there, which the rounded plane
+// coefficients can only approximate), else the two planes compared exactly
+// (zero when the source is the patch's own).
+template <int F>
+__device__ inline int depth_code(const Segments &g, int c, V2 a, V2 b, V2 near, const Plane &sc,
+                                 int source, Tally &tally) {
+  const double za = value(sc, a) - near.x, zb = value(sc, b) - near.y;
+  if constexpr (F == 0) {
+    return 3 * (sign_of(za) + 1) + sign_of(zb) + 1;
+  } else {
+    const V2 mag = g.near_mag[c];
+    const double z[2] = {za, zb};
+    const double bound[2] = {
+        4.0 * pred::kU64 * (fabs(sc.a * a.x) + fabs(sc.b * a.y) + fabs(sc.c) + mag.x),
+        4.0 * pred::kU64 * (fabs(sc.a * b.x) + fabs(sc.b * b.y) + fabs(sc.c) + mag.y)};
+    int sign[2];
+    for (int e = 0; e < 2; ++e) {
+      int stage = pred::kBinary64;
+      if (fabs(z[e]) > bound[e]) {
+        sign[e] = sign_of(z[e]);
+      } else {
+        const int2 srcs = g.near_src[c], vids = g.vid[c];
+        const int s = e ? srcs.y : srcs.x, v = e ? vids.y : vids.x;
+        const V2 x = e ? b : a;
+        if (has_vertex(g, source, v) && has_vertex(g, s, v))
+          sign[e] = 0;
+        else
+          sign[e] = order_sign<F>(sc, value(sc, x), g.scores[s], e ? near.y : near.x, x, stage);
+      }
+      if constexpr (F == 2) tally.add(stage);
+    }
+    if (F == 4 && (sign[0] == pred::kUndecided || sign[1] == pred::kUndecided)) return kDepthOpen;
+    return 3 * (sign[0] + 1) + sign[1] + 1;
+  }
+}
+
+// Predicate tallies of one thread (counted form only).
 struct CutTally {
   Tally side, segment, depth;
 };
 
-// First cutting lane of a batch, or -1; a, b are its segment and `side` this
-// lane's vertex against its line (the split reuses it).  F is the predicate
-// form (edp_filtered.cuh): the plain form evaluates the reference's binary64
-// expressions; the filtered forms take exact signs of the sides, of the
-// segment ends against the patch edges and of the depth differences, and
-// keep binary64 for the clip parameters.  The filter-only form returns
-// kDeferAt - k when its filters cannot decide candidate k (no candidate
-// before k cuts): the patch is then finished by the exact pass from k on.
-constexpr int kDeferAt = -2;
+// ------------------------------------------------------------ candidate lists
+// Only some of the contour segments over a source can ever cut a patch of it.
+// The list of a source holds the ones left after three tests, each with a
+// margin far above what rounding can move a patch vertex (a cut point lies on
+// its patch edge within 1e-16, so every patch lies in its source within 1e-13):
+//   * the segment's line has source vertices more than kSideMargin away on
+//     both sides.  Any other line splits a part off a patch that is at most
+//     kSideMargin wide, whose doubled area is at most kSideMargin times its
+//     perimeter: clean() drops it (below kEps = 1e-10 times the perimeter) and
+//     the cut is cancelled;
+//   * the segment is nowhere more than kOutsideMargin outside a source edge
+//     with both ends: it lies apart from every patch, and the patch edge its
+//     line enters by has both ends on its outside;
+//   * it is nearer than the source at an end, which depends on the source and
+//     the segment alone (depth_code, stored with the entry).
+// The entries are in leaf order, so a patch meets the cutting candidates in
+// the order of the hierarchy walk, and takes the same cuts.
+constexpr double kSideMargin = 1.0e-12;
+constexpr double kOutsideMargin = 1.0e-7;
+constexpr int kListBuffer = 192;  // entries a warp holds before it writes a list
+constexpr int kUnlisted = -1;     // Dev::cand_count of a source without a list
 
+// Can segment c cut a patch of the source v[0..n)?  `code` receives its depth
+// code.
 template <int F>
-__device__ inline int first_cut(Segments g, unsigned batch, int first, V2 p, V2 q, int n,
-                                const Plane &sc, int source, V2 &a, V2 &b, int &side,
-                                CutTally &tally) {
-  const int lane = threadIdx.x & 31;
-  const bool mine = lane < n;
-  const int width = lane_width(n);
-  V2 ca = v2(0.0, 0.0), cb = ca, cn = ca;
-  int cid = 0;  // the lane's candidate: its near sources and vertices are read only
-                // where a depth filter leaves the sign open (rare)
-  if ((batch >> lane) & 1u) {
-    const int c = __ldg(&g.ids[first + lane]);
-    cid = c;
-    ca = g.a[c];
-    cb = g.b[c];
-    cn = g.near[c];
+__device__ inline bool may_cut(const Segments &g, int c, const V2 *v, int n, const Plane &sc,
+                               int source, int &code, CutTally &tally) {
+  const V2 a = g.a[c], b = g.b[c];
+  const double margin = kSideMargin * (fabs(b.x - a.x) + fabs(b.y - a.y));
+  double most = 0.0, least = 0.0;
+  for (int j = 0; j < n; ++j) {
+    const double side = cross(a, b, v[j]);
+    most = fmax(most, side);
+    least = fmin(least, side);
   }
-  while (batch) {
-    const int k = __ffs(int(batch)) - 1;
-    batch &= batch - 1;
-    a = shfl(ca, k);
-    b = shfl(cb, k);
-    int stage = 0;
-    if constexpr (F == 0) {
-      side = sign_of(cross(a, b, p));
-    } else {
-      side = mine ? side_sign<F>(a, b, p, stage) : 0;
-      if constexpr (F == 2)
-        if (mine) tally.side.add(stage);
-      if constexpr (F == 4)
-        if (__any_sync(kFull, side == pred::kUndecided)) return kDeferAt - k;
+  if constexpr (F == 2) {  // the exact sides of the same vertices, for the tally
+    for (int j = 0; j < n; ++j) {
+      int stage = 0;
+      side_sign<F>(a, b, v[j], stage);
+      tally.side.add(stage);
     }
-    if (!__ballot_sync(kFull, mine && side > 0) || !__ballot_sync(kFull, mine && side < 0))
+  }
+  if (!(most > margin && least < -margin)) return false;
+  for (int j = 0; j < n; ++j) {
+    const V2 p = v[j], q = v[j + 1 < n ? j + 1 : 0];
+    const double outside = -kOutsideMargin * (fabs(q.x - p.x) + fabs(q.y - p.y));
+    if (cross(p, q, a) < outside && cross(p, q, b) < outside) return false;
+  }
+  code = depth_code<F>(g, c, a, b, g.near[c], sc, source, tally.depth);
+  return !behind(code);
+}
+
+// One warp per source: its candidate list, and its first patch.  The warp
+// walks the contour hierarchy once with the source's box, a candidate per
+// lane.  A source with an empty list is a final polygon as it is; any other
+// joins the frontier.  A source whose list does not fit the pool is left
+// without one, and its patches walk the hierarchy themselves.
+// Bound by the walk's dependent loads (a warp per source, 4 to 5 steps).
+// Listing once per source replaced a hierarchy walk per patch whose candidates
+// were tested by a whole warp each: on the 65,536-face knot 783K patch walks
+// and 3.7M candidate tests against 65K walks, 0.19 ms here.
+template <int F>
+__global__ void __launch_bounds__(kBlock) k_candidates(Dev d) {
+  __shared__ int2 s_list[kWarps][kListBuffer];
+  __shared__ V2 s_source[kWarps][kSourceVertices];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  const bool fits = int64_t(d.n) <= d.cap.frontier;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && !fits) set_error(d.status, kErrResidual);
+  if (!fits || d.status[kError] != 0) return;
+  const Segments segs = segments_of(d);
+  const int leaves = *d.seg_tree.size;
+  int2 *list = s_list[warp];
+  V2 *v = s_source[warp];
+  CutTally tally;
+  const int warps = int(gridDim.x) * kWarps;
+  for (int s = int(blockIdx.x) * kWarps + warp; s < d.n; s += warps) {
+    const int n = d.src_n[s];
+    if (n == 0) continue;
+    const Plane sc = d.scores[s];
+    __syncwarp();
+    V2 p = v2(0.0, 0.0);
+    if (lane < n) {
+      p = d.src_v[int64_t(kSourceVertices) * s + lane];
+      v[lane] = p;
+    }
+    __syncwarp();
+    float4 lo = d.src_lo[s];
+    const float4 hi = d.src_hi[s];
+    lo.z = -1.0e30f;
+    int total = 0, start = 0;
+    // The first walk lists up to kListBuffer entries; a longer list is written
+    // straight to its place by a second one.
+    for (int pass = 0; pass < 2; ++pass) {
+      WarpWalk w;
+      walk_begin(w, d.seg_tree, leaves, lo, hi, 0);
+      int budget = 0x7fffffff, first, resume, at = 0;
+      unsigned batch;
+      while (walk_next(w, d.seg_tree, leaves, lo, hi, 0, budget, batch, first, resume)) {
+        int c = 0, code = 0;
+        bool keep = false;
+        if ((batch >> lane) & 1u) {
+          c = __ldg(&segs.ids[first + lane]);
+          keep = may_cut<F>(segs, c, v, n, sc, s, code, tally);
+        }
+        const unsigned kept = __ballot_sync(kFull, keep);
+        const int slot = at + __popc(kept & below);
+        if (keep) {
+          if (pass == 1)
+            d.cand[int64_t(start) + slot] = make_int2(c, code);
+          else if (slot < kListBuffer)
+            list[slot] = make_int2(c, code);
+        }
+        at += __popc(kept);
+      }
+      if (pass == 1) break;
+      total = at;
+      if (total == 0) break;
+      if (lane == 0) start = atomicAdd(&d.sc[kCandidates], total);
+      start = __shfl_sync(kFull, start, 0);
+      if (start < 0 || int64_t(start) + total > d.cand_cap) {
+        total = kUnlisted;
+        if (lane == 0) atomicAdd(&d.sc[kCandidates], -at);
+        break;
+      }
+      if (total <= kListBuffer) {
+        __syncwarp();
+        for (int k = lane; k < total; k += 32) d.cand[int64_t(start) + k] = list[k];
+        __syncwarp();
+        break;
+      }
+    }
+    int slot = 0;
+    if (lane == 0) slot = atomicAdd(total == 0 ? &d.status[kPolygons] : &d.status[kResidual], 1);
+    slot = __shfl_sync(kFull, slot, 0);
+    if (total == 0) {
+      if (slot >= d.cap.regions) {
+        if (lane == 0) set_error(d.status, kErrOutput);
+        continue;
+      }
+      if (lane < n) d.out_v[int64_t(kMaxVertices) * slot + lane] = p;
+      if (lane == 0) {
+        d.out_n[slot] = n;
+        d.out_src[slot] = s;
+        d.out_layer[slot] = 0;
+      }
       continue;
-    const V2 near = shfl(cn, k);
-    const double za = value(sc, a) - near.x, zb = value(sc, b) - near.y;
-    int sza, szb;
-    if constexpr (F == 0) {
-      sza = sign_of(za);
-      szb = sign_of(zb);
-    } else {
-      // The patch's depth plane against the plane of the source that gives
-      // the segment its near depth, at the segment's ends.  Each binary64
-      // evaluation is within 3.01 u of its terms' magnitudes (two products,
-      // two sums), so a difference above 4 u of both magnitudes has its sign.
-      // Otherwise: zero when the end is a mesh vertex of both triangles (both
-      // planes pass through it: the projected mesh's exact depths tie there,
-      // which the rounded plane coefficients can only approximate), else the
-      // two planes compared exactly (zero when the source is the patch's
-      // own).
-      int stage_b = 0;
-      const V2 mag = g.near_mag[__shfl_sync(kFull, cid, k)];
-      const double bound_a = 4.0 * pred::kU64 *
-          (fabs(sc.a * a.x) + fabs(sc.b * a.y) + fabs(sc.c) + mag.x);
-      const double bound_b = 4.0 * pred::kU64 *
-          (fabs(sc.a * b.x) + fabs(sc.b * b.y) + fabs(sc.c) + mag.y);
-      const int c = __shfl_sync(kFull, cid, k);
-      if (fabs(za) > bound_a) {
-        sza = sign_of(za);
-        stage = pred::kBinary64;
-      } else {
-        const int sa = g.near_src[c].x, va = g.vid[c].x;
-        if (has_vertex(g, source, va) && has_vertex(g, sa, va)) {
-          sza = 0;
-          stage = pred::kBinary64;
-        } else {
-          sza = order_sign<F>(sc, value(sc, a), g.scores[sa], near.x, a, stage);
-        }
-      }
-      if (fabs(zb) > bound_b) {
-        szb = sign_of(zb);
-        stage_b = pred::kBinary64;
-      } else {
-        const int sb = g.near_src[c].y, vb = g.vid[c].y;
-        if (has_vertex(g, source, vb) && has_vertex(g, sb, vb)) {
-          szb = 0;
-          stage_b = pred::kBinary64;
-        } else {
-          szb = order_sign<F>(sc, value(sc, b), g.scores[sb], near.y, b, stage_b);
-        }
-      }
-      if constexpr (F == 2) {
-        if (lane == 0) {  // the same test on every lane: count it once
-          tally.depth.add(stage);
-          tally.depth.add(stage_b);
-        }
-      }
-      if constexpr (F == 4)
-        if (sza == pred::kUndecided || szb == pred::kUndecided) return kDeferAt - k;
     }
-    if (sza <= 0 && szb <= 0) continue;
-    const double da = cross(p, q, a), db = cross(p, q, b);
-    int sda, sdb;
-    if constexpr (F == 0) {
-      sda = sign_of(da);
-      sdb = sign_of(db);
-    } else {
-      int stage_b = 0;
-      sda = mine ? side_sign<F>(p, q, a, stage) : 0;
-      sdb = mine ? side_sign<F>(p, q, b, stage_b) : 0;
-      if constexpr (F == 2) {
-        if (mine) {
-          tally.segment.add(stage);
-          tally.segment.add(stage_b);
-        }
-      }
-      if constexpr (F == 4)
-        if (__any_sync(kFull, sda == pred::kUndecided || sdb == pred::kUndecided))
-          return kDeferAt - k;
+    // slot < n <= frontier capacity
+    if (lane < n) d.fv[0][int64_t(kMaxVertices) * slot + lane] = p;
+    if (lane == 0) {
+      d.fn[0][slot] = n;
+      d.fsrc[0][slot] = s;
+      d.fcur[0][slot] = 0;
+      d.cand_start[s] = start;
+      d.cand_count[s] = total;
     }
-    if (__ballot_sync(kFull, mine && sda <= 0 && sdb <= 0)) continue;
-    double low, high, rz;
-    if constexpr (F == 0) {
-      const double r = da / (da - db);
-      low = mine && da < 0.0 ? fmax(0.0, r) : 0.0;
-      high = mine && db < 0.0 ? fmin(1.0, r) : 1.0;
-    } else {
-      const double r = crossing(da, db);
-      low = mine && sda < 0 ? r : 0.0;
-      high = mine && sdb < 0 ? r : 1.0;
-    }
-    for (int off = width >> 1; off > 0; off >>= 1) {  // lanes [0, width) hold the edges
-      low = fmax(low, __shfl_xor_sync(kFull, low, off));
-      high = fmin(high, __shfl_xor_sync(kFull, high, off));
-    }
-    low = __shfl_sync(kFull, low, 0);
-    high = __shfl_sync(kFull, high, 0);
-    if constexpr (F == 0)
-      rz = za / (za - zb);
-    else
-      rz = crossing(za, zb);
-    if (sza < 0) low = fmax(low, rz);
-    if (szb < 0) high = fmin(high, rz);
-    if (high > low) return k;
   }
-  return -1;
+  if constexpr (F == 2) {
+    tally.side.flush(d, kPredSide);
+    tally.depth.flush(d, kPredDepth);
+  }
 }
 
-// Split the patch (one vertex per lane, q the next vertex) by the supporting
-// line of a->b into the part on the left (pl, nl) and on the right (pr, nr),
-// both cleaned (warp_split).  The filtered forms (F > 0) classify the vertices
-// by `side`, the exact sign first_cut found, and place the cut points with
-// the binary64 values.
+__global__ void k_loop_condition(Dev d) {
+  d.status[kPeakResidual] = d.status[kResidual];
+  int c = d.status[kResidual] > 0 && d.status[kError] == 0;
+  *d.condition = c;
+  if (d.use_handle) cudaGraphSetConditional(d.cond_handle, unsigned(c));
+}
+
+// ------------------------------------------------------------ rounds
+// Does segment a->b cut the patch?  Its line has patch vertices strictly on
+// both sides, and the part of the segment inside the patch lies strictly in
+// front of it somewhere: the segment's parameter range clipped by each patch
+// edge and by the depth half-plane stays open (frontier.py:81-103).
+//
+// Two tests decide it.  `certainly_missed` takes a candidate per lane against
+// the whole patch and rejects most of a list chunk at once; `cuts` takes one
+// candidate of the few left with a lane per patch edge (p -> q).
+//
+// certainly_missed: no patch vertex on one of the line's sides, or a patch
+// edge with both segment ends on its outside.  F = 0 takes the signs of
+// `cuts`.  The filtered forms take signs that a filter decides: with one
+// difference rounded per factor, the two products and their difference are
+// within 5 u of S = |product| + |product|, so a determinant above 8 u S has its
+// sign; it is zero when S is, and when the point is an end of the edge.
+struct QuickSign {
+  bool positive, negative, zero;  // none: undecided
+};
+
 template <int F>
-__device__ inline bool split_line(V2 p, V2 q, int n, V2 a, V2 b, int side, V2 *left, V2 *right,
-                                  V2 &pl, int &nl, V2 &pr, int &nr) {
-  const V2 dir = b - a;
-  const Plane s{-dir.y, dir.x, 0.0, 0.0};
-  const double du = value(s, p - a);
-  return warp_split<F>(p, q, n, du, F == 0 ? sign_of(du) : side, left, right, pl, nl, pr, nr);
+__device__ inline QuickSign quick_side(V2 a, V2 dir, V2 b, V2 c) {
+  const V2 w = c - a;
+  const double s = dir.x * w.y, t = dir.y * w.x, det = s - t;
+  if constexpr (F == 0) return QuickSign{det > 0.0, det < 0.0, det == 0.0};
+  const double sum = fabs(s) + fabs(t), bound = 8.0 * pred::kU64 * sum;
+  const bool zero = sum == 0.0 || c == b;
+  return QuickSign{!zero && det > bound, !zero && det < -bound, zero};
 }
 
-// The next round's frontier.
+template <int F>
+__device__ inline bool certainly_missed(const V2 *v, int n, int most, V2 a, V2 b, bool meets) {
+  const V2 dir = b - a;
+  bool left = false, right = false;  // some vertex is or may be there
+  for (int j = 0; j < most; ++j) {   // most: the largest n in the warp
+    const QuickSign s = quick_side<F>(a, dir, b, v[j]);
+    left = left || (j < n && !s.negative && !s.zero);
+    right = right || (j < n && !s.positive && !s.zero);
+  }
+  bool missed = !left || !right;
+  if (!__any_sync(kFull, meets && !missed)) return true;
+  V2 p = v[0];
+  for (int j = 0; j < most; ++j) {
+    const V2 q = v[j + 1 < n ? j + 1 : 0], edge = q - p;
+    const QuickSign sa = quick_side<F>(p, edge, q, a), sb = quick_side<F>(p, edge, q, b);
+    missed = missed || (j < n && (sa.negative || sa.zero) && (sb.negative || sb.zero));
+    p = q;
+  }
+  return missed;
+}
+
+// cuts: ballots decide the sides and the closed edges, and butterflies give
+// the clip range, which is a max / min of the same quotients as the
+// sequential clip and so is order-free.  F is the predicate form
+// (edp_filtered.cuh): the plain form evaluates the reference's binary64
+// expressions; the filtered forms take exact signs of the sides and of the
+// segment ends against the patch edges, and keep binary64 for the clip
+// parameters.  The filter-only form gives kOpen when its filters cannot
+// decide.  `side` is left with this lane's vertex against the line (the split
+// reuses it).
+enum CutTest : int { kMiss = 0, kHit = 1, kOpen = 2 };
+
+template <int F, int W>
+__device__ inline int cuts(const Group<W> &g, V2 p, V2 q, int n, const Plane &sc, V2 a, V2 b,
+                           V2 near, int code, int &side, CutTally &tally) {
+  const bool mine = g.lane < n;
+  int stage = 0, stage_a = 0, stage_b = 0, sda, sdb;
+  const double da = cross(p, q, a), db = cross(p, q, b);
+  if constexpr (F == 0) {
+    side = sign_of(cross(a, b, p));
+    sda = sign_of(da);
+    sdb = sign_of(db);
+  } else {
+    side = mine ? side_sign<F>(a, b, p, stage) : 0;
+    sda = mine ? side_sign<F>(p, q, a, stage_a) : 0;
+    sdb = mine ? side_sign<F>(p, q, b, stage_b) : 0;
+    if constexpr (F == 2) {
+      if (mine) {
+        tally.side.add(stage);
+        tally.segment.add(stage_a);
+        tally.segment.add(stage_b);
+      }
+    }
+  }
+  // Every ballot is taken by the whole warp, whatever the groups' answers.
+  const unsigned undecided = F == 4 ? g.ballot(side == pred::kUndecided ||
+                                               sda == pred::kUndecided ||
+                                               sdb == pred::kUndecided)
+                                    : 0u;
+  const unsigned lefts = g.ballot(mine && side > 0), rights = g.ballot(mine && side < 0);
+  const unsigned closed = g.ballot(mine && sda <= 0 && sdb <= 0);
+  const bool open = code == kDepthOpen || undecided != 0;
+  const bool miss = lefts == 0 || rights == 0 || closed != 0 || behind(code);
+  const int sza = code / 3 - 1, szb = code % 3 - 1;
+  double low, high, rz;
+  const double za = value(sc, a) - near.x, zb = value(sc, b) - near.y;
+  if constexpr (F == 0) {
+    const double r = da / (da - db);
+    low = mine && da < 0.0 ? fmax(0.0, r) : 0.0;
+    high = mine && db < 0.0 ? fmin(1.0, r) : 1.0;
+    rz = za / (za - zb);
+  } else {
+    const double r = crossing(da, db);
+    low = mine && sda < 0 ? r : 0.0;
+    high = mine && sdb < 0 ? r : 1.0;
+    rz = crossing(za, zb);
+  }
+  const int width = W == 8 ? 8 : lane_width(n);
+  for (int off = width >> 1; off > 0; off >>= 1) {  // lanes [0, width) hold the edges
+    low = larger(low, g.shfl_xor(low, off));
+    high = smaller(high, g.shfl_xor(high, off));
+  }
+  if (W > 8) {
+    low = g.shfl(low, 0);
+    high = g.shfl(high, 0);
+  }
+  if (sza < 0) low = larger(low, rz);
+  if (szb < 0) high = smaller(high, rz);
+  if (open) return kOpen;
+  return !miss && high > low ? kHit : kMiss;
+}
+
+// A frontier's patch pool.  `n` holds the vertex count and, above it, the
+// patch's generation: how many right-hand parts lie on its way from the
+// source.  A generation at Dev::cap.rounds is the round-capacity error.
+constexpr int kSizeBits = 6;
+constexpr int kSizeMask = (1 << kSizeBits) - 1;
+
 struct Frontier {
   V2 *v;
   int *n, *src, *cur;
@@ -220,182 +397,326 @@ struct Frontier {
   int64_t capacity;
 };
 
-// Append a patch (one vertex per lane) to the next frontier; false on overflow.
-__device__ __noinline__ bool push_patch(Frontier f, V2 p, int n, int source, int cursor) {
-  const int lane = threadIdx.x & 31;
-  int slot = 0;
-  if (lane == 0) slot = atomicAdd(f.count, 1);
-  slot = __shfl_sync(kFull, slot, 0);
-  if (slot >= f.capacity) {
-    if (lane == 0) set_error(f.status, kErrResidual);
-    return false;
+// Append the patches of the groups that `want` it (one vertex per lane) to the
+// frontier, upwards from slot 0, or downwards from its last slot (`top`) for
+// patches left to this round's second pass, counted in `count`.  Returns the
+// slot, or -1 on overflow.
+template <int W>
+__device__ __noinline__ int64_t push_patch(Frontier f, int *count, bool top, bool want, V2 p,
+                                           int size, int source, int cursor) {
+  const Group<W> g;
+  const int k = g.reserve_slot(count, want);
+  if (!want) return -1;
+  const int64_t slot = top ? f.capacity - 1 - k : int64_t(k);
+  if (slot < 0 || slot >= f.capacity) {
+    if (g.lane == 0) set_error(f.status, kErrResidual);
+    return -1;
   }
-  if (lane < n) f.v[int64_t(kMaxVertices) * slot + lane] = p;
-  if (lane == 0) {
-    f.n[slot] = n;
+  if (g.lane < (size & kSizeMask)) f.v[int64_t(kMaxVertices) * slot + g.lane] = p;
+  if (g.lane == 0) {
+    f.n[slot] = size;
     f.src[slot] = source;
     f.cur[slot] = cursor;
   }
-  return true;
+  return slot;
 }
 
-// Park a patch at the top of the next frontier `f` for this round's exact
-// pass (from its cursor on); false when the frontier is full.  `parked`
-// counts the parked patches.
-__device__ __noinline__ bool defer_patch(Frontier f, int *parked, V2 p, int n, int source,
-                                         int cursor) {
-  const int lane = threadIdx.x & 31;
-  int k = 0;
-  if (lane == 0) k = atomicAdd(parked, 1);
-  k = __shfl_sync(kFull, k, 0);
-  const int64_t slot = f.capacity - 1 - k;
-  if (slot < 0) {
-    if (lane == 0) set_error(f.status, kErrResidual);
-    return false;
-  }
-  if (lane < n) f.v[int64_t(kMaxVertices) * slot + lane] = p;
-  if (lane == 0) {
-    f.n[slot] = n;
-    f.src[slot] = source;
-    f.cur[slot] = cursor;
-  }
-  return true;
+// The first leaf batch of the contour hierarchy at or after leaf `cursor`
+// whose leaves meet the box, for a source without a list (a walk from the
+// root each time: no walk state stays live in the caller).
+__device__ __noinline__ unsigned walk_batch(Tree t, int leaves, float4 lo, float4 hi, int cursor,
+                                            int &first) {
+  WarpWalk w;
+  walk_begin(w, t, leaves, lo, hi, cursor);
+  int budget = 0x7fffffff, resume;
+  unsigned batch;
+  return walk_next(w, t, leaves, lo, hi, cursor, budget, batch, first, resume) ? batch : 0u;
 }
 
-// One frontier round, one patch per warp (frontier.py:106-223).  A patch
-// meets the contour segments whose boxes overlap its own in leaf order,
-// starting at its cursor (the first leaf it has not met).  The first segment
-// that cuts it splits it along the segment's line: the right part goes to the
-// next round, the left part continues in this warp, both with the cursor just
-// past the cutting leaf (a collapsed part cancels the cut and the patch
-// continues).  The continuing part keeps its walk: only the cut's leaf group
-// is tested again, against the part's box; pending groups above it are
-// tested against the part's box when they are expanded.  A patch that has
-// met every candidate is final and goes to the output pool; one that spends
-// its budget carries over.  Warps take patches from a shared counter.
+constexpr int kStack = 8;     // patches a group keeps for itself
+constexpr int kLocalCuts = 6; // cuts of one taken patch whose right parts stay local
+constexpr int kMostCuts = 8;  // cuts of one taken patch before its parts go to the next round
+
+// One frontier round (frontier.py:106-223), a patch per group of W lanes.  A
+// patch meets its source's listed segments whose boxes overlap its own, from
+// its cursor on, in leaf order.  The first segment that cuts it splits it
+// along the segment's line; a collapsed part cancels the cut.  The left part
+// continues in the group, and the right part waits on the group's stack, or,
+// past kStack waiting parts or kLocalCuts cuts, in the next round's frontier,
+// where other groups take it; both have the cursor just past the cutting
+// segment.  After kMostCuts cuts the left part goes to the next round too.  A
+// patch that has met every candidate is final and goes to the output pool.  Groups take patches from a shared counter.
 //
-// With filtered binary64 predicates the round runs twice: the filter-only
-// form (F = 4, no exact stage, so fewer registers and less code) over the
-// frontier, parking every patch whose filters cannot decide a test at the top
-// of the next frontier with its cursor at that test; then form 3, with the
-// exact stages, over the parked patches (`deferred_pass`).  Each patch meets
-// the same tests in the same order as in one form-3 pass, so the output is
-// the same.
-template <int F>
-__global__ void __launch_bounds__(kBlock, (F == 0 || F == 4) ? 5 : 4)
-    k_subdivide(Dev d, int deferred_pass) {
-  __shared__ V2 s_parts[kWarps][2][kMaxVertices];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  V2 *left_part = s_parts[warp][0], *right_part = s_parts[warp][1];
+// The groups of a warp run one loop in step: take a patch, find its next
+// candidate, test it, split.  Every step is run by the whole warp when any
+// group needs it.
+//
+// W = 8 is the first pass of a round, with the filter-only form (F = 4) under
+// filtered binary64 predicates (no exact stage, so fewer registers and less
+// code).  It parks a patch at the top of the next frontier, with its cursor
+// at the candidate it stopped at, when its filters cannot decide, when a part
+// would have more than 8 vertices, or when its source has no list.  W = 32 is
+// the second pass, with the exact stages, over the parked patches: it takes
+// each one past the candidate that stopped it and hands it, or its two parts,
+// to the next round (a patch that no group of eight lanes can take goes on).
+// Each patch meets the same tests in the same order as in one exact pass, so
+// the output is the same.
+//
+// The time is instruction issue on patches of three to six vertices, and at
+// small sizes the chain of one group's steps: a warp per patch left 26 of 32
+// lanes idle, and a round per right-hand part made 14 rounds of the knot.
+// Rounds in all (a warp per patch, then this): knot-65536 3.04 -> 1.05 ms,
+// 720K primitives 11.5 -> 3.4 ms, 2,560-face icospheres 0.60 -> 0.40 ms.  The
+// cut bounds trade a round's longest chain against the number of rounds:
+// unbounded chains took 1.2, 3.5 and 0.43 ms.  4 blocks of 128 registers per
+// SM: 5 blocks spill (1.3 ms on the knot), 3 hide less latency (1.13).
+template <int F, int W>
+__global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
+  constexpr int kGroups = kBlock / W;
+  constexpr bool kWide = W == 32;
+  constexpr int kWaiting = kWide ? 1 : kStack;
+  __shared__ V2 s_parts[kGroups][2][W];
+  __shared__ V2 s_patch[kGroups][W];
+  __shared__ V2 s_stack[kGroups][kWaiting][W];
+  __shared__ int2 s_waiting[kGroups][kWaiting];  // size and generation, cursor
+  const Group<W> g;
+  const int slot = threadIdx.x / W, lane = threadIdx.x & 31;
+  V2 *left_part = s_parts[slot][0], *right_part = s_parts[slot][1];
   const int par = *d.parity;
-  const int from = deferred_pass ? par ^ 1 : par;
+  const int from = kWide ? par ^ 1 : par;
   const V2 *fv = d.fv[from];
   const int *fn = d.fn[from], *fsrc = d.fsrc[from], *fcur = d.fcur[from];
-  const int parked = deferred_pass ? int(min(int64_t(d.sc[kDeferred]), d.cap.frontier)) : 0;
-  const int live = deferred_pass ? parked : int(min(int64_t(d.status[kResidual]), d.cap.frontier));
-  int *taken = deferred_pass ? &d.sc[kDeferredNext] : &d.sc[kFrontierNext];
-  const int leaves = *d.seg_tree.size;
-  const int next_lane = lane + 1;
-  const Segments segs{d.seg_tree.ids, d.seg_a, d.seg_b, d.seg_near, d.seg_near_src,
-                      d.seg_near_mag, d.scores, d.seg_vid, d.faces, d.canonical, d.clipped,
-                      d.src_n};
+  const int parked = kWide ? int(min(int64_t(d.sc[kDeferred]), d.cap.frontier)) : 0;
+  const int live = kWide ? parked : int(min(int64_t(d.status[kResidual]), d.cap.frontier));
+  int *taken = kWide ? &d.sc[kDeferredNext] : &d.sc[kFrontierNext];
+  const Segments segs = segments_of(d);
   const Frontier next{d.fv[par ^ 1], d.fn[par ^ 1], d.fsrc[par ^ 1], d.fcur[par ^ 1],
                       &d.status[kNextResidual], d.status, d.cap.frontier - parked};
-  long long visits = 0, tests = 0, splits = 0;  // lane 0's tallies
+  int visits = 0, tests = 0, splits = 0;  // each group's lane 0
   CutTally tally;
+  // The group's patch.
+  bool idle = true, drained = false, changed = false;
+  int waiting = 0, cut_count = 0, budget = 0;
+  int n = 0, generation = 0, source = 0, cursor = 0, start = 0, count = 0;
+  V2 p = v2(0.0, 0.0), q = p;
+  Plane sc{0.0, 0.0, 0.0, 0.0};
+  Box box{empty_lo(), empty_hi()};
+  // The candidates of the current list chunk, one per lane.
+  unsigned batch = 0;
+  int base = 0, id = 0, code = 0;
+  V2 ca = p, cb = p, cn = p;
   for (;;) {
-    int i = 0, failed = 0;
-    if (lane == 0) {
-      i = atomicAdd(taken, 1);
-      failed = *(volatile int *)&d.status[kError];
+    // Take a patch: from the group's stack, else from the frontier.
+    bool fresh = false, park = false, final = false, push = false;
+    if (idle && waiting > 0) {
+      const int2 w = s_waiting[slot][--waiting];
+      n = w.x & kSizeMask;
+      generation = w.x >> kSizeBits;
+      cursor = w.y;
+      p = s_stack[slot][waiting][g.lane];
+      fresh = true;
     }
-    i = __shfl_sync(kFull, i, 0);
-    if (i >= live || __shfl_sync(kFull, failed, 0) != 0) break;
-    if (deferred_pass) i = int(d.cap.frontier) - 1 - i;  // parked from the top down
-    int n = fn[i];
-    if (n == 0) continue;
-    ++visits;
-    const int source = fsrc[i];
-    int cursor = fcur[i];
-    V2 p = lane < n ? fv[int64_t(kMaxVertices) * i + lane] : v2(0.0, 0.0);
-    V2 q = shfl(p, next_lane < n ? next_lane : 0);
-    const Plane sc = d.scores[source];
-    int budget = d.step_budget;
-    float4 lo, hi;
-    {
-      const Box box = warp_bounds(p, n, sc);
-      lo = box.lo;
-      hi = box.hi;
+    const bool want = idle && !fresh && !drained;
+    if (__any_sync(kFull, want)) {
+      const int at = g.reserve_slot(taken, want);
+      const int failed = __shfl_sync(kFull, *(volatile int *)&d.status[kError], 0);
+      if (want && (at >= live || failed != 0)) drained = true;
+      const bool take = want && !drained;
+      const int i = kWide ? int(d.cap.frontier) - 1 - at : at;  // parked from the top down
+      int size = 0;
+      if (take) {
+        size = fn[i];
+        n = size & kSizeMask;
+        generation = size >> kSizeBits;
+        source = fsrc[i];
+        cursor = fcur[i];
+        p = g.lane < n ? fv[int64_t(kMaxVertices) * i + g.lane] : v2(0.0, 0.0);
+        sc = d.scores[source];
+        start = d.cand_start[source];
+        count = d.cand_count[source];
+        cut_count = 0;
+        fresh = true;
+      }
+      if (!kWide) {
+        // A patch too large for a group (left by the second pass of an earlier
+        // round), or one without a list: to this round's second pass.
+        const bool wide = take && (n > W || count == kUnlisted);
+        if (__any_sync(kFull, wide)) {
+          const int64_t to =
+              push_patch<W>(next, &d.sc[kDeferred], true, wide, p, size, source, cursor);
+          if (to >= 0)
+            for (int j = W + g.lane; j < n; j += W)
+              next.v[int64_t(kMaxVertices) * to + j] = fv[int64_t(kMaxVertices) * i + j];
+          fresh = fresh && !wide;
+        }
+      }
     }
-    lo.z = -1.0e30f;
-    WarpWalk w;
-    walk_begin(w, d.seg_tree, leaves, lo, hi, cursor);
+    if (fresh) {
+      idle = false;
+      ++visits;
+      batch = 0;
+      budget = d.step_budget;
+    }
+    if (__all_sync(kFull, idle && drained)) break;
+    if (idle) n = 0;
+    if (__any_sync(kFull, fresh || changed)) {
+      q = g.shfl(p, g.lane + 1 < n ? g.lane + 1 : 0);
+      box = group_bounds<W>(p, n, sc);
+      box.lo.z = -1.0e30f;
+      s_patch[slot][g.lane] = p;
+      changed = false;
+      __syncwarp();
+    }
+    // Find the next chunk with a candidate.
+    const int most = W == 8 ? __reduce_max_sync(kFull, n) : n;
     for (;;) {
-      unsigned batch;
-      int first, resume = leaves, cut = -1, side = 0, defer = -1;
-      V2 a, b;
-      while (walk_next(w, d.seg_tree, leaves, lo, hi, cursor, budget, batch, first, resume)) {
-        cut = first_cut<F>(segs, batch, first, p, q, n, sc, source, a, b, side, tally);
-        if constexpr (F == 4) {
-          if (cut <= kDeferAt) {
-            defer = first + (kDeferAt - cut);
-            break;
+      bool look = !idle && !push && !final && batch == 0;
+      if (!__any_sync(kFull, look)) break;
+      bool meets = false;
+      if (kWide && count == kUnlisted) {
+        const int leaves = *d.seg_tree.size;
+        int first = 0;
+        const unsigned found = walk_batch(d.seg_tree, leaves, box.lo, box.hi, cursor, first);
+        final = found == 0;
+        if (!final) {
+          base = first;
+          cursor = base + W;
+          meets = (found >> g.lane) & 1u;
+          if (meets) {
+            id = __ldg(&segs.ids[base + g.lane]);
+            code = kDepthOpen;
           }
         }
-        tests += __popc(cut >= 0 ? batch & (kFull >> (31 - cut)) : batch);  // met up to the cut
-        if (cut >= 0) break;
-      }
-      if constexpr (F == 4) {
-        if (defer >= 0) {
-          defer_patch(next, &d.sc[kDeferred], p, n, source, defer);
-          break;
+      } else if (look) {
+        if (cursor >= count) {
+          final = true;
+        } else if (--budget < 0) {
+          push = true;  // a long walk carries over, so that one patch does not hold a round
+        } else {
+          base = cursor;
+          cursor += W;
+          if (base + g.lane < count) {
+            const int2 e = d.cand[int64_t(start) + base + g.lane];
+            id = e.x;
+            code = e.y;
+            meets = overlaps(segs.lo[id], segs.hi[id], box.lo, box.hi);
+          }
         }
       }
-      if (cut < 0) {
-        if (resume < leaves) {
-          push_patch(next, p, n, source, resume);
-          break;
-        }
-        int out = 0;
-        if (lane == 0) out = atomicAdd(&d.status[kPolygons], 1);
-        out = __shfl_sync(kFull, out, 0);
+      if (meets) {
+        ca = segs.a[id];
+        cb = segs.b[id];
+        cn = segs.near[id];
+      }
+      tests += __popc(g.ballot(meets));
+      if (!kWide && __any_sync(kFull, meets)) {
+        const bool missed = certainly_missed<F>(s_patch[slot], n, most, ca, cb, meets);
+        meets = meets && !missed;
+      }
+      const unsigned found = g.ballot(meets);
+      if (look) batch = found;
+    }
+    // Final patches.
+    if (__any_sync(kFull, final)) {
+      const int out = g.reserve_slot(&d.status[kPolygons], final);
+      if (final) {
         if (out >= d.cap.regions) {
-          if (lane == 0) set_error(d.status, kErrOutput);
-          break;
+          if (g.lane == 0) set_error(d.status, kErrOutput);
+        } else {
+          if (g.lane < n) d.out_v[int64_t(kMaxVertices) * out + g.lane] = p;
+          if (g.lane == 0) {
+            d.out_n[out] = n;
+            d.out_src[out] = source;
+            d.out_layer[out] = 0;
+          }
         }
-        if (lane < n) d.out_v[int64_t(kMaxVertices) * out + lane] = p;
-        if (lane == 0) {
-          d.out_n[out] = n;
-          d.out_src[out] = source;
-          d.out_layer[out] = 0;
+      }
+    }
+    // Test the next candidate.
+    const bool test = batch != 0;
+    bool cut = false, moved = false;
+    int side = 0, k = 0;
+    V2 a = v2(0.0, 0.0), b = a;
+    if (__any_sync(kFull, test)) {
+      k = test ? __ffs(int(batch)) - 1 : 0;
+      batch &= batch - 1;
+      a = g.shfl(ca, k);
+      b = g.shfl(cb, k);
+      const V2 near = g.shfl(cn, k);
+      int order = g.shfl(code, k);
+      if constexpr (kWide) {
+        const int c = g.shfl(id, k);
+        if (order == kDepthOpen) {
+          Tally rest;  // the same test on every lane: lane 0 counts it
+          order = depth_code<F>(segs, c, a, b, near, sc, source, rest);
+          if (F == 2 && lane == 0) tally.depth.add(rest);
         }
-        break;
       }
-      cursor = first + cut + 1;
-      V2 pl, pr;
-      int nl, nr;
-      if (!split_line<F>(p, q, n, a, b, side, left_part, right_part, pl, nl, pr, nr)) {
-        if (lane == 0) set_error(d.status, kErrPolygon);
-        break;
+      const int result = cuts<F, W>(g, p, q, test ? n : 0, sc, a, b, near, order, side, tally);
+      cut = test && result == kHit;
+      park = test && result == kOpen;
+    }
+    // Split along the segment's line.
+    bool keep_right = false;
+    V2 pr = p;
+    int nr = 0;
+    if (__any_sync(kFull, cut)) {
+      const V2 dir = b - a;
+      const double du = value(Plane{-dir.y, dir.x, 0.0, 0.0}, p - a);
+      if constexpr (F == 0) side = sign_of(du);
+      V2 pl;
+      int nl;
+      const bool fits = group_split<F>(g, p, q, cut ? n : 0, du, side, left_part, right_part, pl,
+                                       nl, pr, nr);
+      if (cut && !fits) {
+        if (kWide && g.lane == 0) set_error(d.status, kErrPolygon);
+        park = true;  // in the second pass, lost to the error
       }
-      if (nl > 0 && nr > 0) {
+      if (cut && nl > 0 && nr > 0) {
         ++splits;
-        if (!push_patch(next, pr, nr, source, cursor)) break;
+        ++cut_count;
+        keep_right = moved = true;
         p = pl;
         n = nl;
-        q = shfl(p, next_lane < n ? next_lane : 0);
-        {
-      const Box box = warp_bounds(p, n, sc);
-      lo = box.lo;
-      hi = box.hi;
-    }
-        lo.z = -1.0e30f;
+        if (generation + 1 >= d.cap.rounds && g.lane == 0) set_error(d.status, kErrRounds);
       }
-      w.set_pending(walk_test(d.seg_tree, leaves, w, lo, hi, cursor));
-      __syncwarp();  // the part buffers are rewritten by the next cut
     }
+    // The right part: to the stack, or to the next round.
+    const int right_size = nr | (generation + 1) << kSizeBits;
+    if (!kWide && keep_right && waiting < kStack && cut_count < kLocalCuts) {
+      s_stack[slot][waiting][g.lane] = pr;
+      if (g.lane == 0) s_waiting[slot][waiting] = make_int2(right_size, base + k + 1);
+      ++waiting;
+      keep_right = false;
+    }
+    if (__any_sync(kFull, keep_right))
+      push_patch<W>(next, next.count, false, keep_right, pr, right_size, source, base + k + 1);
+    // The rest of the chunk is met again by the left part: a segment that ends
+    // on an edge of the patch may cut a part by a rounding of that edge.
+    if (moved) {
+      changed = true;
+      batch = 0;
+      cursor = base + k + 1;
+      push = !kWide && cut_count >= kMostCuts;
+    }
+    if (kWide && test && !park && n <= 8 && count != kUnlisted) {
+      cursor = base + k + 1;  // past its candidate, a group of eight lanes can go on
+      push = true;
+    }
+    // Patches that leave the group: back to the frontier, or from the undecided
+    // candidate on to the second pass.
+    if (__any_sync(kFull, push))
+      push_patch<W>(next, next.count, false, push, p, n | generation << kSizeBits, source, cursor);
+    if (!kWide && __any_sync(kFull, park))
+      push_patch<W>(next, &d.sc[kDeferred], true, park, p, n | generation << kSizeBits, source,
+                    base + k);
+    if (push || park || final) {
+      idle = true;
+      batch = 0;
+    }
+    __syncwarp();  // the stack and the part buffers
   }
-  if (lane == 0) {
+  if (g.lane == 0) {
     count_add(&d.metrics[kTargetVisits], visits);
     count_add(&d.metrics[kContourTests], tests);
     count_add(&d.metrics[kSplits], splits);
@@ -430,19 +751,45 @@ __global__ void k_advance(Dev d) {
 
 }  // namespace
 
-cudaError_t stage_step(const Dev &d, cudaStream_t st) {
-  int64_t g = ceil_div(d.cap.frontier, kWarps);
-  if (g > 148 * int64_t(d.subdivide_blocks)) g = 148 * int64_t(d.subdivide_blocks);
-  if (d.predicates == 3) {  // filtered binary64: filter-only pass, then the exact pass
-    k_subdivide<4><<<unsigned(g), kBlock, 0, st>>>(d, 0);
-    note_launch();
-    // Few patches are parked (a few thousand per extraction on the knot): a
-    // small grid takes them from the counter.
-    k_subdivide<3><<<unsigned(g < 296 ? g : 296), kBlock, 0, st>>>(d, 1);
-  } else {
-    EDP_LAUNCH_FORM(d.predicates, k_subdivide, unsigned(g), kBlock, st, d, 0);
+// The candidate lists, the uncut sources' final polygons and the first
+// frontier.
+cudaError_t stage_lists(const Dev &d, cudaStream_t st) {
+  int64_t g = ceil_div(d.n > 0 ? d.n : 1, kWarps);
+  if (g > 148 * 16) g = 148 * 16;
+  switch (d.predicates) {
+    case 0: k_candidates<0><<<unsigned(g), kBlock, 0, st>>>(d); break;
+    case 1: k_candidates<1><<<unsigned(g), kBlock, 0, st>>>(d); break;
+    case 2: k_candidates<2><<<unsigned(g), kBlock, 0, st>>>(d); break;
+    default: k_candidates<4><<<unsigned(g), kBlock, 0, st>>>(d); break;
   }
   note_launch();
+  k_loop_condition<<<1, 1, 0, st>>>(d);
+  note_launch();
+  return cudaGetLastError();
+}
+
+namespace {
+// The first pass of a round in form N, then the second, over the few parked
+// patches, in form E.
+template <int N, int E>
+void launch_round(const Dev &d, unsigned grid, unsigned second, cudaStream_t st) {
+  k_subdivide<N, 8><<<grid, kBlock, 0, st>>>(d);
+  note_launch();
+  k_subdivide<E, 32><<<second, kBlock, 0, st>>>(d);
+  note_launch();
+}
+}  // namespace
+
+cudaError_t stage_step(const Dev &d, cudaStream_t st) {
+  const int64_t most = 148 * int64_t(d.subdivide_blocks);
+  const unsigned g = unsigned(std::min(ceil_div(d.cap.frontier, kBlock / 8), most));
+  const unsigned second = unsigned(std::min<int64_t>(ceil_div(d.cap.frontier, kWarps), 296));
+  switch (d.predicates) {
+    case 0: launch_round<0, 0>(d, g, second, st); break;
+    case 1: launch_round<1, 1>(d, g, second, st); break;
+    case 2: launch_round<2, 2>(d, g, second, st); break;
+    default: launch_round<4, 3>(d, g, second, st); break;
+  }
   k_advance<<<1, 1, 0, st>>>(d);
   note_launch();
   return cudaGetLastError();

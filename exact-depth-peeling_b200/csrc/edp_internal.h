@@ -135,7 +135,8 @@ enum Scalar : int {
   kSortDeferred = 29,
   kAssignDeferred = 30,
   kDeepGroups = 31,  // hit groups sorted a warp each (k_group_sort_deep)
-  kScalarCount = 32  // k_reset clears them with one warp
+  kCandidates = 32,  // entries of the sources' candidate lists
+  kScalarCount = 33  // k_reset clears them with one block
 };
 
 // Predicate tallies: six classes by three deciding stages (edp_filtered.cuh).
@@ -196,7 +197,12 @@ struct Dev {
   int *seg_table, *seg_min, *seg_slot;
   int seg_mask;
   Tree source_tree, seg_tree, point_tree;
-  // frontier ping-pong
+  // Candidate lists of the subdivision: per source, its entries (segment,
+  // depth code) in leaf order, or a count of -1 where the pool had no room.
+  int2 *cand;
+  int *cand_start, *cand_count;
+  int64_t cand_cap;
+  // frontier ping-pong; fn holds the vertex count and the generation
   V2 *fv[2];
   int *fn[2], *fsrc[2], *fcur[2];
   // output polygons
@@ -331,6 +337,7 @@ cudaError_t order_polygons(const Dev &d, bool layered, SortScratch &s, cudaStrea
 // enqueues kernels on `st`.
 cudaError_t stage_prepare(const Dev &d, SortScratch &s, TreeBuffers &source_tree,
                           TreeBuffers &seg_tree, cudaStream_t st);
+cudaError_t stage_lists(const Dev &d, cudaStream_t st);
 cudaError_t stage_step(const Dev &d, cudaStream_t st);
 cudaError_t stage_rank(const Dev &d, SortScratch &s, cudaStream_t st);
 cudaError_t stage_mesh(const Dev &d, SortScratch &s, TreeBuffers &point_tree, cudaStream_t st);

@@ -387,35 +387,6 @@ __global__ void k_segment_compact(Dev d) {
   }
 }
 
-// Seed the frontier with every projected source, in source order; empty
-// sources keep size 0 and are skipped by the subdivision (frontier.py:15-42).
-__global__ void k_seed(Dev d) {
-  const bool fits = int64_t(d.n) <= d.cap.frontier;
-  for (int64_t i = tid(); fits && i < d.n; i += stride()) {
-    int n = d.status[kError] == 0 ? d.src_n[i] : 0;
-    V2 *dst = d.fv[0] + int64_t(kMaxVertices) * i;
-    const V2 *src = d.src_v + kSourceVertices * i;
-    for (int j = 0; j < n; ++j) dst[j] = src[j];
-    d.fn[0][i] = n;
-    d.fsrc[0][i] = int(i);
-    d.fcur[0][i] = 0;  // first contour leaf not yet met
-  }
-  if (tid() == 0) {
-    if (!fits) set_error(d.status, kErrResidual);
-    d.status[kResidual] = fits ? d.n : 0;
-    d.status[kPeakResidual] = d.status[kResidual];
-    d.sc[kFrontierNext] = 0;
-    d.sc[kDeferred] = 0;
-    d.sc[kDeferredNext] = 0;
-  }
-}
-
-__global__ void k_loop_condition(Dev d) {
-  int c = d.status[kResidual] > 0 && d.status[kError] == 0;
-  *d.condition = c;
-  if (d.use_handle) cudaGraphSetConditional(d.cond_handle, unsigned(c));
-}
-
 unsigned blocks(int64_t n) {
   int64_t g = ceil_div(n > 0 ? n : 1, kBlock);
   return unsigned(g < 148 * 16 ? g : 148 * 16);
@@ -425,7 +396,7 @@ unsigned blocks(int64_t n) {
 
 cudaError_t stage_prepare_common(const Dev &d, SortScratch &s, TreeBuffers &source_tree,
                                  cudaStream_t st) {
-  k_reset<<<1, 32, 0, st>>>(d);
+  k_reset<<<1, 64, 0, st>>>(d);
   note_launch();
   EDP_CHECK(cudaMemsetAsync(d.weld_table, 0xff, sizeof(int) * (int64_t(d.weld_mask) + 1), st));
   EDP_CHECK(cudaMemsetAsync(d.weld_min, 0x7f, sizeof(int) * (int64_t(d.weld_mask) + 1), st));
@@ -472,11 +443,7 @@ cudaError_t stage_prepare(const Dev &d, SortScratch &s, TreeBuffers &source_tree
     note_launch();
   }
   EDP_CHECK(tree_build(seg_tree, d.seg_lo, d.seg_hi, d.sc + kSegmentCount, 0, false, s, st));
-  k_seed<<<blocks(d.n), kBlock, 0, st>>>(d);
-  note_launch();
-  k_loop_condition<<<1, 1, 0, st>>>(d);
-  note_launch();
-  return cudaGetLastError();
+  return stage_lists(d, st);
 }
 
 }  // namespace edp

@@ -196,6 +196,12 @@ cudaError_t allocate_event(edp_peeler *p) {
   EDP_CHECK(alloc(p, &d.seg_srcb, int64_t(d.seg_mask) + 1));
   EDP_CHECK(alloc(p, &d.seg_table, int64_t(d.seg_mask) + 1));
   EDP_CHECK(alloc(p, &d.seg_min, int64_t(d.seg_mask) + 1));
+  // Candidate lists hold a handful of segments per source on average; sources
+  // past the pool walk the contour hierarchy instead.
+  d.cand_cap = 24 * n + 4096;
+  EDP_CHECK(alloc(p, &d.cand, d.cand_cap));
+  EDP_CHECK(alloc(p, &d.cand_start, n));
+  EDP_CHECK(alloc(p, &d.cand_count, n));
   for (int k = 0; k < 2; ++k) {
     EDP_CHECK(alloc(p, &d.fv[k], F * kMaxVertices));
     EDP_CHECK(alloc(p, &d.fn[k], F));

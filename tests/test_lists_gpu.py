@@ -1,0 +1,93 @@
+"""The subdivision's candidate lists and lane groups where they end: convex
+patches of up to 30 vertices (a group holds 8), lists longer than a warp's
+buffer, and sources whose lists do not fit the pool and walk the hierarchy."""
+
+import math
+from dataclasses import replace
+
+import numpy as np
+import pytest
+import parity
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+FORMS = ["filtered64", "filtered", "binary64"]
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _device():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+
+
+def polygon_over_triangle(sides):
+    """A triangulated regular polygon in front of one large triangle, whose
+    middle patch takes the polygon's shape."""
+    angles = 2.0 * math.pi * (np.arange(sides) + 0.25) / sides
+    rim = np.stack([0.5 * np.cos(angles), 0.5 * np.sin(angles), np.ones(sides)], 1)
+    v = np.concatenate([rim, [[0.01, 0.02, 1.0]], [[-3.0, -2.0, 2.0], [3.0, -2.0, 2.0],
+                                                   [0.0, 4.0, 2.0]]])
+    f = [(j, (j + 1) % sides, sides) for j in range(sides)] + [(sides + 1, sides + 2, sides + 3)]
+    return (v, np.array(f, dtype=np.int32), np.eye(4),
+            np.array([-1.0, -1.0, 1.0, 1.0, 0.0, 0.01]))
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("sides", [8, 9, 16, 30])
+def test_many_sided_patches_against_the_oracle(sides, form):
+    from peel_b200 import EventCapacities, EventPeeler, scenes
+
+    arrays = polygon_over_triangle(sides)
+    p = EventPeeler(*scenes.to_device(arrays), predicates=form,
+                    capacities=replace(EventCapacities.for_mesh(256), layers=64))
+    p.run()
+    parity.check_against_oracle(p, parity.exact_scene_of(*arrays), range(sides + 1))
+    assert max(len(v) for _, _, v in parity.polygons(p)) >= sides
+
+
+def tiles_over_sheets(side, sheets):
+    """side x side small disjoint triangles in front of ``sheets`` large
+    triangles: every sheet's list holds every tile's edges."""
+    i, j = np.meshgrid(np.arange(side), np.arange(side), indexing="ij")
+    step = 1.0 / side
+    # Uneven sizes, so that no two tile edges lie on one line.
+    size = step * (0.3 + 0.2 * np.random.default_rng(1).uniform(size=(side, side, 3, 2)))
+    corner = np.array([[0.0, 0.0], [1.0, 0.0], [0.0, 1.0]])
+    xy = -0.5 + step * np.stack([i, j], -1)[:, :, None, :] + size + corner * (0.4 * step)
+    tiles = np.concatenate([xy, np.ones((side, side, 3, 1))], -1).reshape(-1, 3)
+    big = [[[-3.0, -2.0, 2.0 + k], [3.0, -2.0, 2.0 + k], [0.0, 4.0, 2.0 + k]]
+           for k in range(sheets)]
+    v = np.concatenate([tiles, np.array(big).reshape(-1, 3)])
+    return (v, np.arange(len(v), dtype=np.int32).reshape(-1, 3), np.eye(4),
+            np.array([-1.0, -1.0, 1.0, 1.0, 0.0, 0.01]))
+
+
+# 3 side^2 segments per sheet against a pool of 24 (side^2 + sheets) + 4096:
+# one sheet's list above the 192 buffered entries, and 40 sheets' lists above
+# the pool.
+@pytest.mark.parametrize("form", ["filtered64", "binary64"])
+@pytest.mark.parametrize("side,sheets", [(10, 1), (20, 40)])
+def test_long_lists_and_sources_without_one(side, sheets, form):
+    from peel_b200 import EventCapacities, scenes
+    from peel_b200.sizing import fit_event_capacities
+
+    arrays = tiles_over_sheets(side, sheets)
+    n = len(arrays[1])
+    p, _ = fit_event_capacities(scenes.to_device(arrays), EventCapacities.for_mesh(16 * n),
+                                attempts=12, predicates=form)
+    info = p.read_status()
+    assert info["layers"] == sheets + 1
+    corners = arrays[0][arrays[1]][:, :, :2] * 0.5
+    u, w = corners[:, 1] - corners[:, 0], corners[:, 2] - corners[:, 0]
+    tiles = 0.5 * (u[:, 0] * w[:, 1] - u[:, 1] * w[:, 0])[: side * side]
+    areas = parity.gpu_areas(parity.polygons(p), range(n))
+    covered = float(tiles.sum())
+    for s in range(side * side):
+        assert abs(areas[(0, s)] - tiles[s]) <= 1e-9
+    for k in range(sheets):  # the window shows a sheet's whole unit square
+        s = side * side + k
+        whole = areas[(k, s)] + areas[(k + 1, s)]
+        assert abs(areas[(k + 1, s)] - covered) <= 1e-9
+        assert abs(whole - areas[(0, n - sheets)] - areas[(1, n - sheets)]) <= 1e-9
+        assert {key for key in areas if key[1] == s} == {(k, s), (k + 1, s)}
