@@ -4,6 +4,7 @@
 // (warp_peel/kernels.py:941-1204, events.py:720-780).
 #include "../../include/edp.h"
 #include "edp_internal.h"
+#include "edp_warp.cuh"
 
 namespace edp {
 namespace {
@@ -176,9 +177,9 @@ __device__ inline void lift(const Dev &d, V2 x, const Plane &s, double *w) {
 // acceptance test and therefore the triangles are the same.
 constexpr int kPolygonSplits = 256;  // split points buffered per polygon
 // Candidate points x edges above which a polygon is noded by a whole warp
-// (k_mesh_heavy) rather than by one thread, so that a few large polygons in
-// dense cells do not hold 31 idle lanes of a warp: Dev::heavy_noding_work
-// (1024 unless tuned).
+// (k_mesh_heavy) rather than by eight lanes, so that a few large polygons in
+// dense cells do not hold up the other groups of a warp:
+// Dev::heavy_noding_work (1024 unless tuned).
 
 // The centroid fan of polygon p (n vertices, centroid `center`) through its
 // split points sorted by (edge, parameter).  Counts the fan triangles (signed
@@ -251,7 +252,10 @@ __device__ inline void emit_fan(const Dev &d, const V2 *p, int n, V2 center, int
   }
 }
 
+// Without the point grid (more layers than it has rows for), one thread per
+// polygon and one point-hierarchy query each.
 __global__ void __launch_bounds__(kBlock, 8) k_mesh_polygons(Dev d, int edge_capacity) {
+  if (d.sc[kGridOn] != 0) return;
   const int live = d.sc[kLivePolygons];
   const int leaves = *d.point_tree.size;
   double split_t[kPolygonSplits];
@@ -274,24 +278,6 @@ __global__ void __launch_bounds__(kBlock, 8) k_mesh_polygons(Dev d, int edge_cap
                                   float(layer), 0.f);
     const float4 hi = make_float4(__double2float_ru(hx + 2.0e-7), __double2float_ru(hy + 2.0e-7),
                                   float(layer), 0.f);
-    // The grid cells meeting the polygon's box grown by 1e-9 hold every
-    // same-layer point within 1e-10 of its boundary, hence every split point.
-    const bool grid = d.sc[kGridOn] != 0;
-    const int g = d.point_grid;
-    const double qlx = lx - 1.0e-9, qly = ly - 1.0e-9, qhx = hx + 1.0e-9, qhy = hy + 1.0e-9;
-    const int cx0 = grid_cell(qlx, g), cx1 = grid_cell(qhx, g);
-    const int cy0 = grid_cell(qly, g), cy1 = grid_cell(qhy, g);
-    if (grid) {
-      int64_t candidates = 0;
-      for (int cy = cy0; cy <= cy1; ++cy) {
-        const int64_t row = (int64_t(layer) * g + cy) * g;
-        candidates += d.cell_start[row + cx1 + 1] - d.cell_start[row + cx0];
-      }
-      if (candidates * n > d.heavy_noding_work) {
-        d.heavy_polygons[atomicAdd(&d.sc[kHeavyPolygons], 1)] = int(i);
-        continue;
-      }
-    }
     int count = 0, per_edge[kMaxVertices];
     for (int e = 0; e < n; ++e) per_edge[e] = 0;
     bool overflow = false;
@@ -321,24 +307,12 @@ __global__ void __launch_bounds__(kBlock, 8) k_mesh_polygons(Dev d, int edge_cap
         }
       }
     };
-    if (grid) {
-      for (int cy = cy0; cy <= cy1 && !overflow; ++cy) {
-        const int64_t row = (int64_t(layer) * g + cy) * g;
-        const int end = d.cell_start[row + cx1 + 1];
-        for (int j = d.cell_start[row + cx0]; j < end && !overflow; ++j) {
-          const V2 x = d.grid_pts[j];
-          if (x.x < qlx || x.x > qhx || x.y < qly || x.y > qhy) continue;
-          node_point(x);
-        }
-      }
-    } else {
-      int node = 1;
-      while (node > 0 && !overflow) {
-        int j;
-        node = query_next(d.point_tree, leaves, lo, hi, node, 0, j);
-        if (j < 0) break;
-        node_point(d.uverts[j]);
-      }
+    int node = 1;
+    while (node > 0 && !overflow) {
+      int j;
+      node = query_next(d.point_tree, leaves, lo, hi, node, 0, j);
+      if (j < 0) break;
+      node_point(d.uverts[j]);
     }
     if (overflow) {
       set_error(d.status, kErrEdgeNoding);
@@ -361,7 +335,267 @@ __global__ void __launch_bounds__(kBlock, 8) k_mesh_polygons(Dev d, int edge_cap
   }
 }
 
-// One polygon edge as the split-point test of k_mesh_polygons uses it, with
+// Noding and emission with the point grid, eight lanes per polygon, four
+// polygons per warp in step.  A lane owns a polygon edge.  The rows of grid
+// cells meeting the polygon's box grown by 1e-9 hold every same-layer point
+// within 1e-10 of its boundary, hence every split point; eight of their points
+// are loaded at a time, the box rejects most, and the ones left wait until
+// there are eight to test, a point per lane, against every edge.  A lane keeps its
+// edge's split points in order, so the fan needs no sort: a lane writes its
+// edge's triangles, the lanes' counts are scanned in edge order, and a warp's
+// triangles are staged in shared memory and written as one run.
+// Polygons of more than eight vertices, with more than Dev::heavy_noding_work
+// candidate x edge tests, or with more than kEdgeSplits points on an edge go
+// to k_mesh_heavy, a warp each.
+//
+// Bound by instruction issue (about 10 of a polygon's 55 cell points lie in
+// its box).  A thread per polygon ran 4.6 of 32 lanes, which waited for the
+// one with the most candidates, and wrote 48- and 72-byte pieces.  Noding and
+// emission together: knot-65536 1.36 -> 0.87 ms, its 9,702-face relative 0.55
+// -> 0.13, 720K primitives 4.0 -> 3.45, 640-face icospheres 0.12 -> 0.035.
+// Testing each near point by all edges at once instead of eight at a time took
+// 1.01 ms on the knot.  6 blocks of 80 registers per SM: 4 and 5 hide less
+// latency (0.97 and 0.91 ms), 7 spill (1.22).  The line to the warp kernel at
+// 1024 tests: 512 takes 0.94 and 2048 takes 1.01 ms on the knot, 3.8 and 3.3
+// on the 720K primitives.
+constexpr int kLanes = 8;
+constexpr int kMeshGroups = kBlock / kLanes;
+constexpr int kEdgeSplits = 8;
+constexpr int kStaged = 32;  // triangles of one warp staged in shared memory
+constexpr int kNear = 16;    // points in a polygon's box that wait for their edge tests
+
+struct Staging {
+  V2 uv[3 * kStaged];
+  double world[9 * kStaged];
+  int src[kStaged], layer[kStaged];
+};
+
+__global__ void __launch_bounds__(kBlock, 6) k_mesh_groups(Dev d, int edge_capacity) {
+  __shared__ V2 s_a[kMeshGroups][kLanes], s_dir[kMeshGroups][kLanes];
+  __shared__ double s_slack[kMeshGroups][kLanes];
+  __shared__ V2 s_near[kMeshGroups][kNear];
+  __shared__ double s_t[kMeshGroups][kLanes][kEdgeSplits];
+  __shared__ Staging s_staging[kBlock / 32];
+  if (d.sc[kGridOn] == 0) return;
+  const Group<kLanes> w;
+  const int lane = threadIdx.x & 31, slot = threadIdx.x / kLanes;
+  double *split_t = s_t[slot][w.lane];
+  const V2 *edge_a = s_a[slot], *edge_dir = s_dir[slot];
+  const double *edge_slack = s_slack[slot];
+  V2 *waiting = s_near[slot];
+  Staging &out = s_staging[threadIdx.x / 32];
+  const int live = d.sc[kLivePolygons], g = d.point_grid;
+  for (int64_t k0 = tid() >> 5 << 2; k0 < live; k0 += stride() >> 5 << 2) {
+    if (__shfl_sync(kFull, *(volatile int *)&d.status[kError], 0) != 0) return;
+    const int64_t k = k0 + (lane >> 3);
+    const int i = k < live ? d.order[k] : 0;
+    int n = k < live ? d.out_n[i] : 0;
+    const int layer = d.out_layer[i], source = d.out_src[i];
+    if (n < 3) n = 0;
+    bool heavy = n > kLanes;
+    if (heavy) n = 0;
+    const bool mine = w.lane < n;
+    const V2 a = mine ? d.out_v[int64_t(kMaxVertices) * i + w.lane] : v2(0.0, 0.0);
+    const V2 b = w.shfl(a, w.lane + 1 < n ? w.lane + 1 : 0);
+    // Box, and the centroid summed in vertex order.
+    double lx = mine ? a.x : 1.0e30, ly = mine ? a.y : 1.0e30;
+    double hx = mine ? a.x : -1.0e30, hy = mine ? a.y : -1.0e30;
+    for (int off = kLanes / 2; off > 0; off >>= 1) {
+      lx = smaller(lx, w.shfl_xor(lx, off));
+      ly = smaller(ly, w.shfl_xor(ly, off));
+      hx = larger(hx, w.shfl_xor(hx, off));
+      hy = larger(hy, w.shfl_xor(hy, off));
+    }
+    waiting[w.lane] = a / double(n > 0 ? n : 1);
+    const V2 dir = b - a;
+    const double length2 = dot(dir, dir);
+    s_a[slot][w.lane] = a;
+    s_dir[slot][w.lane] = dir;
+    s_slack[slot][w.lane] = 4.0 * kEps * kEps * length2;
+    __syncwarp();
+    V2 center = v2(0.0, 0.0);
+    for (int j = 0; j < kLanes; ++j)
+      if (j < n) center = center + waiting[j];
+    __syncwarp();
+    const double qlx = lx - 1.0e-9, qly = ly - 1.0e-9, qhx = hx + 1.0e-9, qhy = hy + 1.0e-9;
+    const int cx0 = n ? grid_cell(qlx, g) : 0, cx1 = n ? grid_cell(qhx, g) : 0;
+    const int cy0 = n ? grid_cell(qly, g) : 0, cy1 = n ? grid_cell(qhy, g) : -1;
+    const int most = __reduce_max_sync(kFull, n);
+    int count = 0;       // this lane's edge's split points
+    bool full = false;   // more than kEdgeSplits of them
+    int candidates = 0;  // of the polygon, up to the current rows
+    int near_n = 0;      // points waiting
+    // Up to eight waiting points of each group, a point per lane: the edges
+    // whose line it lies on (4x slack over the exact test) and that it does
+    // not end (an edge's own end point has parameter 0 or 1 exactly: never a
+    // split).  The few found are then tested by the lanes that own the edges.
+    auto node_waiting = [&](bool take) {
+      const int points = take ? min(near_n, kLanes) : 0;
+      const V2 x = waiting[w.lane];
+      unsigned on = 0, end = 0;
+      for (int e = 0; e < most; ++e) {
+        const V2 u = edge_a[e], dir_e = edge_dir[e], to = x - u;
+        const double off = dir_e.x * to.y - dir_e.y * to.x;  // cross(a, b, x)
+        on |= unsigned(!(off * off > edge_slack[e])) << e;
+        end |= unsigned(x == u) << e;
+      }
+      if (n > 0) on &= ~(end | end >> 1 | (end & 1u) << (n - 1)) & ((1u << n) - 1u);
+      unsigned found = w.ballot(w.lane < points && on != 0);
+      while (__any_sync(kFull, found != 0)) {
+        const int c = found ? __ffs(int(found)) - 1 : 0;
+        const V2 y = w.shfl(x, c);
+        const unsigned edges = w.shfl(on, c);
+        if (found && (edges >> w.lane & 1u) && length2 > 0.0) {
+          const V2 to = y - a;
+          const double off = dir.x * to.y - dir.y * to.x;
+          const double tt = dot(to, dir) / length2;
+          if (tt > kEps && tt < 1.0 - kEps && fabs(off) <= kEps * sqrt(length2)) {
+            full = full || count == kEdgeSplits;
+            if (!full) {
+              int m = count++;
+              for (; m > 0 && split_t[m - 1] > tt; --m) split_t[m] = split_t[m - 1];
+              split_t[m] = tt;
+            }
+          }
+        }
+        found &= found - 1;
+      }
+      const V2 rest = waiting[kNear - kLanes + w.lane];
+      __syncwarp();
+      if (take) {
+        waiting[w.lane] = rest;
+        near_n -= points;
+      }
+      __syncwarp();
+    };
+    for (int row0 = cy0; __any_sync(kFull, row0 <= cy1); row0 += kLanes) {
+      // Eight rows, one per lane, and the scan of their point counts.
+      int begin = 0, points = 0;
+      if (row0 + w.lane <= cy1) {
+        const int64_t row = (int64_t(layer) * g + row0 + w.lane) * g;
+        begin = d.cell_start[row + cx0];
+        points = d.cell_start[row + cx1 + 1] - begin;
+      }
+      int before = points;
+      for (int off = 1; off < kLanes; off <<= 1) {
+        const int y = __shfl_up_sync(kFull, before, off, kLanes);
+        if (w.lane >= off) before += y;
+      }
+      int total = w.shfl(before, kLanes - 1);
+      before -= points;
+      candidates += total;
+      if (int64_t(candidates) * n > d.heavy_noding_work) heavy = true;
+      if (heavy) total = 0;
+      for (int t0 = 0; __any_sync(kFull, t0 < total); t0 += kLanes) {
+        const int t = t0 + w.lane;
+        int r = 0;  // the row that holds the t-th point: the last one that begins at or before t
+        for (int off = kLanes / 2; off > 0; off >>= 1)
+          if (w.shfl(before, r + off) <= t) r += off;
+        const int at = w.shfl(begin, r) + t - w.shfl(before, r);
+        V2 x = v2(0.0, 0.0);
+        bool near = t < total;
+        if (near) {
+          x = d.grid_pts[at];
+          near = !(x.x < qlx || x.x > qhx || x.y < qly || x.y > qhy);
+        }
+        const unsigned nears = w.ballot(near);
+        if (near) waiting[near_n + __popc(nears & ((1u << w.lane) - 1u))] = x;
+        near_n += __popc(nears);
+        __syncwarp();
+        if (__any_sync(kFull, near_n >= kLanes)) node_waiting(near_n >= kLanes);
+      }
+    }
+    if (__any_sync(kFull, near_n > 0)) node_waiting(true);
+    if (w.ballot(full)) heavy = true;
+    if (heavy && w.lane == 0) d.heavy_polygons[atomicAdd(&d.sc[kHeavyPolygons], 1)] = i;
+    const bool over = !heavy && mine && count > edge_capacity;
+    if (__any_sync(kFull, over)) {
+      if (over) set_error(d.status, kErrEdgeNoding);
+      return;
+    }
+    // The fan of emit_fan() with a lane per edge.
+    const bool active = mine && !heavy;
+    int emitted = 0;
+    if (active) {
+      double previous = 0.0;
+      V2 cursor = a;
+      for (int m = 0; m <= count; ++m) {
+        const double following = m == count ? 1.0 : split_t[m];
+        if (following > previous + kEps) {
+          const V2 next = a + following * dir;
+          if (cross(center, cursor, next) > kEps * kEps) ++emitted;
+          cursor = next;
+          previous = following;
+        }
+      }
+    }
+    int offset = emitted;
+    for (int off = 1; off < 32; off <<= 1) {
+      const int y = __shfl_up_sync(kFull, offset, off);
+      if (lane >= off) offset += y;
+    }
+    const int total = __shfl_sync(kFull, offset, 31);
+    offset -= emitted;
+    int base = 0;
+    if (lane == 0 && total) base = atomicAdd(&d.status[kTriangles], total);
+    base = __shfl_sync(kFull, base, 0);
+    if (int64_t(base) + total > d.cap.triangles) {
+      if (lane == 0) set_error(d.status, kErrTriangles);
+      return;
+    }
+    const bool staged = total <= kStaged;
+    V2 *uvs = staged ? out.uv : d.tri_uv + 3 * int64_t(base);
+    double *worlds = staged ? out.world : d.tri_world + 9 * int64_t(base);
+    int *srcs = staged ? out.src : d.tri_src + base, *layers = staged ? out.layer : d.tri_layer + base;
+    if (active) {
+      const Plane sc = d.scores[source];
+      double w_center[3], w_cursor[3];
+      lift(d, center, sc, w_center);
+      lift(d, a, sc, w_cursor);
+      double previous = 0.0;
+      V2 cursor = a;
+      int at = offset;
+      for (int m = 0; m <= count; ++m) {
+        const double following = m == count ? 1.0 : split_t[m];
+        if (following > previous + kEps) {
+          const V2 next = a + following * dir;
+          double w_next[3];
+          lift(d, next, sc, w_next);
+          if (cross(center, cursor, next) > kEps * kEps) {
+            V2 *uv = uvs + 3 * at;
+            double *v = worlds + 9 * at;
+            uv[0] = center;
+            uv[1] = cursor;
+            uv[2] = next;
+            for (int c = 0; c < 3; ++c) {
+              v[c] = w_center[c];
+              v[3 + c] = w_cursor[c];
+              v[6 + c] = w_next[c];
+            }
+            srcs[at] = source;
+            layers[at] = layer;
+            ++at;
+          }
+          cursor = next;
+          for (int c = 0; c < 3; ++c) w_cursor[c] = w_next[c];
+          previous = following;
+        }
+      }
+    }
+    __syncwarp();
+    if (staged) {
+      for (int m = lane; m < 3 * total; m += 32) d.tri_uv[3 * int64_t(base) + m] = out.uv[m];
+      for (int m = lane; m < 9 * total; m += 32) d.tri_world[9 * int64_t(base) + m] = out.world[m];
+      for (int m = lane; m < total; m += 32) {
+        d.tri_src[base + m] = out.src[m];
+        d.tri_layer[base + m] = out.layer[m];
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// One polygon edge as the split-point test uses it, with
 // the quantities that test derives from the edge computed once.
 struct NodeEdge {
   V2 a, b, dir;
@@ -370,7 +604,7 @@ struct NodeEdge {
 
 constexpr int kHeavyWarps = kBlock / 32;
 
-// Noding and emission of the polygons k_mesh_polygons queued as heavy, one
+// Noding and emission of the polygons k_mesh_groups queued as heavy, one
 // polygon per warp.  Lanes take the polygon's grid candidates 32 at a time
 // and test each against every edge with the thread kernel's expressions, so
 // the split points are the same.  Each split point is placed by its edge and
@@ -607,6 +841,9 @@ cudaError_t stage_mesh_index(const Dev &d, SortScratch &s, TreeBuffers &point_tr
 cudaError_t stage_mesh_emit(const Dev &d, cudaStream_t st) {
   int cap = int(d.cap.edge_vertices < kMaxEdgeVertices ? d.cap.edge_vertices : kMaxEdgeVertices);
   EDP_CHECK(cudaMemsetAsync(d.sc + kHeavyPolygons, 0, sizeof(int), st));
+  k_mesh_groups<<<unsigned(std::min<int64_t>(ceil_div(d.cap.regions, kMeshGroups), 148 * 6)),
+                  kBlock, 0, st>>>(d, cap);
+  note_launch();
   k_mesh_polygons<<<blocks(d.cap.regions), kBlock, 0, st>>>(d, cap);
   note_launch();
   k_mesh_heavy<<<148 * 5, kBlock, 0, st>>>(d, cap);
