@@ -89,7 +89,7 @@ struct Caps {
   int64_t frontier, regions, hits, vertices, triangles, rounds, layers, edge_vertices;
 };
 
-constexpr int kRayCells = 16;  // most source-grid cells one source is listed in
+constexpr int kRayCells = 16;  // most source-grid cells one source is listed in, at least
 constexpr int kSegCells = 4;   // most segment-grid cells one contour segment is listed in
 
 // Device scalars kept between kernels of one extraction.
@@ -253,10 +253,12 @@ struct Dev {
   int point_grid, grid_layers;
   int grid_size;  // cells per axis of the source and segment grids
   // Source grid for rays (EventPeeler): grid_size x grid_size cells over the
-  // window, listing each source whose box (grown by 1e-6) meets at most kRayCells of
-  // them; larger sources in ray_big.  leaf_of: each source's leaf in the
+  // window, listing each source whose box (grown by 1e-6) meets at most ray_cells of
+  // them, with its box (lo.x, lo.y, hi.x, hi.y); larger sources in ray_big.  leaf_of: each source's leaf in the
   // source hierarchy.
   int *ray_count, *ray_start, *ray_entries, *ray_big, *leaf_of;
+  float4 *ray_boxes, *ray_edges;  // ray_edges: three binary32 edge functions per source
+  int ray_cells;                  // most cells one source is listed in
   // Contour segment grid for the connection test: distinct segments listed in
   // the cells their box (grown by 1e-6) meets, at most kSegCells each.
   int *seg_count, *seg_start, *seg_entries, *seg_big;

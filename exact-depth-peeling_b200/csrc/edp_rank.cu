@@ -7,6 +7,7 @@
 #include "../../include/edp.h"
 #include "edp_filtered.cuh"
 #include "edp_internal.h"
+#include "edp_warp.cuh"
 
 namespace edp {
 namespace {
@@ -557,11 +558,42 @@ __device__ inline bool source_cells(const Dev &d, int s, int &cx0, int &cx1, int
   return true;
 }
 
+// A triangle's edge functions in binary32: e(x) = A x + B y + C, positive
+// inside, and a bound on its error.  A, B and C carry a relative error of u =
+// 2^-24 each, the point's coordinates and the products u, and the two sums u
+// of their terms, in all at most 6 u (|A| + |B| + |C|) for a point of the
+// unit window; the bound is 8 u.  Sources that are not triangles get the zero
+// function, which excludes nothing.
+__device__ inline void edge_functions(const Dev &d, int64_t s) {
+  const V2 *p = d.src_v + int64_t(kSourceVertices) * s;
+  const bool triangle = d.src_n[s] == 3;
+  for (int j = 0; j < 3; ++j) {
+    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (triangle) {
+      const V2 a = p[j], b = p[(j + 1) % 3];
+      const double ea = a.y - b.y, eb = b.x - a.x, ec = -(ea * a.x + eb * a.y);
+      f = make_float4(float(ea), float(eb), float(ec),
+                      -float(8.0 * double(pred::kU32) * (fabs(ea) + fabs(eb) + fabs(ec))));
+    }
+    d.ray_edges[3 * s + j] = f;
+  }
+}
+
+// The point certainly lies outside an edge of source s, so the source does
+// not contain it in any predicate form.  Nine of ten candidates end here.
+__device__ inline bool edges_exclude(const Dev &d, int s, float x, float y) {
+  const float4 *f = d.ray_edges + 3 * int64_t(s);
+  const float4 a = f[0], b = f[1], c = f[2];
+  return a.x * x + a.y * y + a.z < a.w || b.x * x + b.y * y + b.z < b.w ||
+         c.x * x + c.y * y + c.z < c.w;
+}
+
 __global__ void k_ray_grid_count(Dev d) {
   for (int64_t s = tid(); s < d.n; s += stride()) {
+    edge_functions(d, s);
     int cx0, cx1, cy0, cy1;
     if (!source_cells(d, int(s), cx0, cx1, cy0, cy1)) continue;
-    if ((cx1 - cx0 + 1) * (cy1 - cy0 + 1) > kRayCells) {
+    if ((cx1 - cx0 + 1) * (cy1 - cy0 + 1) > d.ray_cells) {
       d.ray_big[reserve(&d.sc[kRayBig], 1)] = int(s);
       continue;
     }
@@ -577,11 +609,15 @@ __global__ void k_ray_grid_fill(Dev d) {
   for (int64_t s = tid(); s < d.n; s += stride()) {
     int cx0, cx1, cy0, cy1;
     if (!source_cells(d, int(s), cx0, cx1, cy0, cy1)) continue;
-    if ((cx1 - cx0 + 1) * (cy1 - cy0 + 1) > kRayCells) continue;
+    if ((cx1 - cx0 + 1) * (cy1 - cy0 + 1) > d.ray_cells) continue;
+    const float4 lo = d.src_lo[s], hi = d.src_hi[s];
+    const float4 box = make_float4(lo.x, lo.y, hi.x, hi.y);
     for (int cy = cy0; cy <= cy1; ++cy)
       for (int cx = cx0; cx <= cx1; ++cx) {
         const int c = cy * d.grid_size + cx;
-        d.ray_entries[d.ray_start[c] + atomicSub(&d.ray_count[c], 1) - 1] = int(s);
+        const int e = d.ray_start[c] + atomicSub(&d.ray_count[c], 1) - 1;
+        d.ray_entries[e] = int(s);
+        d.ray_boxes[e] = box;
       }
   }
 }
@@ -618,13 +654,182 @@ struct HitBuffer {
   }
 };
 
-// One ray per group leader: up to kCandidatesPerPass sources, the rest of the
-// traversal is queued for the persistent continuation (event_kernels.py:196-245).
+// Rays over the source grid, eight lanes per ray, four rays per warp in step.
+// Every source whose box meets the ray's query box is listed in the point's
+// cell (or among the big ones).  The lanes read eight entries and their boxes
+// at a time (both contiguous in the cell); the sources whose box meets the
+// query box are the hierarchy's candidates.  The ones that edges_exclude
+// leaves wait in shared memory until there are eight to test for containment,
+// a source per lane.  The hits of a ray go to the shared pool with one
+// reservation per warp.
+//
+// Up to kGroupRays polygons the bound is the latency of one ray's chain of
+// loads, which eight lanes shorten; above it there are threads enough to hide
+// it, and a thread per ray (k_ray_hits) issues fewer instructions.  A thread
+// per ray against this: 9,702-face knot 0.14 and 0.045 ms, 2,560-face
+// icospheres 0.071 and 0.020, 165K polygons of a resolved scene 0.231 and
+// 0.213; but 424K polygons of the 65,536-face knot 0.36 and 0.48, 2.2M of the
+// 720K primitives 1.67 and 2.02.  Before the binary32 edge test and the boxes
+// by entry those two took 0.49 and 2.03 ms, and the 9,702-face knot, whose
+// larger sources kept its rays out of the grid, 0.32.
+constexpr int kRayLanes = 8;
+constexpr int kRaysPerBlock = kBlock / kRayLanes;
+constexpr int kRayQueue = 16;  // candidates waiting for their containment test
+constexpr int kRayHeld = 64;   // hits held per ray before they go to the pool
+constexpr int kGroupRays = 262144;  // most live polygons whose rays take eight lanes each
+
+template <int F>
+__global__ void __launch_bounds__(kBlock) k_ray_groups(Dev d) {
+  __shared__ int s_queue[kRaysPerBlock][kRayQueue];
+  __shared__ int s_source[kRaysPerBlock][kRayHeld];
+  __shared__ double s_depth[kRaysPerBlock][kRayHeld];
+  if (d.sc[kRayGridOn] == 0 || live_polygons(d) > kGroupRays) return;
+  const Group<kRayLanes> w;
+  const int lane = threadIdx.x & 31, slot = threadIdx.x / kRayLanes;
+  const unsigned below = (1u << w.lane) - 1u;
+  int *queue = s_queue[slot], *held_source = s_source[slot];
+  double *held_depth = s_depth[slot];
+  const int live = live_polygons(d), g = d.grid_size, big = d.sc[kRayBig];
+  const int leaves = *d.source_tree.size;
+  int groups = 0, heavy_rays = 0;
+  long long tests = 0;
+  Tally contain;
+  for (int64_t k0 = tid() >> 5 << 2; k0 < live; k0 += stride() >> 5 << 2) {
+    if (__shfl_sync(kFull, *(volatile int *)&d.status[kError], 0) != 0) return;
+    const int64_t k = k0 + (lane >> 3);
+    const int i = k < live ? d.order[k] : -1;  // spatial order: neighbouring rays share cells
+    const bool leader = i >= 0 && d.groups[i] == i;
+    if (!__any_sync(kFull, leader)) continue;
+    const V2 x = leader ? d.samples[i] : v2(0.0, 0.0);
+    const float lx = lower_f(x.x - 2.0e-7), ly = lower_f(x.y - 2.0e-7);
+    const float hx = upper_f(x.x + 2.0e-7), hy = upper_f(x.y + 2.0e-7);
+    const float fx = float(x.x), fy = float(x.y);
+    const int c = ray_cell(x.y, g) * g + ray_cell(x.x, g);
+    const int begin = d.ray_start[c], listed = d.ray_start[c + 1] - begin;
+    const int total = leader ? listed + big : 0;
+    int met = 0, found = 0, held = 0, queued = 0;
+    // Move the held hits of the groups that `want` it to the pool.
+    auto flush = [&](bool want) {
+      const int count = want ? held : 0;
+      int at = w.lane == 0 ? count : 0;  // scan over the warp's four groups
+      for (int off = kRayLanes; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(kFull, at, off);
+        if (lane >= off) at += y;
+      }
+      const int all = __shfl_sync(kFull, at, 24);
+      const int mine = w.shfl(at, 0) - count;
+      unsigned long long base = 0;
+      if (lane == 0 && all)
+        base = atomicAdd(reinterpret_cast<unsigned long long *>(&d.metrics[kRayHits]),
+                         (unsigned long long)all);
+      const long long to = (long long)__shfl_sync(kFull, base, 0) + mine;
+      if (to + count > d.cap.hits) {
+        set_error(d.status, kErrHits);
+      } else {
+        for (int m = w.lane; m < count; m += kRayLanes) {
+          d.hit_depth[to + m] = held_depth[m];
+          d.hit_src[to + m] = held_source[m];
+          d.hit_group[to + m] = i;
+        }
+      }
+      __syncwarp();
+      if (want) held = 0;
+    };
+    // Containment of up to eight waiting candidates of the groups that `take`.
+    auto test_queue = [&](bool take) {
+      const int count = take ? min(queued, kRayLanes) : 0;
+      const bool mine = w.lane < count;
+      const int s = queue[w.lane];
+      bool hit = false;
+      if (mine) {
+        const int inside = contains_form<F>(d, s, x, contain);
+        if (F == 4 && inside == pred::kUndecided)
+          defer_contains(d, i, s);
+        else
+          hit = inside != 0;
+      }
+      const unsigned hits = w.ballot(hit);
+      if (hit) {
+        const int m = held + __popc(hits & below);
+        held_source[m] = s;
+        held_depth[m] = value(d.scores[s], x);
+      }
+      held += __popc(hits);
+      found += __popc(hits);
+      const int rest = queue[kRayQueue - kRayLanes + w.lane];
+      __syncwarp();
+      if (take) {
+        queue[w.lane] = rest;
+        queued -= count;
+      }
+      __syncwarp();
+      const bool filled = held > kRayHeld - kRayLanes;
+      if (__any_sync(kFull, filled)) flush(filled);
+    };
+    for (int t0 = 0; __any_sync(kFull, t0 < total); t0 += kRayLanes) {
+      const int t = t0 + w.lane;
+      bool meets = false;
+      int s = 0;
+      if (t < total) {
+        float4 box;
+        if (t < listed) {
+          s = d.ray_entries[begin + t];
+          box = d.ray_boxes[begin + t];
+        } else {
+          s = d.ray_big[t - listed];
+          const float4 lo = d.src_lo[s], hi = d.src_hi[s];
+          box = make_float4(lo.x, lo.y, hi.x, hi.y);
+        }
+        meets = box.x <= hx && box.y <= hy && box.z >= lx && box.w >= ly;
+      }
+      met += __popc(w.ballot(meets));
+      if (meets) meets = !edges_exclude(d, s, fx, fy);
+      const unsigned left = w.ballot(meets);
+      if (meets) queue[queued + __popc(left & below)] = s;
+      queued += __popc(left);
+      __syncwarp();
+      const bool ready = queued >= kRayLanes;
+      if (__any_sync(kFull, ready)) test_queue(ready);
+    }
+    if (__any_sync(kFull, queued > 0)) test_queue(true);
+    if (__any_sync(kFull, held > 0)) flush(true);
+    // A ray the binary walk's primary pass would leave unfinished: more than
+    // kCandidatesPerPass candidates, or that many with leaves after the last.
+    bool heavy = met > kCandidatesPerPass;
+    if (__any_sync(kFull, met == kCandidatesPerPass)) {
+      int last = -1;
+      for (int t = w.lane; met == kCandidatesPerPass && t < total; t += kRayLanes) {
+        const int s = t < listed ? d.ray_entries[begin + t] : d.ray_big[t - listed];
+        const float4 lo = d.src_lo[s], hi = d.src_hi[s];
+        if (lo.x <= hx && lo.y <= hy && hi.x >= lx && hi.y >= ly) last = max(last, d.leaf_of[s]);
+      }
+      for (int off = kRayLanes / 2; off > 0; off >>= 1) last = max(last, w.shfl_xor(last, off));
+      heavy = heavy || (met == kCandidatesPerPass && last != leaves - 1);
+    }
+    if (leader && w.lane == 0) {
+      d.group_counts[i] = found;
+      ++groups;
+      tests += met;
+      heavy_rays += heavy;
+    }
+  }
+  count_add(&d.metrics[kRayGroups], groups);
+  count_add(&d.metrics[kRayCandidateTests], tests);
+  count_add(&d.metrics[kHeavyRayGroups], heavy_rays);
+  if constexpr (F == 2) contain.flush(d, kPredContain);
+}
+
+// One ray per thread.  With the grid, for more rays than k_ray_groups takes:
+// neighbouring rays fill the lanes with like work, and a ray costs the fewest
+// instructions.  Without it (many large sources), over the source hierarchy:
+// up to kCandidatesPerPass sources, the rest of the traversal is queued for
+// the persistent continuation (event_kernels.py:196-245).
 template <int F>
 __global__ void k_ray_hits(Dev d) {
   const int live = live_polygons(d);
   const int leaves = *d.source_tree.size;
   const bool grid = d.sc[kRayGridOn] != 0;
+  if (grid && live <= kGroupRays) return;  // k_ray_groups took them
   long long groups = 0, tests = 0, heavy_rays = 0;
   HitBuffer hits;
   Tally contain;
@@ -642,12 +847,23 @@ __global__ void k_ray_hits(Dev d) {
       // hierarchy's candidates, the whole ray in one pass.
       const int g = d.grid_size, c = ray_cell(x.y, g) * g + ray_cell(x.x, g);
       const int begin = d.ray_start[c], end = d.ray_start[c + 1], big = d.sc[kRayBig];
+      const float fx = float(x.x), fy = float(x.y);
       int met = 0, last = -1, found = 0;
       for (int e = begin; e < end + big; ++e) {
-        const int s = e < end ? d.ray_entries[e] : d.ray_big[e - end];
-        if (!overlaps(d.src_lo[s], d.src_hi[s], lo, hi)) continue;
+        int s;
+        float4 box;
+        if (e < end) {
+          s = d.ray_entries[e];
+          box = d.ray_boxes[e];
+        } else {
+          s = d.ray_big[e - end];
+          const float4 a = d.src_lo[s], b = d.src_hi[s];
+          box = make_float4(a.x, a.y, b.x, b.y);
+        }
+        if (!(box.x <= hi.x && box.y <= hi.y && box.z >= lo.x && box.w >= lo.y)) continue;
         ++met;
-        last = max(last, d.leaf_of[s]);
+        if (met <= kCandidatesPerPass) last = max(last, d.leaf_of[s]);
+        if (edges_exclude(d, s, fx, fy)) continue;
         const int inside = contains_form<F>(d, s, x, contain);
         if (F == 4 && inside == pred::kUndecided) {
           defer_contains(d, i, s);
@@ -1311,9 +1527,15 @@ cudaError_t stage_rank(const Dev &d, SortScratch &s, cudaStream_t st) {
   // Filtered binary64 predicates: the filter-only kernels, then exact passes
   // over what their filters left undecided (same results as form 3 alone).
   const bool split_exact = d.predicates == 3;
+  const unsigned ray_blocks =
+      unsigned(std::min<int64_t>(ceil_div(std::min<int64_t>(R, kGroupRays), kRaysPerBlock), 148 * 8));
   if (split_exact) {
+    k_ray_groups<4><<<ray_blocks, kBlock, 0, st>>>(d);
+    note_launch();
     k_ray_hits<4><<<blocks(R), kBlock, 0, st>>>(d);
   } else {
+    EDP_LAUNCH_FORM(d.predicates, k_ray_groups, ray_blocks, kBlock, st, d);
+    note_launch();
     EDP_LAUNCH_FORM(d.predicates, k_ray_hits, blocks(R), kBlock, st, d);
   }
   note_launch();

@@ -225,7 +225,13 @@ cudaError_t allocate_event(edp_peeler *p) {
     const int64_t cells = int64_t(d.grid_size) * d.grid_size;
     EDP_CHECK(alloc(p, &d.ray_count, cells));
     EDP_CHECK(alloc(p, &d.ray_start, cells + 1));
-    EDP_CHECK(alloc(p, &d.ray_entries, int64_t(kRayCells) * (n > 0 ? n : 1)));
+    // Small meshes have sources of many cells: up to 2^20 listings in all, so
+    // that their rays use the grid too.
+    d.ray_cells = int(std::min(cells, std::max<int64_t>(kRayCells, (int64_t(1) << 20) /
+                                                                       (n > 0 ? n : 1))));
+    EDP_CHECK(alloc(p, &d.ray_entries, int64_t(d.ray_cells) * (n > 0 ? n : 1)));
+    EDP_CHECK(alloc(p, &d.ray_boxes, int64_t(d.ray_cells) * (n > 0 ? n : 1)));
+    EDP_CHECK(alloc(p, &d.ray_edges, 3 * n));
     EDP_CHECK(alloc(p, &d.ray_big, n > 0 ? n : 1));
     EDP_CHECK(alloc(p, &d.leaf_of, n > 0 ? n : 1));
     EDP_CHECK(alloc(p, &d.seg_count, cells));
