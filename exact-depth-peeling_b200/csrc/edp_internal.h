@@ -36,27 +36,31 @@ inline unsigned grid_for(int64_t n, int block) {
 
 // ---------------------------------------------------------------- primitives
 // Scratch for scans and radix sorts, sized once for the largest pool.
+//
+// State of the one-launch scans and radix passes: published words, and
+// control[] = {next tile, blocks finished, epoch}.  Launches that share it run
+// one after another (one stream).
+struct LookBack {
+  unsigned long long *words;
+  int *control;
+  int *error;  // where a wait that runs out sets its error bit
+};
+
+constexpr int kSortPasses = 8;
+
 struct SortScratch {
-  int *hist = nullptr;     // [256][tiles]
-  int *totals = nullptr;   // [256]
-  int *partials = nullptr; // scan tile sums
+  int *hist = nullptr;     // [kSortPasses][256], zero between sorts
+  LookBack look_back{};
   int64_t tiles = 0;       // capacity in radix tiles
   int64_t scan_tiles = 0;  // capacity in scan tiles
 };
 
-// Exclusive scan of in[0, *count) into out; out[*count..capacity) untouched.
-// The total is written to *total.  Counts are read on the device.
-cudaError_t scan_exclusive(const int *in, int *out, const int *count, int64_t capacity,
-                           int *total, SortScratch &s, cudaStream_t st);
+// out = exclusive scan of in over *count elements; the total goes to `total`
+// when given.  `clear` zeroes `in` on the way.
+cudaError_t scan_exclusive(int *in, int *out, const int *count, int64_t capacity, int *total,
+                           SortScratch &s, cudaStream_t st, bool clear = false);
 
-// Stable LSD radix sort of (key, value) pairs over the first *count items
-// (device scalar); items at and after *count are left untouched.  `bits` is
-// the number of low key bits that can be non-zero.  The sorted pairs end in
-// keys/vals; keys_tmp/vals_tmp are scratch of the same capacity.
 cudaError_t sort_pairs_u64(uint64_t *keys, uint64_t *keys_tmp, int *vals, int *vals_tmp,
-                           const int *count, int64_t capacity, int bits, SortScratch &s,
-                           cudaStream_t st);
-cudaError_t sort_pairs_u32(uint32_t *keys, uint32_t *keys_tmp, int *vals, int *vals_tmp,
                            const int *count, int64_t capacity, int bits, SortScratch &s,
                            cudaStream_t st);
 

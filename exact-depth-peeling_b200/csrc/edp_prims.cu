@@ -2,8 +2,6 @@
 // the implicit-tree hierarchy build.  Counts are device scalars so that one
 // captured CUDA graph handles any live size up to the allocated capacity
 // (the role of the reference's conditional sort buckets, events.py:637-718).
-#include <cub/warp/warp_scan.cuh>
-
 #include "../../include/edp.h"
 #include "edp_internal.h"
 
@@ -39,120 +37,192 @@ __device__ inline int block_exclusive(int v, int *smem, int &total) {
   return r;
 }
 
+// ---------------------------------------------------------------- look-back
+// Scans and radix passes run as one launch each, by decoupled look-back
+// (Merrill and Garland 2016; Adinets and Merrill 2022 for the radix pass):
+// blocks take tiles in order from a ticket, publish their tile's sums, and add
+// up the published sums before it.  A tile waits only for tiles whose blocks
+// hold earlier tickets and publish without waiting, so every wait ends; each
+// is bounded all the same, and running out sets an error.
+//
+// A published word holds the sum, a state and the launch's epoch, so the words
+// need no clearing between launches.  The last block to finish gives the
+// ticket back and starts the next epoch.
+//
+// Three launches per scan and per pass (counts, their scan, the scatter) cost
+// small extractions mostly gaps between launches: 157 kernels outside the
+// subdivision loop, 83 now.  Replays: icospheres-640 0.81 -> 0.72 ms,
+// knot-9702 1.14 -> 1.03, a batch of 16 small scenes 3.44 -> 3.03.
+enum Published : unsigned { kNothing = 0, kSum = 1, kPrefix = 2 };
+constexpr int kPollLimit = 1 << 22;
+
+__device__ inline unsigned long long publish_word(unsigned epoch, unsigned state, int value) {
+  return (unsigned long long)(epoch << 2 | state) << 32 | unsigned(value);
+}
+
+// The word at `p` once it is of this epoch.
+__device__ inline unsigned long long await_word(const unsigned long long *p, unsigned epoch,
+                                                int *error) {
+  const volatile unsigned long long *v = p;
+  unsigned long long w = *v;
+  for (int polls = 0; unsigned(w >> 34) != epoch || (unsigned(w >> 32) & 3u) == kNothing; w = *v) {
+    if (++polls > kPollLimit) {
+      if (error) atomicOr(error, int(kErrOutput));
+      return publish_word(epoch, kPrefix, 0);
+    }
+  }
+  return w;
+}
+
+// This block's tile (shared by all its threads) and the launch's epoch.
+__device__ inline int take_tile(LookBack s, int *shared, unsigned &epoch) {
+  if (threadIdx.x == 0) shared[0] = atomicAdd(&s.control[0], 1);
+  epoch = *(volatile unsigned *)&s.control[2] & 0x3fffffffu;
+  __syncthreads();
+  return shared[0];
+}
+
+// Counts the block as finished; true in thread 0 of the launch's last block,
+// after the state is ready for the next launch.
+__device__ inline bool finish_tile(LookBack s, int tiles) {
+  __syncthreads();
+  if (threadIdx.x != 0) return false;
+  __threadfence();
+  if (atomicAdd(&s.control[1], 1) != tiles - 1) return false;
+  s.control[0] = 0;
+  s.control[1] = 0;
+  s.control[2] = s.control[2] + 1;
+  return true;
+}
+
 // ---------------------------------------------------------------- scan
-__global__ void k_scan_reduce(const int *__restrict__ in, const int *count, int *partials) {
+// Exclusive scan in one launch and one pass over memory; `clear` zeroes the
+// input behind itself (counters for the next extraction).
+__global__ void __launch_bounds__(256)
+k_scan(int *in, int *out, const int *count, LookBack s, int *total_out, int clear) {
   __shared__ int smem[33];
+  __shared__ int s_tile[1], s_before;
   const int n = *count;
-  const int64_t base = int64_t(blockIdx.x) * kScanTile;
-  if (base >= n) return;
-  int sum = 0;
-  for (int k = threadIdx.x; k < kScanTile; k += blockDim.x) {
-    int64_t i = base + k;
-    if (i < n) sum += in[i];
+  if (n == 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && total_out) *total_out = 0;
+    return;
   }
-  int total;
-  block_exclusive(sum, smem, total);
-  if (threadIdx.x == 0) partials[blockIdx.x] = total;
-}
-
-__global__ void k_scan_partials(int *partials, const int *count) {
-  __shared__ int smem[33];
-  const int tiles = int(ceil_div(*count, kScanTile));
-  int carry = 0;
-  for (int base = 0; base < tiles; base += blockDim.x) {
-    int i = base + threadIdx.x;
-    int v = i < tiles ? partials[i] : 0;
-    int total;
-    int e = block_exclusive(v, smem, total);
-    if (i < tiles) partials[i] = carry + e;
-    carry += total;
-  }
-}
-
-__global__ void k_scan_apply(const int *__restrict__ in, int *out, const int *count,
-                             const int *partials, int *total_out) {
-  __shared__ int smem[33];
-  const int n = *count;
-  const int64_t base = int64_t(blockIdx.x) * kScanTile;
-  if (n == 0 && blockIdx.x == 0 && threadIdx.x == 0 && total_out) *total_out = 0;
-  if (base >= n) return;
+  const int tiles = int(ceil_div(n, kScanTile));
+  if (int(blockIdx.x) >= tiles) return;
+  unsigned epoch;
+  const int tile = take_tile(s, s_tile, epoch);
   constexpr int per = kScanTile / 256;  // blockDim.x == 256
+  const int64_t first = int64_t(tile) * kScanTile + int64_t(threadIdx.x) * per;
   int v[per];
   int sum = 0;
-  const int64_t first = base + int64_t(threadIdx.x) * per;
 #pragma unroll
-  for (int k = 0; k < per; ++k) {
-    int64_t i = first + k;
-    v[k] = i < n ? in[i] : 0;
-    sum += v[k];
+  for (int k = 0; k < per; k += 4) {
+    int4 x = make_int4(0, 0, 0, 0);
+    if (first + k + 3 < n) {
+      x = *reinterpret_cast<const int4 *>(in + first + k);
+      if (clear) *reinterpret_cast<int4 *>(in + first + k) = make_int4(0, 0, 0, 0);
+    } else {
+      int *y = reinterpret_cast<int *>(&x);
+      for (int c = 0; c < 4; ++c)
+        if (first + k + c < n) {
+          y[c] = in[first + k + c];
+          if (clear) in[first + k + c] = 0;
+        }
+    }
+    v[k] = x.x; v[k + 1] = x.y; v[k + 2] = x.z; v[k + 3] = x.w;
+    sum += x.x + x.y + x.z + x.w;
   }
   int total;
-  int e = block_exclusive(sum, smem, total) + partials[blockIdx.x];
-#pragma unroll
-  for (int k = 0; k < per; ++k) {
-    int64_t i = first + k;
-    if (i < n) {
-      out[i] = e;
-      if (i == n - 1 && total_out) *total_out = e + v[k];
+  int e = block_exclusive(sum, smem, total);
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int before = 0;
+    if (tile > 0) {
+      if (lane == 0) *(volatile unsigned long long *)&s.words[tile] = publish_word(epoch, kSum, total);
+      for (int look = tile - 1;; look -= 32) {
+        const int at = look - lane;
+        const unsigned long long w = at >= 0 ? await_word(s.words + at, epoch, s.error)
+                                             : publish_word(epoch, kPrefix, 0);
+        const unsigned full = __ballot_sync(0xffffffffu, (unsigned(w >> 32) & 3u) == kPrefix);
+        const int last = full ? __ffs(int(full)) - 1 : 31;
+        before += __reduce_add_sync(0xffffffffu, lane <= last ? int(unsigned(w)) : 0);
+        if (full) break;
+      }
     }
-    e += v[k];
+    if (lane == 0) {
+      *(volatile unsigned long long *)&s.words[tile] = publish_word(epoch, kPrefix, before + total);
+      s_before = before;
+    }
   }
+  __syncthreads();
+  e += s_before;
+#pragma unroll
+  for (int k = 0; k < per; k += 4) {
+    int4 x;
+    x.x = e; e += v[k];
+    x.y = e; e += v[k + 1];
+    x.z = e; e += v[k + 2];
+    x.w = e; e += v[k + 3];
+    if (first + k + 3 < n) {
+      *reinterpret_cast<int4 *>(out + first + k) = x;
+    } else {
+      const int *y = reinterpret_cast<const int *>(&x);
+      for (int c = 0; c < 4; ++c)
+        if (first + k + c < n) out[first + k + c] = y[c];
+    }
+  }
+  if (threadIdx.x == 0 && total_out && tile == tiles - 1) *total_out = s_before + total;
+  finish_tile(s, tiles);
 }
 
 // ---------------------------------------------------------------- radix sort
+// Digit counts of every pass at once: the digits of a key are those of the
+// key set, whatever its order, so one read serves all passes.  `hist` is
+// [passes][256], zero on entry (the last pass of a sort clears it).
 template <class K>
-__global__ void k_radix_hist(const K *__restrict__ keys, const int *count, int64_t tiles_cap,
-                             int shift, int *hist) {
-  __shared__ int h[256];
+__device__ inline void count_digits(K key, int passes, int *local) {
+  for (int p = 0; p < passes; ++p) atomicAdd(&local[256 * p + int((key >> (8 * p)) & 255u)], 1);
+}
+
+__device__ inline void add_digits(const int *local, int passes, int *hist) {
+  for (int k = threadIdx.x; k < 256 * passes; k += blockDim.x)
+    if (local[k]) atomicAdd(&hist[k], local[k]);
+}
+
+template <class K>
+__global__ void k_radix_hist(const K *__restrict__ keys, const int *count, int passes, int *hist) {
+  __shared__ int local[256 * kSortPasses];
   const int n = *count;
-  const int64_t base = int64_t(blockIdx.x) * kSortTile;
-  if (base >= n) return;
-  h[threadIdx.x] = 0;
+  if (n == 0) return;
+  for (int k = threadIdx.x; k < 256 * passes; k += blockDim.x) local[k] = 0;
   __syncthreads();
-  for (int k = threadIdx.x; k < kSortTile; k += blockDim.x) {
-    int64_t i = base + k;
-    if (i < n) atomicAdd(&h[int((keys[i] >> shift) & 255u)], 1);
-  }
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
+       i += int64_t(gridDim.x) * blockDim.x)
+    count_digits(keys[i], passes, local);
   __syncthreads();
-  hist[int64_t(threadIdx.x) * tiles_cap + blockIdx.x] = h[threadIdx.x];
+  add_digits(local, passes, hist);
 }
 
-// One block per digit: exclusive scan of that digit's counts across tiles.
-__global__ void k_radix_scan(int *hist, const int *count, int64_t tiles_cap, int *totals) {
-  __shared__ int smem[33];
-  const int tiles = int(ceil_div(*count, kSortTile));
-  int *row = hist + int64_t(blockIdx.x) * tiles_cap;
-  int carry = 0;
-  for (int base = 0; base < tiles; base += blockDim.x) {
-    int i = base + threadIdx.x;
-    int v = i < tiles ? row[i] : 0;
-    int total;
-    int e = block_exclusive(v, smem, total);
-    if (i < tiles) row[i] = carry + e;
-    carry += total;
-  }
-  if (threadIdx.x == 0) totals[blockIdx.x] = carry;
-}
-
-// Stable scatter: warp w owns a contiguous run of 256 keys of the tile, in
+// One stable pass.  Warp w of a tile owns a contiguous run of 256 keys, in
 // eight rounds of 32; peers with equal digits are ranked with match_any.
+// Thread d looks back over the tiles before for digit d, eight at a time.
 template <class K>
-__global__ void __launch_bounds__(kSortBlock) k_radix_scatter(
+__global__ void __launch_bounds__(kSortBlock) k_radix_pass(
     const K *__restrict__ keys, const int *__restrict__ vals, K *keys_out, int *vals_out,
-    const int *count, int64_t tiles_cap, int shift, const int *hist, const int *totals) {
-  __shared__ int base[256];
+    const int *count, int pass, int passes, int *hist, LookBack s) {
   __shared__ int wcount[kSortBlock / 32][256];
   __shared__ int smem[33];
+  __shared__ int s_tile[1];
   const int n = *count;
-  const int64_t tile0 = int64_t(blockIdx.x) * kSortTile;
-  if (tile0 >= n) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  {
-    int t = totals[threadIdx.x];
-    int total;
-    int e = block_exclusive(t, smem, total);
-    base[threadIdx.x] = e + hist[int64_t(threadIdx.x) * tiles_cap + blockIdx.x];
-  }
+  if (n == 0) return;
+  const int tiles = int(ceil_div(n, kSortTile));
+  if (int(blockIdx.x) >= tiles) return;
+  unsigned epoch;
+  const int tile = take_tile(s, s_tile, epoch);
+  const int64_t tile0 = int64_t(tile) * kSortTile;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, shift = 8 * pass;
+  int total;
+  int running = block_exclusive(hist[256 * pass + threadIdx.x], smem, total);
   for (int w = 0; w < kSortBlock / 32; ++w) wcount[w][threadIdx.x] = 0;
   __syncthreads();
   K k[kSortItems];
@@ -177,7 +247,33 @@ __global__ void __launch_bounds__(kSortBlock) k_radix_scatter(
   }
   __syncthreads();
   {
-    int running = base[threadIdx.x];
+    int mine = 0;
+    for (int w = 0; w < kSortBlock / 32; ++w) mine += wcount[w][threadIdx.x];
+    unsigned long long *words = s.words + threadIdx.x;
+    int before = 0;
+    if (tile > 0) {
+      *(volatile unsigned long long *)&words[256 * int64_t(tile)] = publish_word(epoch, kSum, mine);
+      constexpr int kWindow = 8;
+      for (int look = tile - 1, done = 0; !done; look -= kWindow) {
+        unsigned long long w[kWindow];
+#pragma unroll
+        for (int c = 0; c < kWindow; ++c)
+          w[c] = look - c >= 0
+                     ? *(const volatile unsigned long long *)&words[256 * int64_t(look - c)]
+                     : publish_word(epoch, kPrefix, 0);
+#pragma unroll
+        for (int c = 0; c < kWindow; ++c) {
+          if (done) continue;
+          if (unsigned(w[c] >> 34) != epoch || (unsigned(w[c] >> 32) & 3u) == kNothing)
+            w[c] = await_word(words + 256 * int64_t(look - c), epoch, s.error);
+          before += int(unsigned(w[c]));
+          done = (unsigned(w[c] >> 32) & 3u) == kPrefix;
+        }
+      }
+    }
+    *(volatile unsigned long long *)&words[256 * int64_t(tile)] =
+        publish_word(epoch, kPrefix, before + mine);
+    running += before;
     for (int w = 0; w < kSortBlock / 32; ++w) {
       int c = wcount[w][threadIdx.x];
       wcount[w][threadIdx.x] = running;
@@ -198,6 +294,13 @@ __global__ void __launch_bounds__(kSortBlock) k_radix_scatter(
     if (d[r] < 256 && lane == __ffs(peers) - 1) wcount[warp][d[r]] += __popc(peers);
     __syncwarp();
   }
+  const bool last = finish_tile(s, tiles);
+  if (pass == passes - 1) {  // every block has read the digit counts
+    if (threadIdx.x == 0) s_tile[0] = last;
+    __syncthreads();
+    if (s_tile[0])
+      for (int p = 0; p < passes; ++p) hist[256 * p + threadIdx.x] = 0;
+  }
 }
 
 template <class K>
@@ -211,43 +314,55 @@ __global__ void k_copy_pairs(const K *keys, const int *vals, K *keys_out, int *v
   }
 }
 
+// The passes of a sort whose digit counts are in s.hist.
 template <class K>
-cudaError_t sort_pairs(K *keys, K *keys_tmp, int *vals, int *vals_tmp, const int *count,
-                       int64_t capacity, int bits, SortScratch &s, cudaStream_t st) {
+cudaError_t sort_passes(K *keys, K *keys_tmp, int *vals, int *vals_tmp, const int *count,
+                        int64_t capacity, int passes, SortScratch &s, cudaStream_t st) {
   const int64_t tiles = ceil_div(capacity, kSortTile);
-  if (tiles > s.tiles) return cudaErrorInvalidValue;
-  const int passes = int(ceil_div(bits, 8));
+  if (tiles > s.tiles || passes > kSortPasses) return cudaErrorInvalidValue;
   K *ka = keys, *kb = keys_tmp;
   int *va = vals, *vb = vals_tmp;
   for (int p = 0; p < passes; ++p) {
-    const int shift = 8 * p;
-    k_radix_hist<K><<<unsigned(tiles), kSortBlock, 0, st>>>(ka, count, s.tiles, shift, s.hist);
-    note_launch();
-    k_radix_scan<<<256, 256, 0, st>>>(s.hist, count, s.tiles, s.totals);
-    note_launch();
-    k_radix_scatter<K><<<unsigned(tiles), kSortBlock, 0, st>>>(ka, va, kb, vb, count, s.tiles, shift, s.hist, s.totals);
+    k_radix_pass<K><<<unsigned(tiles), kSortBlock, 0, st>>>(ka, va, kb, vb, count, p, passes,
+                                                             s.hist, s.look_back);
     note_launch();
     K *tk = ka; ka = kb; kb = tk;
     int *tv = va; va = vb; vb = tv;
   }
-  if (ka != keys)
+  if (ka != keys) {
     k_copy_pairs<K><<<592, 256, 0, st>>>(ka, va, keys, vals, count);
     note_launch();
+  }
   return cudaGetLastError();
 }
 
-// ---------------------------------------------------------------- hierarchy
-__global__ void k_tree_size(const int *count_ptr, int static_count, int *count_out, int *size) {
-  int c = count_ptr ? *count_ptr : static_count;
-  int p = 1;
-  while (p < c) p <<= 1;
-  *count_out = c;
-  *size = p;
+template <class K>
+cudaError_t sort_pairs(K *keys, K *keys_tmp, int *vals, int *vals_tmp, const int *count,
+                       int64_t capacity, int bits, SortScratch &s, cudaStream_t st) {
+  const int passes = int(ceil_div(bits, 8));
+  k_radix_hist<K><<<unsigned(std::min<int64_t>(ceil_div(capacity, kSortTile), 148 * 4)),
+                    kSortBlock, 0, st>>>(keys, count, passes, s.hist);
+  note_launch();
+  return sort_passes(keys, keys_tmp, vals, vals_tmp, count, capacity, passes, s, st);
 }
 
-__global__ void k_tree_keys(const float4 *lo, const float4 *hi, const int *count, const int *size,
-                            uint64_t *keys, int *ids, int layered) {
-  const int n = *count, leaves = *size;
+// ---------------------------------------------------------------- hierarchy
+// The build's item and leaf counts, the leaves' keys, and the keys' digit
+// counts for the sort.
+__global__ void k_tree_keys(const float4 *lo, const float4 *hi, const int *count_ptr,
+                            int static_count, int *count_out, int *size, uint64_t *keys, int *ids,
+                            int layered, int passes, int *hist) {
+  __shared__ int local[256 * kSortPasses];
+  const int n = count_ptr ? *count_ptr : static_count;
+  int leaves = 1;
+  while (leaves < n) leaves <<= 1;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *count_out = n;
+    *size = leaves;
+  }
+  if (int64_t(blockIdx.x) * blockDim.x >= leaves) return;
+  for (int k = threadIdx.x; k < 256 * passes; k += blockDim.x) local[k] = 0;
+  __syncthreads();
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < leaves;
        i += int64_t(gridDim.x) * blockDim.x) {
     ids[i] = int(i);
@@ -261,9 +376,12 @@ __global__ void k_tree_keys(const float4 *lo, const float4 *hi, const int *count
         key = uint64_t(part1by1(x) | (part1by1(y) << 1));
         if (layered) key |= uint64_t(int(a.z)) << 32;
       }
+      count_digits(key, passes, local);
     }
     keys[i] = key;
   }
+  __syncthreads();
+  add_digits(local, passes, hist);
 }
 
 // Every node of a fresh hierarchy holds the empty box, which overlaps nothing.
@@ -362,15 +480,11 @@ k_tree_fit(float4 *nodes, const int *ids, const float4 *lo, const float4 *hi, co
 
 }  // namespace
 
-cudaError_t scan_exclusive(const int *in, int *out, const int *count, int64_t capacity,
-                           int *total, SortScratch &s, cudaStream_t st) {
+cudaError_t scan_exclusive(int *in, int *out, const int *count, int64_t capacity, int *total,
+                           SortScratch &s, cudaStream_t st, bool clear) {
   const int64_t tiles = ceil_div(capacity > 0 ? capacity : 1, kScanTile);
   if (tiles > s.scan_tiles) return cudaErrorInvalidValue;
-  k_scan_reduce<<<unsigned(tiles), 256, 0, st>>>(in, count, s.partials);
-  note_launch();
-  k_scan_partials<<<1, 1024, 0, st>>>(s.partials, count);
-  note_launch();
-  k_scan_apply<<<unsigned(tiles), 256, 0, st>>>(in, out, count, s.partials, total);
+  k_scan<<<unsigned(tiles), 256, 0, st>>>(in, out, count, s.look_back, total, clear ? 1 : 0);
   note_launch();
   return cudaGetLastError();
 }
@@ -379,11 +493,6 @@ cudaError_t sort_pairs_u64(uint64_t *keys, uint64_t *keys_tmp, int *vals, int *v
                            const int *count, int64_t capacity, int bits, SortScratch &s,
                            cudaStream_t st) {
   return sort_pairs<uint64_t>(keys, keys_tmp, vals, vals_tmp, count, capacity, bits, s, st);
-}
-cudaError_t sort_pairs_u32(uint32_t *keys, uint32_t *keys_tmp, int *vals, int *vals_tmp,
-                           const int *count, int64_t capacity, int bits, SortScratch &s,
-                           cudaStream_t st) {
-  return sort_pairs<uint32_t>(keys, keys_tmp, vals, vals_tmp, count, capacity, bits, s, st);
 }
 
 cudaError_t tree_refit(TreeBuffers &t, const float4 *lo, const float4 *hi, cudaStream_t st) {
@@ -423,16 +532,15 @@ void tree_free(TreeBuffers &t) {
 
 cudaError_t tree_build(TreeBuffers &t, const float4 *lo, const float4 *hi, const int *count_ptr,
                        int static_count, bool layered, SortScratch &s, cudaStream_t st) {
-  k_tree_size<<<1, 1, 0, st>>>(count_ptr, static_count, t.count, t.size);
-  note_launch();
-  const unsigned g = grid_for(t.leaves_cap, 256) < 4 * 148 ? grid_for(t.leaves_cap, 256) : 4 * 148;
-  k_tree_keys<<<g, 256, 0, st>>>(lo, hi, t.count, t.size, t.keys, t.ids, layered ? 1 : 0);
-  note_launch();
   // Layered keys hold the layer above 30 Morton bits; 48 key bits order them
   // for up to 65536 layers.  Deeper scenes leave higher layer bits unordered,
   // which only loosens the hierarchy: any leaf order gives the same queries.
-  int bits = layered ? 48 : 30;
-  EDP_CHECK(sort_pairs_u64(t.keys, t.keys_tmp, t.ids, t.ids_tmp, t.count, t.leaves_cap, bits, s, st));
+  const int passes = layered ? 6 : 4;
+  const unsigned g = grid_for(t.leaves_cap, 256) < 4 * 148 ? grid_for(t.leaves_cap, 256) : 4 * 148;
+  k_tree_keys<<<g, 256, 0, st>>>(lo, hi, count_ptr, static_count, t.count, t.size, t.keys, t.ids,
+                                 layered ? 1 : 0, passes, s.hist);
+  note_launch();
+  EDP_CHECK(sort_passes(t.keys, t.keys_tmp, t.ids, t.ids_tmp, t.count, t.leaves_cap, passes, s, st));
   return tree_refit(t, lo, hi, st);
 }
 

@@ -163,11 +163,13 @@ cudaError_t allocate_shared(edp_peeler *p) {
 }
 
 cudaError_t allocate_scratch(edp_peeler *p, int64_t largest_sort, int64_t largest_scan) {
-  p->scratch.tiles = ceil_div(largest_sort, kSortTile);
-  p->scratch.scan_tiles = ceil_div(largest_scan, kScanTile);
-  EDP_CHECK(alloc(p, &p->scratch.hist, 256 * p->scratch.tiles));
-  EDP_CHECK(alloc(p, &p->scratch.totals, 256));
-  EDP_CHECK(alloc(p, &p->scratch.partials, p->scratch.scan_tiles));
+  SortScratch &s = p->scratch;
+  s.tiles = ceil_div(largest_sort, kSortTile);
+  s.scan_tiles = ceil_div(largest_scan, kScanTile);
+  EDP_CHECK(alloc(p, &s.hist, 256 * kSortPasses));
+  EDP_CHECK(alloc(p, &s.look_back.words, std::max(256 * s.tiles, s.scan_tiles)));
+  EDP_CHECK(alloc(p, &s.look_back.control, 3));
+  s.look_back.error = p->d.status + kError;
   return cudaSuccess;
 }
 
