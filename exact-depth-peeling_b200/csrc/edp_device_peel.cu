@@ -677,21 +677,12 @@ __global__ void k_layer_next(Dev d) {
   if (d.use_handle) cudaGraphSetConditional(d.cond_handle, unsigned(c));
 }
 
-__global__ void k_device_finish(Dev d) {
-  d.sc[kLivePolygons] = int(min(int64_t(d.status[kPolygons]), d.cap.regions));
-}
-
 }  // namespace
-
-cudaError_t stage_device_finish(const Dev &d, cudaStream_t st) {
-  k_device_finish<<<1, 1, 0, st>>>(d);
-  note_launch();
-  return cudaGetLastError();
-}
 
 cudaError_t stage_device_prepare(const Dev &d, SortScratch &s, TreeBuffers &source_tree,
                                  TreeBuffers &contour_tree, cudaStream_t st) {
-  EDP_CHECK(stage_prepare_common(d, s, source_tree, st));
+  EDP_CHECK(stage_prepare_common(d, false, st));
+  EDP_CHECK(tree_build(source_tree, d.src_lo, d.src_hi, nullptr, d.n, false, s, st));
   EDP_CHECK(cudaMemsetAsync(d.stats, 0, sizeof(long long) * 3 * d.cap.layers, st));
   k_contour_bounds<<<blocks(d.n), kBlock, 0, st>>>(d);
   note_launch();

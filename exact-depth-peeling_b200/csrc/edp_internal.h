@@ -21,7 +21,7 @@ int record_cuda_failure(cudaError_t e, const char *site);
 constexpr int kSortBlock = 256;
 constexpr int kSortItems = 8;
 constexpr int kSortTile = kSortBlock * kSortItems;  // keys per radix tile
-constexpr int kScanTile = 2048;
+constexpr int kScanTile = 4096;
 
 __host__ __device__ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline int64_t pow2_at_least(int64_t v) {
@@ -140,7 +140,8 @@ enum Scalar : int {
   kAssignDeferred = 30,
   kDeepGroups = 31,  // hit groups sorted a warp each (k_group_sort_deep)
   kCandidates = 32,  // entries of the sources' candidate lists
-  kScalarCount = 33  // k_reset clears them with one block
+  kOrderLive = 33,   // buckets of the current work order
+  kScalarCount = 34  // k_reset clears them with its first threads
 };
 
 // Predicate tallies: six classes by three deciding stages (edp_filtered.cuh).
@@ -274,7 +275,11 @@ struct Dev {
   // their box centre (optionally below the layer), rebuilt by each stage that
   // uses it, so that neighbouring threads walk neighbouring parts of a
   // hierarchy.  No result depends on it.
+  // (A counting sort into buckets; with merging, which breaks its ties by the
+  // order, the rank stage's is a full radix sort.)
   uint64_t *order_keys, *order_keys_tmp;
+  int *order_count, *order_start;  // [2^order_bits]; the counts are zero between sorts
+  int order_bits;
   int *order, *order_tmp;
   V2 *tri_uv;        // [triangles][3]
   double *tri_world; // [triangles][3][3]
@@ -322,11 +327,9 @@ __device__ inline bool contour_edge(const Dev &d, int64_t source, int edge) {
 
 // Reset, validation, welding, projection, mesh contours and the source
 // hierarchy: the part of preparation both peelers share.
-cudaError_t stage_prepare_common(const Dev &d, SortScratch &s, TreeBuffers &source_tree,
-                                 cudaStream_t st);
+cudaError_t stage_prepare_common(const Dev &d, bool event, cudaStream_t st);
 cudaError_t stage_device_prepare(const Dev &d, SortScratch &s, TreeBuffers &source_tree,
                                  TreeBuffers &contour_tree, cudaStream_t st);
-cudaError_t stage_device_finish(const Dev &d, cudaStream_t st);
 // One layer pass on `st`; its clipping rounds are recorded on `rounds` when
 // `st` is capturing (a nested conditional WHILE node), else host-driven.
 cudaError_t stage_device_layer(const Dev &d, SortScratch &s, TreeBuffers &source_tree,
@@ -338,6 +341,13 @@ cudaError_t tree_refit(TreeBuffers &t, const float4 *lo, const float4 *hi, cudaS
 // Rebuild Dev::order over the live output polygons: by Morton code of the box
 // centre, below the layer when `layered`.
 cudaError_t order_polygons(const Dev &d, bool layered, SortScratch &s, cudaStream_t st);
+// The rank stage's order as a full sort (for merging).
+cudaError_t sort_polygons(const Dev &d, SortScratch &s, cudaStream_t st);
+
+cudaError_t conditional_handle(cudaStream_t st, cudaGraphConditionalHandle &handle);
+cudaError_t conditional_begin(cudaStream_t st, cudaGraphConditionalHandle handle,
+                              cudaStream_t body);
+cudaError_t conditional_end(cudaStream_t body);
 
 // Stage launchers (edp_prepare.cu, edp_frontier.cu, edp_rank.cu, edp_mesh.cu).  Each
 // enqueues kernels on `st`.

@@ -15,43 +15,6 @@ constexpr int kMaxEdgeVertices = 128;  // edge noding capacity (solver.py:140-14
 __device__ inline int64_t tid() { return blockIdx.x * int64_t(blockDim.x) + threadIdx.x; }
 __device__ inline int64_t stride() { return int64_t(gridDim.x) * blockDim.x; }
 
-// Boundary vertex slots follow the polygons' (layer, Morton) order, so the
-// copies of one point, which neighbouring polygons share, meet the point table
-// close together in time.
-__global__ void k_mesh_counts(Dev d) {
-  const int live = d.sc[kLivePolygons];
-  for (int64_t k = tid(); k < live; k += stride())
-    d.counts[k] = d.status[kError] == 0 ? d.out_n[d.order[k]] : 0;
-}
-
-__global__ void k_mesh_check(Dev d) {
-  d.sc[kUniqueVertices] = 0;
-  int total = d.sc[kLiveVertices];
-  d.status[kBoundaryVertices] = total;
-  if (int64_t(total) > d.cap.vertices) {
-    set_error(d.status, kErrVertices);
-    d.sc[kLiveVertices] = int(d.cap.vertices);
-  }
-}
-
-// Boundary vertices with their layer, one slot per polygon vertex
-// (kernels.py:953-991, event_kernels.py:504-516).
-__global__ void k_scatter(Dev d) {
-  const int live = d.sc[kLivePolygons];
-  for (int64_t k = tid(); k < live; k += stride()) {
-    if (d.status[kError] != 0) return;
-    const int i = d.order[k];
-    const V2 *p = d.out_v + int64_t(kMaxVertices) * i;
-    const int layer = d.out_layer[i];
-    const int64_t base = d.offsets[k];
-    const int n = int(min(int64_t(d.out_n[i]), d.cap.vertices - base));
-    for (int j = 0; j < n; ++j) {
-      d.bverts[base + j] = p[j];
-      d.blayers[base + j] = layer;
-    }
-  }
-}
-
 // Grid column (or row) of a window coordinate: floor(v G) clamped to the
 // grid.  Monotone in v, so a query interval's cells hold every point inside it.
 __device__ inline int grid_cell(double v, int g) {
@@ -59,29 +22,53 @@ __device__ inline int grid_cell(double v, int g) {
   return c < 0.0 ? 0 : c > double(g - 1) ? g - 1 : int(c);
 }
 
-// The grid serves this extraction when it has a row for every layer;
-// otherwise the point hierarchy does.
-__global__ void k_grid_begin(Dev d) {
-  const int layers = d.status[kLayers];
-  const bool on = d.status[kError] == 0 && layers <= d.grid_layers;
-  d.sc[kGridOn] = on ? 1 : 0;
-  d.sc[kGridCells] = on ? int(int64_t(layers) * d.point_grid * d.point_grid) : 0;
-}
-
-// Zero the point counts of the cells this extraction uses.
-__global__ void k_grid_clear(Dev d) {
-  const int cells = d.sc[kGridCells];
-  for (int64_t c = tid(); c < cells; c += stride()) d.cell_count[c] = 0;
-}
-
-__global__ void k_tree_points(Dev d) {
-  d.sc[kTreePoints] = d.sc[kGridOn] ? 0 : d.sc[kUniqueVertices];
+// Boundary vertices with their layer, one slot per polygon vertex
+// (kernels.py:953-991, event_kernels.py:504-516), in the polygons' (layer,
+// Morton) order, so that the copies of one point, which neighbouring polygons
+// share, meet the point table close together in time.  The point grid serves
+// this extraction when it has a row for every layer; otherwise the point
+// hierarchy does.
+__global__ void k_scatter(Dev d) {
+  const int live = d.sc[kLivePolygons];
+  const int total = d.sc[kLiveVertices];  // or the capacity, once clamped below
+  const bool fits = int64_t(total) <= d.cap.vertices;
+  if (tid() == 0) {
+    const int layers = d.status[kLayers];
+    const bool on = d.status[kError] == 0 && fits && layers <= d.grid_layers;
+    d.sc[kGridOn] = on ? 1 : 0;
+    d.sc[kGridCells] = on ? int(int64_t(layers) * d.point_grid * d.point_grid) : 0;
+    d.status[kBoundaryVertices] = total;
+    if (!fits) {
+      set_error(d.status, kErrVertices);
+      d.sc[kLiveVertices] = int(d.cap.vertices);
+    }
+  }
+  if (!fits) return;
+  for (int64_t k = tid(); k < live; k += stride()) {
+    if (d.status[kError] != 0) return;
+    const int i = d.order[k];
+    const V2 *p = d.out_v + int64_t(kMaxVertices) * i;
+    const int layer = d.out_layer[i];
+    const int64_t base = d.offsets[k];
+    const int n = d.out_n[i];
+    for (int j = 0; j < n; ++j) {
+      d.bverts[base + j] = p[j];
+      d.blayers[base + j] = layer;
+    }
+  }
 }
 
 // Counting sort of the distinct points by (layer, cell): the scan of the
 // counts gives each cell's start, and each point takes a slot of its cell.
-__global__ void k_grid_scatter(Dev d) {
-  if (!d.sc[kGridOn] || d.status[kError] != 0) return;
+// Taking the slots counts every cell back down to zero, so the counts need no
+// clearing between extractions.
+__global__ void k_grid_scatter(Dev d, cudaGraphConditionalHandle handle, int conditional) {
+  if (tid() == 0) {
+    // The point hierarchy's items, and in a graph whether its node runs.
+    d.sc[kTreePoints] = d.sc[kGridOn] ? 0 : d.sc[kUniqueVertices];
+    if (conditional) cudaGraphSetConditional(handle, d.sc[kGridOn] ? 0u : 1u);
+  }
+  if (!d.sc[kGridOn]) return;
   const int total = d.sc[kUniqueVertices], g = d.point_grid;
   if (tid() == 0) d.cell_start[d.sc[kGridCells]] = total;
   for (int64_t u = tid(); u < total; u += stride()) {
@@ -134,24 +121,91 @@ __global__ void k_unique_points(Dev d) {
 // Sort key of each live output polygon: the Morton code of its box centre
 // (the 15-bit-per-axis code of the hierarchies, kernels.py:67-91, cut to 12
 // bits per axis), below its layer when `layered`.
-__global__ void k_order_keys(Dev d, int layered) {
-  const int live = d.sc[kLivePolygons];
+__device__ inline uint64_t morton_of(const Dev &d, int64_t i) {
+  const V2 *p = d.out_v + int64_t(kMaxVertices) * i;
+  const int n = min(max(d.out_n[i], 1), kMaxVertices);
+  double lx = p[0].x, ly = p[0].y, hx = p[0].x, hy = p[0].y;
+  for (int j = 1; j < n; ++j) {
+    lx = fmin(lx, p[j].x); ly = fmin(ly, p[j].y);
+    hx = fmax(hx, p[j].x); hy = fmax(hy, p[j].y);
+  }
+  const float cx = fminf(fmaxf(float(0.5 * (lx + hx)), 0.f), 1.f);
+  const float cy = fminf(fmaxf(float(0.5 * (ly + hy)), 0.f), 1.f);
+  const uint32_t x = uint32_t(int(cx * 32767.0f)), y = uint32_t(int(cy * 32767.0f));
+  // 12 bits per axis (a 4096 x 4096 grid) are plenty for locality.
+  return (part1by1(x) | (part1by1(y) << 1)) >> 6;
+}
+
+__device__ inline int live_outputs(const Dev &d) {
+  return int(min(int64_t(d.status[kPolygons]), d.cap.regions));
+}
+
+__global__ void k_order_keys(Dev d) {
+  const int live = live_outputs(d);
+  if (tid() == 0) d.sc[kLivePolygons] = live;
   for (int64_t i = tid(); i < live; i += stride()) {
-    const V2 *p = d.out_v + int64_t(kMaxVertices) * i;
-    const int n = min(max(d.out_n[i], 1), kMaxVertices);
-    double lx = p[0].x, ly = p[0].y, hx = p[0].x, hy = p[0].y;
-    for (int j = 1; j < n; ++j) {
-      lx = fmin(lx, p[j].x); ly = fmin(ly, p[j].y);
-      hx = fmax(hx, p[j].x); hy = fmax(hy, p[j].y);
-    }
-    const float cx = fminf(fmaxf(float(0.5 * (lx + hx)), 0.f), 1.f);
-    const float cy = fminf(fmaxf(float(0.5 * (ly + hy)), 0.f), 1.f);
-    const uint32_t x = uint32_t(int(cx * 32767.0f)), y = uint32_t(int(cy * 32767.0f));
-    // 12 bits per axis (a 4096 x 4096 grid) are plenty for locality.
-    uint64_t key = (part1by1(x) | (part1by1(y) << 1)) >> 6;
-    if (layered) key |= uint64_t(uint32_t(d.out_layer[i]) & 0xffffu) << 24;
-    d.order_keys[i] = key;
+    d.order_keys[i] = morton_of(d, i);
     d.order[i] = int(i);
+  }
+}
+
+// The same order by a counting sort: buckets of the leading Morton bits, below
+// the layer when `layered`, 4 to 8 per polygon (the polygons cover a small part
+// of the window) and at most 2^Dev::order_bits.  Three launches where the radix
+// sort took 5 and 7; the order inside a bucket is left to chance, which no
+// result depends on.  Twice the buckets cost as much in their scan as they
+// gain in locality (both within 0.03 ms on the 65,536-face knot), but with 2^20
+// at most the rays and the noding of 2.2M polygons of the 720K primitives took
+// 2.11 and 3.69 ms instead of 1.70 and 3.60.
+__device__ inline int ceil_log2(int v) { return v <= 1 ? 0 : 32 - __clz(v - 1); }
+
+__device__ inline void order_bits(const Dev &d, int live, int layered, int &layer_shift,
+                                  int &layer_bits, int &morton_bits) {
+  const int most = d.order_bits, want = min(most, ceil_log2(live) + 2);
+  layer_bits = layered ? ceil_log2(max(d.status[kLayers], 1)) : 0;
+  layer_shift = max(0, layer_bits - most);
+  layer_bits -= layer_shift;
+  morton_bits = max(0, want - layer_bits);
+}
+
+__global__ void k_order_count(Dev d, int layered) {
+  const int live = live_outputs(d);
+  int layer_shift, layer_bits, morton_bits;
+  order_bits(d, live, layered, layer_shift, layer_bits, morton_bits);
+  if (tid() == 0) {
+    d.sc[kLivePolygons] = live;
+    d.sc[kOrderLive] = 1 << (layer_bits + morton_bits);
+  }
+  for (int64_t i = tid(); i < live; i += stride()) {
+    int bucket = int(morton_of(d, i) >> (24 - morton_bits));
+    if (layered) {
+      // A layer past the limit (an error, or a suppressed polygon) shares the last.
+      const int layer = min(max(d.out_layer[i], 0) >> layer_shift, (1 << layer_bits) - 1);
+      bucket |= layer << morton_bits;
+    }
+    d.order_keys[i] = uint64_t(bucket) << 32 | unsigned(atomicAdd(&d.order_count[bucket], 1));
+  }
+}
+
+// Places the polygons, and lays out what the stage scans next: each polygon's
+// vertex count in this order.
+__global__ void k_order_place(Dev d, int layered) {
+  const int live = d.sc[kLivePolygons];
+  if (layered && tid() == 0) {
+    d.sc[kUniqueVertices] = 0;
+    d.sc[kHeavyPolygons] = 0;
+  }
+  const bool failed = layered && d.status[kError] != 0;
+  for (int64_t i = tid(); i < live; i += stride()) {
+    const uint64_t key = d.order_keys[i];
+    const int at = d.order_start[key >> 32] + int(unsigned(key));
+    d.order[at] = int(i);
+    d.counts[at] = failed ? 0 : d.out_n[i];
+    if (!layered) {
+      d.parents[i] = int(i);
+      d.group_counts[i] = 0;
+      d.group_fill[i] = 0;
+    }
   }
 }
 
@@ -801,46 +855,60 @@ unsigned blocks(int64_t n) {
 
 cudaError_t order_polygons(const Dev &d, bool layered, SortScratch &s, cudaStream_t st) {
   const int64_t R = d.cap.regions;
-  k_order_keys<<<blocks(R), kBlock, 0, st>>>(d, layered ? 1 : 0);
+  k_order_count<<<blocks(R), kBlock, 0, st>>>(d, layered ? 1 : 0);
   note_launch();
-  // 16 layer bits above 24 Morton bits.
+  EDP_CHECK(scan_exclusive(d.order_count, d.order_start, d.sc + kOrderLive,
+                           int64_t(1) << d.order_bits, nullptr, s, st, true));
+  k_order_place<<<blocks(R), kBlock, 0, st>>>(d, layered ? 1 : 0);
+  note_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t sort_polygons(const Dev &d, SortScratch &s, cudaStream_t st) {
+  const int64_t R = d.cap.regions;
+  k_order_keys<<<blocks(R), kBlock, 0, st>>>(d);
+  note_launch();
   return sort_pairs_u64(d.order_keys, d.order_keys_tmp, d.order, d.order_tmp,
-                        d.sc + kLivePolygons, R, layered ? 40 : 24, s, st);
+                        d.sc + kLivePolygons, R, 24, s, st);
 }
 
 cudaError_t stage_mesh_index(const Dev &d, SortScratch &s, TreeBuffers &point_tree,
                              cudaStream_t st) {
   const int64_t R = d.cap.regions, E = d.cap.vertices;
   EDP_CHECK(order_polygons(d, true, s, st));
-  k_mesh_counts<<<blocks(R), kBlock, 0, st>>>(d);
-  note_launch();
   EDP_CHECK(scan_exclusive(d.counts, d.offsets, d.sc + kLivePolygons, R, d.sc + kLiveVertices, s, st));
-  k_mesh_check<<<1, 1, 0, st>>>(d);
-  note_launch();
   EDP_CHECK(cudaMemsetAsync(d.point_table, 0xff, sizeof(int) * (int64_t(d.point_mask) + 1), st));
   const int64_t cells = int64_t(d.grid_layers) * d.point_grid * d.point_grid;
-  k_grid_begin<<<1, 1, 0, st>>>(d);
-  note_launch();
-  k_grid_clear<<<blocks(cells), kBlock, 0, st>>>(d);
-  note_launch();
   k_scatter<<<blocks(R), kBlock, 0, st>>>(d);
   note_launch();
   k_unique_points<<<blocks(E), kBlock, 0, st>>>(d);
   note_launch();
   EDP_CHECK(stage_mark(EDP_STAGE_MESH_VERTICES, st));
   EDP_CHECK(scan_exclusive(d.cell_count, d.cell_start, d.sc + kGridCells, cells, nullptr, s, st));
-  k_grid_scatter<<<blocks(E), kBlock, 0, st>>>(d);
+  // The point hierarchy sits in a conditional IF node of a captured graph (run
+  // eagerly, it takes its count, zero with the grid, from the device).
+  cudaGraphConditionalHandle handle{};
+  const bool branch = d.use_handle && d.aux_stream;
+  if (branch) EDP_CHECK(conditional_handle(st, handle));
+  k_grid_scatter<<<blocks(E), kBlock, 0, st>>>(d, handle, branch ? 1 : 0);
   note_launch();
-  k_tree_points<<<1, 1, 0, st>>>(d);
-  note_launch();
-  EDP_CHECK(tree_build(point_tree, d.pt_lo, d.pt_hi, d.sc + kTreePoints, 0, true, s, st));
+  if (branch) {
+    EDP_CHECK(conditional_begin(st, handle, d.aux_stream));
+    const int64_t first = launch_count();
+    cudaError_t built = tree_build(point_tree, d.pt_lo, d.pt_hi, d.sc + kTreePoints, 0, true, s,
+                                   d.aux_stream);
+    EDP_CHECK(conditional_end(d.aux_stream));
+    EDP_CHECK(built);
+    forget_launches(launch_count() - first);
+  } else {
+    EDP_CHECK(tree_build(point_tree, d.pt_lo, d.pt_hi, d.sc + kTreePoints, 0, true, s, st));
+  }
   EDP_CHECK(stage_mark(EDP_STAGE_MESH_INDEX, st));
   return cudaGetLastError();
 }
 
 cudaError_t stage_mesh_emit(const Dev &d, cudaStream_t st) {
   int cap = int(d.cap.edge_vertices < kMaxEdgeVertices ? d.cap.edge_vertices : kMaxEdgeVertices);
-  EDP_CHECK(cudaMemsetAsync(d.sc + kHeavyPolygons, 0, sizeof(int), st));
   k_mesh_groups<<<unsigned(std::min<int64_t>(ceil_div(d.cap.regions, kMeshGroups), 148 * 6)),
                   kBlock, 0, st>>>(d, cap);
   note_launch();

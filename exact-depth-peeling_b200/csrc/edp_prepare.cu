@@ -11,18 +11,40 @@ constexpr int kBlock = 128;
 __device__ inline int64_t tid() { return blockIdx.x * int64_t(blockDim.x) + threadIdx.x; }
 __device__ inline int64_t stride() { return int64_t(gridDim.x) * blockDim.x; }
 
-__global__ void k_reset(Dev d) {
+// Tables to fill with one 32-bit word each, 16 bytes at a time.
+struct FillList {
+  static constexpr int kMost = 12;
+  uint4 *at[kMost];
+  int64_t quads[kMost];
+  unsigned word[kMost];
+  int count = 0;
+  template <class T>
+  void add(T *p, int64_t elements, unsigned value) {  // alloc() pads to 16 bytes
+    at[count] = reinterpret_cast<uint4 *>(p);
+    quads[count] = ceil_div(elements * int64_t(sizeof(T)), 16);
+    word[count++] = value;
+  }
+};
+
+// Counters and every table an extraction fills, in one launch.
+__global__ void k_reset(Dev d, FillList fills) {
   const int i = int(tid());
   if (i < kStatusSlots) d.status[i] = 0;
   if (i < kMetrics) d.metrics[i] = 0;
-  if (i < kScalarCount) d.sc[i] = 0;
   if (i < kPredCounters) d.pred_counts[i] = 0;
+  if (i < kScalarCount)
+    d.sc[i] = i == kSourceCount    ? d.n
+              : i == kSegmentSlots ? kSourceVertices * d.n
+              : i == kRayGridCells ? d.grid_size * d.grid_size
+                                   : 0;
   if (i == 0) {
-    d.sc[kSourceCount] = d.n;
-    d.sc[kSegmentSlots] = kSourceVertices * d.n;
-    d.sc[kRayGridCells] = d.grid_size * d.grid_size;
     *d.parity = 0;
     *d.condition = 0;
+  }
+  for (int f = 0; f < fills.count; ++f) {
+    const unsigned w = fills.word[f];
+    for (int64_t q = tid(); q < fills.quads[f]; q += stride())
+      fills.at[f][q] = make_uint4(w, w, w, w);
   }
 }
 
@@ -38,9 +60,35 @@ __device__ inline double det4(const double *m) {
   return m[0] * c0 - m[1] * c1 + m[2] * c2 - m[3] * c3;
 }
 
-// Input validation (kernels.py:309-350): finite values, face indices in
+// Exact-position welding: the canonical id of a vertex is the smallest index
+// with an equal position, signed zeros equal (kernels.py:269-306).  The
+// reference sorts positions; an open-addressing table gives the same ids.
+__device__ inline uint64_t position_hash(const double *v) {
+  uint64_t h = mix64(key_bits(v[0]));
+  h = mix64(h ^ key_bits(v[1]));
+  return mix64(h ^ key_bits(v[2]));
+}
+
+__device__ inline void weld_insert(const Dev &d) {
+  for (int64_t i = tid(); i < d.nv; i += stride()) {
+    const double *v = d.vertices + 3 * i;
+    uint32_t slot = uint32_t(position_hash(v)) & uint32_t(d.weld_mask);
+    for (int probe = 0; probe <= d.weld_mask; ++probe) {
+      int cur = atomicCAS(&d.weld_table[slot], -1, int(i));
+      if (cur == -1) break;
+      const double *w = d.vertices + 3 * int64_t(cur);
+      if (w[0] == v[0] && w[1] == v[1] && w[2] == v[2]) break;
+      slot = (slot + 1) & uint32_t(d.weld_mask);
+    }
+    atomicMin(&d.weld_min[slot], int(i));
+    d.weld_slot[i] = int(slot);
+  }
+}
+
+// The weld table, and input validation (kernels.py:309-350): finite values, face indices in
 // range, an invertible affine camera and a valid window and near plane.
 __global__ void k_validate(Dev d) {
+  weld_insert(d);
   for (int64_t i = tid(); i < max(max(d.nv, d.n), 1); i += stride()) {
     if (i < d.nv) {
       for (int j = 0; j < 3; ++j)
@@ -87,38 +135,10 @@ __global__ void k_validate(Dev d) {
   }
 }
 
-// Exact-position welding: the canonical id of a vertex is the smallest index
-// with an equal position, signed zeros equal (kernels.py:269-306).  The
-// reference sorts positions; an open-addressing table gives the same ids.
-__device__ inline uint64_t position_hash(const double *v) {
-  uint64_t h = mix64(key_bits(v[0]));
-  h = mix64(h ^ key_bits(v[1]));
-  return mix64(h ^ key_bits(v[2]));
-}
-
-__global__ void k_weld_insert(Dev d) {
-  for (int64_t i = tid(); i < d.nv; i += stride()) {
-    const double *v = d.vertices + 3 * i;
-    uint32_t slot = uint32_t(position_hash(v)) & uint32_t(d.weld_mask);
-    for (int probe = 0; probe <= d.weld_mask; ++probe) {
-      int cur = atomicCAS(&d.weld_table[slot], -1, int(i));
-      if (cur == -1) break;
-      const double *w = d.vertices + 3 * int64_t(cur);
-      if (w[0] == v[0] && w[1] == v[1] && w[2] == v[2]) break;
-      slot = (slot + 1) & uint32_t(d.weld_mask);
-    }
-    atomicMin(&d.weld_min[slot], int(i));
-    d.weld_slot[i] = int(slot);
-  }
-}
-
-__global__ void k_weld_resolve(Dev d) {
-  for (int64_t i = tid(); i < d.nv; i += stride()) d.canonical[i] = d.weld_min[d.weld_slot[i]];
-}
-
 // Camera transform, near clip, projection, depth plane, facing and window
-// clip of one triangle (kernels.py:353-468).
+// clip of one triangle (kernels.py:353-468), after the vertices' canonical ids.
 __global__ void k_project(Dev d) {
+  for (int64_t i = tid(); i < d.nv; i += stride()) d.canonical[i] = d.weld_min[d.weld_slot[i]];
   for (int64_t i = tid(); i < d.n; i += stride()) {
     V2 *out = d.src_v + kSourceVertices * i;
     if (d.status[kError] != 0) {
@@ -394,44 +414,43 @@ unsigned blocks(int64_t n) {
 
 }  // namespace
 
-cudaError_t stage_prepare_common(const Dev &d, SortScratch &s, TreeBuffers &source_tree,
-                                 cudaStream_t st) {
-  k_reset<<<1, 64, 0, st>>>(d);
+cudaError_t stage_prepare_common(const Dev &d, bool event, cudaStream_t st) {
+  FillList fills;
+  fills.add(d.weld_table, int64_t(d.weld_mask) + 1, 0xffffffffu);
+  fills.add(d.weld_min, int64_t(d.weld_mask) + 1, 0x7f7f7f7fu);
+  fills.add(d.ekey_table, int64_t(d.ekey_mask) + 1, 0xffffffffu);
+  fills.add(d.ekey_count, int64_t(d.ekey_mask) + 1, 0u);
+  if (event) {
+    const int64_t slots = int64_t(d.seg_mask) + 1;
+    fills.add(d.seg_table, slots, 0xffffffffu);
+    fills.add(d.seg_min, slots, 0x7f7f7f7fu);
+    // 0x7f bytes are 1.38e306 as binary64: above every finite depth we store.
+    fills.add(d.seg_za, slots, 0x7f7f7f7fu);
+    fills.add(d.seg_zb, slots, 0x7f7f7f7fu);
+    fills.add(d.seg_srca, slots, 0x7f7f7f7fu);
+    fills.add(d.seg_srcb, slots, 0x7f7f7f7fu);
+  }
+  k_reset<<<148 * 4, 256, 0, st>>>(d, fills);
   note_launch();
-  EDP_CHECK(cudaMemsetAsync(d.weld_table, 0xff, sizeof(int) * (int64_t(d.weld_mask) + 1), st));
-  EDP_CHECK(cudaMemsetAsync(d.weld_min, 0x7f, sizeof(int) * (int64_t(d.weld_mask) + 1), st));
-  EDP_CHECK(cudaMemsetAsync(d.ekey_table, 0xff, sizeof(unsigned long long) * (int64_t(d.ekey_mask) + 1), st));
-  EDP_CHECK(cudaMemsetAsync(d.ekey_count, 0, sizeof(int) * (int64_t(d.ekey_mask) + 1), st));
   k_validate<<<blocks(std::max(d.nv, d.n)), kBlock, 0, st>>>(d);
   note_launch();
-  if (d.nv > 0) {
-    k_weld_insert<<<blocks(d.nv), kBlock, 0, st>>>(d);
-    note_launch();
-    k_weld_resolve<<<blocks(d.nv), kBlock, 0, st>>>(d);
+  if (d.nv > 0 || d.n > 0) {
+    k_project<<<blocks(std::max(d.nv, d.n)), kBlock, 0, st>>>(d);
     note_launch();
   }
   if (d.n > 0) {
-    k_project<<<blocks(d.n), kBlock, 0, st>>>(d);
-    note_launch();
     k_edge_insert<<<blocks(3 * int64_t(d.n)), kBlock, 0, st>>>(d);
     note_launch();
     k_edge_mark<<<blocks(3 * int64_t(d.n)), kBlock, 0, st>>>(d);
     note_launch();
   }
-  EDP_CHECK(tree_build(source_tree, d.src_lo, d.src_hi, nullptr, d.n, false, s, st));
   return cudaGetLastError();
 }
 
 cudaError_t stage_prepare(const Dev &d, SortScratch &s, TreeBuffers &source_tree,
                           TreeBuffers &seg_tree, cudaStream_t st) {
-  EDP_CHECK(stage_prepare_common(d, s, source_tree, st));
-  EDP_CHECK(cudaMemsetAsync(d.seg_table, 0xff, sizeof(int) * (int64_t(d.seg_mask) + 1), st));
-  EDP_CHECK(cudaMemsetAsync(d.seg_min, 0x7f, sizeof(int) * (int64_t(d.seg_mask) + 1), st));
-  // 0x7f bytes are 1.38e306 as binary64: above every finite depth we store.
-  EDP_CHECK(cudaMemsetAsync(d.seg_za, 0x7f, sizeof(double) * (int64_t(d.seg_mask) + 1), st));
-  EDP_CHECK(cudaMemsetAsync(d.seg_zb, 0x7f, sizeof(double) * (int64_t(d.seg_mask) + 1), st));
-  EDP_CHECK(cudaMemsetAsync(d.seg_srca, 0x7f, sizeof(int) * (int64_t(d.seg_mask) + 1), st));
-  EDP_CHECK(cudaMemsetAsync(d.seg_srcb, 0x7f, sizeof(int) * (int64_t(d.seg_mask) + 1), st));
+  EDP_CHECK(stage_prepare_common(d, true, st));
+  EDP_CHECK(tree_build(source_tree, d.src_lo, d.src_hi, nullptr, d.n, false, s, st));
   if (d.n > 0) {
     k_segments<<<blocks(kSourceVertices * int64_t(d.n)), kBlock, 0, st>>>(d);
     note_launch();

@@ -51,7 +51,7 @@ __device__ inline int block_exclusive(int v, int *smem, int &total) {
 //
 // Three launches per scan and per pass (counts, their scan, the scatter) cost
 // small extractions mostly gaps between launches: 157 kernels outside the
-// subdivision loop, 83 now.  Replays: icospheres-640 0.81 -> 0.72 ms,
+// subdivision loop became 97.  Replays: icospheres-640 0.81 -> 0.72 ms,
 // knot-9702 1.14 -> 1.03, a batch of 16 small scenes 3.44 -> 3.03.
 enum Published : unsigned { kNothing = 0, kSum = 1, kPrefix = 2 };
 constexpr int kPollLimit = 1 << 22;
@@ -572,5 +572,44 @@ cudaError_t stage_mark(int stage, cudaStream_t st) {
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+}  // namespace edp
+
+namespace edp {
+// A conditional IF node of the graph being captured on `st` (default: not
+// taken): a kernel sets the handle, then the body is recorded on `body`
+// between conditional_begin and conditional_end.
+cudaError_t conditional_handle(cudaStream_t st, cudaGraphConditionalHandle &handle) {
+  cudaStreamCaptureStatus cs;
+  cudaGraph_t g = nullptr;
+  const cudaGraphNode_t *deps = nullptr;
+  size_t ndeps = 0;
+  EDP_CHECK(cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, &ndeps));
+  return cudaGraphConditionalHandleCreate(&handle, g, 0, cudaGraphCondAssignDefault);
+}
+
+cudaError_t conditional_begin(cudaStream_t st, cudaGraphConditionalHandle handle,
+                              cudaStream_t body) {
+  cudaStreamCaptureStatus cs;
+  cudaGraph_t g = nullptr;
+  const cudaGraphNode_t *deps = nullptr;
+  size_t ndeps = 0;
+  EDP_CHECK(cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, &ndeps));
+  alignas(cudaGraphNodeParams) unsigned char raw[sizeof(cudaGraphNodeParams)] = {};
+  cudaGraphNodeParams &params = *reinterpret_cast<cudaGraphNodeParams *>(raw);
+  params.type = cudaGraphNodeTypeConditional;
+  params.conditional.handle = handle;
+  params.conditional.type = cudaGraphCondTypeIf;
+  params.conditional.size = 1;
+  cudaGraphNode_t node;
+  EDP_CHECK(cudaGraphAddNode(&node, g, deps, ndeps, &params));
+  EDP_CHECK(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
+  return cudaStreamBeginCaptureToGraph(body, params.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                       cudaStreamCaptureModeRelaxed);
+}
+
+cudaError_t conditional_end(cudaStream_t body) {
+  cudaGraph_t captured = nullptr;
+  return cudaStreamEndCapture(body, &captured);
 }
 }  // namespace edp

@@ -26,8 +26,9 @@ __device__ inline int live_polygons(const Dev &d) { return d.sc[kLivePolygons]; 
 __device__ inline float lower_f(double x) { return __double2float_rd(x); }
 __device__ inline float upper_f(double x) { return __double2float_ru(x); }
 
-__global__ void k_rank_begin(Dev d) {
-  d.sc[kLivePolygons] = int(min(int64_t(d.status[kPolygons]), d.cap.regions));
+// Patch edges that have a slot.
+__device__ inline int patch_edges(const Dev &d) {
+  return int(min(int64_t(d.sc[kPatchEdges]), d.cap.vertices));
 }
 
 // counts[k] is the edge count of the k-th polygon in spatial order, so that
@@ -38,14 +39,7 @@ __global__ void k_polygon_init(Dev d) {
     d.counts[i] = d.out_n[d.order[i]];
     d.parents[i] = int(i);
     d.group_counts[i] = 0;
-  }
-}
-
-__global__ void k_check_edges(Dev d) {
-  int total = d.sc[kPatchEdges];
-  if (int64_t(total) > d.cap.vertices) {
-    set_error(d.status, kErrVertices);
-    d.sc[kPatchEdges] = int(d.cap.vertices);
+    d.group_fill[i] = 0;
   }
 }
 
@@ -54,6 +48,7 @@ __global__ void k_check_edges(Dev d) {
 // itself (components.py:287-327).
 __global__ void k_patch_edges(Dev d) {
   const int live = live_polygons(d);
+  if (tid() == 0 && int64_t(d.sc[kPatchEdges]) > d.cap.vertices) set_error(d.status, kErrVertices);
   for (int64_t o = tid(); o < live; o += stride()) {
     if (d.status[kError] != 0) return;
     const int i = d.order[o];
@@ -96,7 +91,7 @@ __device__ inline uint64_t point_key(V2 x) {
 // of another patch that has the same owner (components.py:330-366).  The key
 // is symmetric in the endpoints so both directions probe the same chain.
 __global__ void k_match_edges(Dev d) {
-  const int total = d.sc[kPatchEdges];
+  const int total = patch_edges(d);
   for (int64_t i = tid(); i < total; i += stride()) {
     if (d.status[kError] != 0) return;
     V2 a = d.starts[i], b = d.ends[i];
@@ -206,7 +201,7 @@ __global__ void k_seg_grid_fill(Dev d) {
 // contour hierarchy.  Any blocking segment decides, so the order does not
 // matter; the visit counter counts segments met until the first blocker.
 __global__ void k_connect(Dev d) {
-  const int total = d.sc[kPatchEdges];
+  const int total = patch_edges(d);
   const int leaves = *d.seg_tree.size;
   for (int64_t i = tid(); i < total; i += stride()) {
     if (d.status[kError] != 0) return;
@@ -269,24 +264,26 @@ __global__ void k_connect(Dev d) {
   }
 }
 
-__global__ void k_roots(Dev d, int connected) {
+// Each polygon's representative, and its canonical interior sample: the
+// vertex mean accumulated from the lexicographically smallest vertex, so that
+// rotated copies of one footprint share bit-identical samples
+// (event_kernels.py:28-48).  Also clears what the rank stage fills next.
+__global__ void k_samples(Dev d, int connected) {
   const int live = live_polygons(d);
+  if (tid() == 0) d.status[kLayers] = 0;
+  for (int64_t c = tid(); c < kCells; c += stride()) {
+    d.cell_min[c] = 0x7fffffff;
+    d.cell_valid[c] = 0;
+    d.cell_bounds[4 * c + 0] = 1.0e30;
+    d.cell_bounds[4 * c + 1] = 1.0e30;
+    d.cell_bounds[4 * c + 2] = -1.0e30;
+    d.cell_bounds[4 * c + 3] = -1.0e30;
+  }
   int components = 0;
   for (int64_t i = tid(); i < live; i += stride()) {
-    int r = connected ? uf_root(d.parents, int(i)) : int(i);
+    const int r = connected ? uf_root(d.parents, int(i)) : int(i);
     d.reps[i] = r;
     components += r == int(i);
-  }
-  if (components) add_metric(d, kRankComponents, d.propagate_ranks ? components : 0);
-}
-
-// Canonical interior sample of each polygon's representative: the vertex mean
-// accumulated from the lexicographically smallest vertex, so that rotated
-// copies of one footprint share bit-identical samples (event_kernels.py:28-48).
-__global__ void k_samples(Dev d) {
-  const int live = live_polygons(d);
-  for (int64_t i = tid(); i < live; i += stride()) {
-    int r = d.reps[i];
     const V2 *p = d.out_v + int64_t(kMaxVertices) * r;
     int n = d.out_n[r];
     int anchor = 0;
@@ -296,6 +293,7 @@ __global__ void k_samples(Dev d) {
     for (int j = 0; j < n; ++j) x = x + p[(anchor + j) % n] / double(n);
     d.samples[i] = x;
   }
+  if (components) add_metric(d, kRankComponents, d.propagate_ranks ? components : 0);
 }
 
 __device__ inline int cell_of(V2 x) {
@@ -340,23 +338,6 @@ __global__ void k_group_insert(Dev d) {
         atomic_max_double(&d.cell_bounds[4 * c + 3], hy);
       }
     }
-  }
-}
-
-__global__ void k_group_resolve(Dev d) {
-  const int live = live_polygons(d);
-  for (int64_t i = tid(); i < live; i += stride()) d.groups[i] = d.sample_min[d.sample_slot[i]];
-}
-
-__global__ void k_cells_reset(Dev d) {
-  int c = int(tid());
-  if (c < kCells) {
-    d.cell_min[c] = 0x7fffffff;
-    d.cell_valid[c] = 0;
-    d.cell_bounds[4 * c + 0] = 1.0e30;
-    d.cell_bounds[4 * c + 1] = 1.0e30;
-    d.cell_bounds[4 * c + 2] = -1.0e30;
-    d.cell_bounds[4 * c + 3] = -1.0e30;
   }
 }
 
@@ -468,15 +449,19 @@ __global__ void k_certify_heavy(Dev d) {
   }
 }
 
-__global__ void k_apply_cells(Dev d) {
+// Each polygon's query group: its sample's, or its certified cell's.
+__global__ void k_groups(Dev d) {
   const int live = live_polygons(d);
   for (int64_t i = tid(); i < live; i += stride()) {
-    int c = cell_of(d.samples[i]);
-    if (d.cell_valid[c] != 0) {
-      int root = d.cell_min[c];
-      d.groups[i] = root;
-      if (root == int(i)) add_metric(d, kCertifiedBeams, 1);
+    int group = d.sample_min[d.sample_slot[i]];
+    if (d.share_regions) {
+      const int c = cell_of(d.samples[i]);
+      if (d.cell_valid[c] != 0) {
+        group = d.cell_min[c];
+        if (group == int(i)) add_metric(d, kCertifiedBeams, 1);
+      }
     }
+    d.groups[i] = group;
   }
 }
 
@@ -589,6 +574,12 @@ __device__ inline bool edges_exclude(const Dev &d, int s, float x, float y) {
 }
 
 __global__ void k_ray_grid_count(Dev d) {
+  // Each source's leaf in the source hierarchy (the order of its binary walk).
+  const int leaves = *d.source_tree.size;
+  for (int64_t leaf = tid(); leaf < leaves; leaf += stride()) {
+    const int s = d.source_tree.ids[leaf];
+    if (s < d.n) d.leaf_of[s] = int(leaf);
+  }
   for (int64_t s = tid(); s < d.n; s += stride()) {
     edge_functions(d, s);
     int cx0, cx1, cy0, cy1;
@@ -619,16 +610,6 @@ __global__ void k_ray_grid_fill(Dev d) {
         d.ray_entries[e] = int(s);
         d.ray_boxes[e] = box;
       }
-  }
-}
-
-// Each source's leaf in the source hierarchy (the order of its binary walk).
-__global__ void k_leaf_of(Dev d) {
-  const int count = d.n;
-  const int leaves = *d.source_tree.size;
-  for (int64_t leaf = tid(); leaf < leaves; leaf += stride()) {
-    const int s = d.source_tree.ids[leaf];
-    if (s < count) d.leaf_of[s] = int(leaf);
   }
 }
 
@@ -1015,13 +996,6 @@ __global__ void k_ray_exact(Dev d) {
   }
 }
 
-__global__ void k_check_hits(Dev d) {
-  long long total = d.metrics[kRayHits];
-  if (total > d.cap.hits) set_error(d.status, kErrHits);
-  d.sc[kLiveHits] = int(min(total, (long long)d.cap.hits));
-  d.sc[kSortHits] = 0;
-}
-
 // Hits of one ray group are ordered by (depth, source) within the group.  A
 // group holds one hit per source along its ray, so groups are as deep as the
 // scene's depth complexity: up to kGroupSort hits are sorted by one thread in
@@ -1032,17 +1006,23 @@ constexpr int kGroupSort = 128;
 // thread's insertion sort of a deep group held its warp's other lanes.
 constexpr int kWarpSort = 32;
 
-__global__ void k_group_sizes(Dev d) {
+// The live hits, and whether some group is too deep for k_group_sort: then
+// every hit goes through the global passes, in a graph by their node's
+// condition.  (kSortHits is zero here: the subdivision left its counter so.)
+__global__ void k_group_sizes(Dev d, cudaGraphConditionalHandle handle, int conditional) {
   const int live = live_polygons(d);
+  const long long total = d.metrics[kRayHits];
+  const int hits = int(min(total, (long long)d.cap.hits));
+  if (tid() == 0) {
+    if (total > d.cap.hits) set_error(d.status, kErrHits);
+    d.sc[kLiveHits] = hits;
+  }
   bool large = false;
   for (int64_t i = tid(); i < live; i += stride()) large |= d.group_counts[i] > kGroupSort;
-  if (__any_sync(0xffffffffu, large) && (threadIdx.x & 31) == 0) d.sc[kSortHits] = d.sc[kLiveHits];
-}
-
-// The condition of the global hit passes: some group is too deep for
-// k_group_sort.
-__global__ void k_sort_switch(Dev d, cudaGraphConditionalHandle handle) {
-  cudaGraphSetConditional(handle, d.sc[kSortHits] != 0 ? 1u : 0u);
+  if (__any_sync(0xffffffffu, large) && (threadIdx.x & 31) == 0) {
+    d.sc[kSortHits] = hits;
+    if (conditional && hits) cudaGraphSetConditional(handle, 1u);
+  }
 }
 
 // Place each hit in its group's range (group_offsets is the scan of
@@ -1338,8 +1318,6 @@ __global__ void k_assign(Dev d, int deferred_pass) {
   if constexpr (F == 2) order.flush(d, kPredOrder);
 }
 
-__global__ void k_layers_reset(Dev d) { d.status[kLayers] = 0; }
-
 // ---------------------------------------------------------------- merging
 // Optional convex coalescing (components.py:274-395).  A matched pair of
 // patch edges whose polygons share source and layer proposes a merge when the
@@ -1347,7 +1325,7 @@ __global__ void k_layers_reset(Dev d) { d.status[kLayers] = 0; }
 // proposing edge, and a pair merges when both of its polygons chose it.  Each
 // polygon is in at most one merge, so merges never touch the same slot.
 __global__ void k_merge_propose(Dev d) {
-  const int total = d.sc[kPatchEdges];
+  const int total = patch_edges(d);
   for (int64_t t = tid(); t < total; t += stride()) {
     if (d.status[kError] != 0) return;
     const int other = d.partners[t];
@@ -1371,7 +1349,7 @@ __global__ void k_merge_propose(Dev d) {
 // edge, then b's vertices but the shared two; exactly collinear vertices are
 // dropped.  The merged polygon replaces a, and b is emptied.
 __global__ void k_merge(Dev d) {
-  const int total = d.sc[kPatchEdges];
+  const int total = patch_edges(d);
   long long merged = 0;
   for (int64_t t = tid(); t < total; t += stride()) {
     if (d.status[kError] != 0) break;
@@ -1458,17 +1436,17 @@ int bits_for(int64_t n) {
 
 cudaError_t stage_rank(const Dev &d, SortScratch &s, cudaStream_t st) {
   const int64_t R = d.cap.regions, E = d.cap.vertices;
-  k_rank_begin<<<1, 1, 0, st>>>(d);
-  note_launch();
-  EDP_CHECK(order_polygons(d, false, s, st));
-  k_polygon_init<<<blocks(R), kBlock, 0, st>>>(d);
-  note_launch();
+  if (d.merge_regions) {  // merging breaks ties by this order
+    EDP_CHECK(sort_polygons(d, s, st));
+    k_polygon_init<<<blocks(R), kBlock, 0, st>>>(d);
+    note_launch();
+  } else {
+    EDP_CHECK(order_polygons(d, false, s, st));
+  }
   EDP_CHECK(stage_mark(EDP_STAGE_RANK_ORDER, st));
   const bool connected = d.propagate_ranks || d.merge_regions;
   if (connected) {
     EDP_CHECK(scan_exclusive(d.counts, d.offsets, d.sc + kLivePolygons, R, d.sc + kPatchEdges, s, st));
-    k_check_edges<<<1, 1, 0, st>>>(d);
-    note_launch();
     k_patch_edges<<<blocks(R), kBlock, 0, st>>>(d);
     note_launch();
     EDP_CHECK(cudaMemsetAsync(d.edge_hash, 0xff, sizeof(int) * (int64_t(d.edge_hash_mask) + 1), st));
@@ -1476,7 +1454,6 @@ cudaError_t stage_rank(const Dev &d, SortScratch &s, cudaStream_t st) {
     note_launch();
     if (d.propagate_ranks) {
       const int64_t cells = int64_t(d.grid_size) * d.grid_size;
-      EDP_CHECK(cudaMemsetAsync(d.seg_count, 0, sizeof(int) * cells, st));
       k_seg_grid_count<<<blocks(kSourceVertices * int64_t(d.n)), kBlock, 0, st>>>(d);
       note_launch();
       EDP_CHECK(scan_exclusive(d.seg_count, d.seg_start, d.sc + kRayGridCells, cells,
@@ -1488,18 +1465,12 @@ cudaError_t stage_rank(const Dev &d, SortScratch &s, cudaStream_t st) {
     note_launch();
   }
   EDP_CHECK(stage_mark(EDP_STAGE_RANK_CONNECTIVITY, st));
-  k_roots<<<blocks(R), kBlock, 0, st>>>(d, d.propagate_ranks ? 1 : 0);
-  note_launch();
-  k_samples<<<blocks(R), kBlock, 0, st>>>(d);
+  k_samples<<<blocks(R), kBlock, 0, st>>>(d, d.propagate_ranks ? 1 : 0);
   note_launch();
   EDP_CHECK(stage_mark(EDP_STAGE_RANK_SAMPLES, st));
   EDP_CHECK(cudaMemsetAsync(d.sample_table, 0xff, sizeof(int) * (int64_t(d.sample_mask) + 1), st));
   EDP_CHECK(cudaMemsetAsync(d.sample_min, 0x7f, sizeof(int) * (int64_t(d.sample_mask) + 1), st));
-  k_cells_reset<<<kCells / 128, 128, 0, st>>>(d);
-  note_launch();
   k_group_insert<<<blocks(R), kBlock, 0, st>>>(d);
-  note_launch();
-  k_group_resolve<<<blocks(R), kBlock, 0, st>>>(d);
   note_launch();
   EDP_CHECK(stage_mark(EDP_STAGE_RANK_QUERY_GROUPS, st));
   if (d.share_regions) {
@@ -1507,15 +1478,12 @@ cudaError_t stage_rank(const Dev &d, SortScratch &s, cudaStream_t st) {
     note_launch();
     k_certify_heavy<<<kHeavyBlocks, kHeavyBlock, 0, st>>>(d);
     note_launch();
-    k_apply_cells<<<blocks(R), kBlock, 0, st>>>(d);
-    note_launch();
   }
+  k_groups<<<blocks(R), kBlock, 0, st>>>(d);
+  note_launch();
   EDP_CHECK(stage_mark(EDP_STAGE_RANK_CERTIFY, st));
   {
     const int64_t cells = int64_t(d.grid_size) * d.grid_size;
-    EDP_CHECK(cudaMemsetAsync(d.ray_count, 0, sizeof(int) * cells, st));
-    k_leaf_of<<<blocks(d.n), kBlock, 0, st>>>(d);
-    note_launch();
     k_ray_grid_count<<<blocks(d.n), kBlock, 0, st>>>(d);
     note_launch();
     EDP_CHECK(scan_exclusive(d.ray_count, d.ray_start, d.sc + kRayGridCells, cells,
@@ -1550,38 +1518,18 @@ cudaError_t stage_rank(const Dev &d, SortScratch &s, cudaStream_t st) {
   note_launch();
   EDP_CHECK(stage_mark(EDP_STAGE_RANK_RAY_HEAVY, st));
   EDP_CHECK(scan_exclusive(d.group_counts, d.group_offsets, d.sc + kLivePolygons, R, nullptr, s, st));
-  k_check_hits<<<1, 1, 0, st>>>(d);
-  note_launch();
-  k_group_sizes<<<blocks(R), kBlock, 0, st>>>(d);
-  note_launch();
   // Global passes: over all hits when some group is large, else over none.
   // In a captured graph they sit in a conditional IF node, so an extraction
-  // whose groups all sort in k_group_sort launches none of their 40-odd
+  // whose groups all sort in k_group_sort launches none of their 30-odd
   // kernels; run eagerly, they take their count (zero) from the device.
   cudaStream_t radix = st;
   const bool branch = d.use_handle && d.aux_stream;
+  cudaGraphConditionalHandle handle{};
+  if (branch) EDP_CHECK(conditional_handle(st, handle));
+  k_group_sizes<<<blocks(R), kBlock, 0, st>>>(d, handle, branch ? 1 : 0);
+  note_launch();
   if (branch) {
-    cudaStreamCaptureStatus cs;
-    cudaGraph_t g = nullptr;
-    const cudaGraphNode_t *deps = nullptr;
-    size_t ndeps = 0;
-    EDP_CHECK(cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, &ndeps));
-    cudaGraphConditionalHandle handle;
-    EDP_CHECK(cudaGraphConditionalHandleCreate(&handle, g, 0, cudaGraphCondAssignDefault));
-    k_sort_switch<<<1, 1, 0, st>>>(d, handle);
-    note_launch();
-    EDP_CHECK(cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, &ndeps));
-    alignas(cudaGraphNodeParams) unsigned char raw[sizeof(cudaGraphNodeParams)] = {};
-    cudaGraphNodeParams &params = *reinterpret_cast<cudaGraphNodeParams *>(raw);
-    params.type = cudaGraphNodeTypeConditional;
-    params.conditional.handle = handle;
-    params.conditional.type = cudaGraphCondTypeIf;
-    params.conditional.size = 1;
-    cudaGraphNode_t node;
-    EDP_CHECK(cudaGraphAddNode(&node, g, deps, ndeps, &params));
-    EDP_CHECK(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
-    EDP_CHECK(cudaStreamBeginCaptureToGraph(d.aux_stream, params.conditional.phGraph_out[0],
-                                            nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
+    EDP_CHECK(conditional_begin(st, handle, d.aux_stream));
     radix = d.aux_stream;
   }
   const int pass_bits[3] = {bits_for(d.n), 64, bits_for(R)};
@@ -1595,14 +1543,10 @@ cudaError_t stage_rank(const Dev &d, SortScratch &s, cudaStream_t st) {
                             d.sc + kSortHits, d.cap.hits, pass_bits[stage], s, radix);
   }
   if (branch) {
-    cudaGraph_t body = nullptr;
-    cudaError_t end = cudaStreamEndCapture(d.aux_stream, &body);
-    EDP_CHECK(sorted);
-    EDP_CHECK(end);
+    EDP_CHECK(conditional_end(d.aux_stream));
     forget_launches(launch_count() - body_first);
   }
   EDP_CHECK(sorted);
-  EDP_CHECK(cudaMemsetAsync(d.group_fill, 0, sizeof(int) * R, st));
   k_hit_place<<<blocks(d.cap.hits), kBlock, 0, st>>>(d);
   note_launch();
   if (split_exact) {
@@ -1618,8 +1562,6 @@ cudaError_t stage_rank(const Dev &d, SortScratch &s, cudaStream_t st) {
   }
   note_launch();
   EDP_CHECK(stage_mark(EDP_STAGE_RANK_HIT_SORT, st));
-  k_layers_reset<<<1, 1, 0, st>>>(d);
-  note_launch();
   if (split_exact) {
     k_assign<4><<<blocks(R), kBlock, 0, st>>>(d, 0);
     note_launch();

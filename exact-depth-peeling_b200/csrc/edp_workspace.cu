@@ -62,11 +62,12 @@ int cuda_fail(cudaError_t e, const char *site) { return edp::record_cuda_failure
 template <class T>
 cudaError_t alloc(edp_peeler *p, T **ptr, int64_t count) {
   if (count < 1) count = 1;
-  cudaError_t e = cudaMalloc(reinterpret_cast<void **>(ptr), sizeof(T) * size_t(count));
+  const size_t bytes = (sizeof(T) * size_t(count) + 15) / 16 * 16;  // whole 16-byte words
+  cudaError_t e = cudaMalloc(reinterpret_cast<void **>(ptr), bytes);
   if (e == cudaSuccess) {
     p->allocations.push_back(*ptr);
-    p->bytes += int64_t(sizeof(T)) * count;
-    e = cudaMemset(*ptr, 0, sizeof(T) * size_t(count));
+    p->bytes += int64_t(bytes);
+    e = cudaMemset(*ptr, 0, bytes);
   }
   return e;
 }
@@ -121,6 +122,10 @@ cudaError_t allocate_shared(edp_peeler *p) {
   EDP_CHECK(alloc(p, &d.order_keys_tmp, R));
   EDP_CHECK(alloc(p, &d.order, R));
   EDP_CHECK(alloc(p, &d.order_tmp, R));
+  d.order_bits = 12;
+  while (d.order_bits < 24 && (int64_t(1) << d.order_bits) < 16 * R) ++d.order_bits;
+  EDP_CHECK(alloc(p, &d.order_count, int64_t(1) << d.order_bits));
+  EDP_CHECK(alloc(p, &d.order_start, int64_t(1) << d.order_bits));
   EDP_CHECK(alloc(p, &d.counts, R));
   EDP_CHECK(alloc(p, &d.offsets, R));
   EDP_CHECK(alloc(p, &d.bverts, E));
@@ -167,6 +172,7 @@ cudaError_t allocate_scratch(edp_peeler *p, int64_t largest_sort, int64_t larges
   s.tiles = ceil_div(largest_sort, kSortTile);
   s.scan_tiles = ceil_div(largest_scan, kScanTile);
   EDP_CHECK(alloc(p, &s.hist, 256 * kSortPasses));
+  s.scan_tiles = std::max<int64_t>(s.scan_tiles, (int64_t(1) << p->d.order_bits) / kScanTile);
   EDP_CHECK(alloc(p, &s.look_back.words, std::max(256 * s.tiles, s.scan_tiles)));
   EDP_CHECK(alloc(p, &s.look_back.control, 3));
   s.look_back.error = p->d.status + kError;
@@ -341,7 +347,6 @@ cudaError_t run_finish(edp_peeler *p, const Dev &d, cudaStream_t st) {
     EDP_CHECK(stage_rank(d, p->scratch, st));
   } else {  // its finish is timed as the assignment stage
     EDP_CHECK(stage_mark(EDP_STAGE_RANK_HIT_SORT, st));
-    EDP_CHECK(stage_device_finish(d, st));
     EDP_CHECK(stage_mark(EDP_STAGE_RANK_MERGE, st));
   }
   EDP_CHECK(stage_mesh_index(d, p->scratch, p->point_tree, st));
@@ -691,6 +696,8 @@ int edp_run_stage(edp_peeler *p, int32_t stage) {
       e = stage_mesh_index(d, p->scratch, p->point_tree, p->stream);
     } else {
       e = cudaMemsetAsync(d.status + kTriangles, 0, sizeof(int), p->stream);
+      if (e == cudaSuccess)
+        e = cudaMemsetAsync(d.sc + kHeavyPolygons, 0, sizeof(int), p->stream);
       if (e == cudaSuccess) e = stage_mesh_emit(d, p->stream);
     }
     cudaGraph_t g = nullptr;
