@@ -29,6 +29,15 @@ inline int64_t pow2_at_least(int64_t v) {
   while (p < v) p <<= 1;
   return p;
 }
+// Fill 16-byte words with one 32-bit value, thread `t` of `threads`.  The big
+// tables are cleared by the kernel before the one that fills them, which then
+// finds them in L2.
+__device__ inline void fill_words(void *at, int64_t quads, unsigned word, int64_t t,
+                                  int64_t threads) {
+  uint4 *q = reinterpret_cast<uint4 *>(at);
+  for (; t < quads; t += threads) q[t] = make_uint4(word, word, word, word);
+}
+
 inline unsigned grid_for(int64_t n, int block) {
   int64_t g = ceil_div(n > 0 ? n : 1, block);
   return static_cast<unsigned>(g);
@@ -286,6 +295,7 @@ struct Dev {
   int *tri_src, *tri_layer;
   unsigned long long cond_handle;  // cudaGraphConditionalHandle of the subdivision loop
   int use_handle;
+  int use_side;  // the workspace's own graph has the side branch
 
   // DevicePeeler (iterative clipping) only.
   float4 *contour_lo, *contour_hi;  // per source: box of its contour edges
@@ -351,8 +361,22 @@ cudaError_t conditional_end(cudaStream_t body);
 
 // Stage launchers (edp_prepare.cu, edp_frontier.cu, edp_rank.cu, edp_mesh.cu).  Each
 // enqueues kernels on `st`.
+// The branch of a captured extraction that runs beside its preparation and
+// subdivision (Dev::use_side): what only the rank stage reads.  Otherwise that
+// runs in line.
+struct Side {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t forked = nullptr, joined = nullptr;
+  SortScratch scratch;  // its own: its scans run beside the main branch's
+};
+
 cudaError_t stage_prepare(const Dev &d, SortScratch &s, TreeBuffers &source_tree,
-                          TreeBuffers &seg_tree, cudaStream_t st);
+                          TreeBuffers &seg_tree, Side &side, cudaStream_t st);
+cudaError_t side_join(const Dev &d, Side &side, cudaStream_t st);
+// The grids of the rays (over the sources) and of the connection test (over
+// the contour segments).
+cudaError_t stage_ray_grid(const Dev &d, SortScratch &s, cudaStream_t st);
+cudaError_t stage_segment_grid(const Dev &d, SortScratch &s, cudaStream_t st);
 cudaError_t stage_lists(const Dev &d, cudaStream_t st);
 cudaError_t stage_step(const Dev &d, cudaStream_t st);
 cudaError_t stage_rank(const Dev &d, SortScratch &s, cudaStream_t st);

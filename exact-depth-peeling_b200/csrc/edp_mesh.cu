@@ -32,6 +32,7 @@ __global__ void k_scatter(Dev d) {
   const int live = d.sc[kLivePolygons];
   const int total = d.sc[kLiveVertices];  // or the capacity, once clamped below
   const bool fits = int64_t(total) <= d.cap.vertices;
+  fill_words(d.point_table, ceil_div(int64_t(d.point_mask) + 1, 4), 0xffffffffu, tid(), stride());
   if (tid() == 0) {
     const int layers = d.status[kLayers];
     const bool on = d.status[kError] == 0 && fits && layers <= d.grid_layers;
@@ -877,7 +878,6 @@ cudaError_t stage_mesh_index(const Dev &d, SortScratch &s, TreeBuffers &point_tr
   const int64_t R = d.cap.regions, E = d.cap.vertices;
   EDP_CHECK(order_polygons(d, true, s, st));
   EDP_CHECK(scan_exclusive(d.counts, d.offsets, d.sc + kLivePolygons, R, d.sc + kLiveVertices, s, st));
-  EDP_CHECK(cudaMemsetAsync(d.point_table, 0xff, sizeof(int) * (int64_t(d.point_mask) + 1), st));
   const int64_t cells = int64_t(d.grid_layers) * d.point_grid * d.point_grid;
   k_scatter<<<blocks(R), kBlock, 0, st>>>(d);
   note_launch();

@@ -49,6 +49,7 @@ __global__ void k_polygon_init(Dev d) {
 __global__ void k_patch_edges(Dev d) {
   const int live = live_polygons(d);
   if (tid() == 0 && int64_t(d.sc[kPatchEdges]) > d.cap.vertices) set_error(d.status, kErrVertices);
+  fill_words(d.edge_hash, ceil_div(int64_t(d.edge_hash_mask) + 1, 4), 0xffffffffu, tid(), stride());
   for (int64_t o = tid(); o < live; o += stride()) {
     if (d.status[kError] != 0) return;
     const int i = d.order[o];
@@ -271,6 +272,9 @@ __global__ void k_connect(Dev d) {
 __global__ void k_samples(Dev d, int connected) {
   const int live = live_polygons(d);
   if (tid() == 0) d.status[kLayers] = 0;
+  const int64_t quads = ceil_div(int64_t(d.sample_mask) + 1, 4);
+  fill_words(d.sample_table, quads, 0xffffffffu, tid(), stride());
+  fill_words(d.sample_min, quads, 0x7f7f7f7fu, tid(), stride());
   for (int64_t c = tid(); c < kCells; c += stride()) {
     d.cell_min[c] = 0x7fffffff;
     d.cell_valid[c] = 0;
@@ -1434,6 +1438,28 @@ int bits_for(int64_t n) {
 
 }  // namespace
 
+cudaError_t stage_ray_grid(const Dev &d, SortScratch &s, cudaStream_t st) {
+  const int64_t cells = int64_t(d.grid_size) * d.grid_size;
+  k_ray_grid_count<<<blocks(d.n), kBlock, 0, st>>>(d);
+  note_launch();
+  EDP_CHECK(scan_exclusive(d.ray_count, d.ray_start, d.sc + kRayGridCells, cells,
+                           d.ray_start + cells, s, st));
+  k_ray_grid_fill<<<blocks(d.n), kBlock, 0, st>>>(d);
+  note_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t stage_segment_grid(const Dev &d, SortScratch &s, cudaStream_t st) {
+  const int64_t cells = int64_t(d.grid_size) * d.grid_size;
+  k_seg_grid_count<<<blocks(kSourceVertices * int64_t(d.n)), kBlock, 0, st>>>(d);
+  note_launch();
+  EDP_CHECK(scan_exclusive(d.seg_count, d.seg_start, d.sc + kRayGridCells, cells,
+                           d.seg_start + cells, s, st));
+  k_seg_grid_fill<<<blocks(kSourceVertices * int64_t(d.n)), kBlock, 0, st>>>(d);
+  note_launch();
+  return cudaGetLastError();
+}
+
 cudaError_t stage_rank(const Dev &d, SortScratch &s, cudaStream_t st) {
   const int64_t R = d.cap.regions, E = d.cap.vertices;
   if (d.merge_regions) {  // merging breaks ties by this order
@@ -1449,27 +1475,17 @@ cudaError_t stage_rank(const Dev &d, SortScratch &s, cudaStream_t st) {
     EDP_CHECK(scan_exclusive(d.counts, d.offsets, d.sc + kLivePolygons, R, d.sc + kPatchEdges, s, st));
     k_patch_edges<<<blocks(R), kBlock, 0, st>>>(d);
     note_launch();
-    EDP_CHECK(cudaMemsetAsync(d.edge_hash, 0xff, sizeof(int) * (int64_t(d.edge_hash_mask) + 1), st));
     k_match_edges<<<blocks(E), kBlock, 0, st>>>(d);
     note_launch();
     if (d.propagate_ranks) {
-      const int64_t cells = int64_t(d.grid_size) * d.grid_size;
-      k_seg_grid_count<<<blocks(kSourceVertices * int64_t(d.n)), kBlock, 0, st>>>(d);
-      note_launch();
-      EDP_CHECK(scan_exclusive(d.seg_count, d.seg_start, d.sc + kRayGridCells, cells,
-                               d.seg_start + cells, s, st));
-      k_seg_grid_fill<<<blocks(kSourceVertices * int64_t(d.n)), kBlock, 0, st>>>(d);
-      note_launch();
       k_connect<<<blocks(E), kBlock, 0, st>>>(d);
+      note_launch();
     }
-    note_launch();
   }
   EDP_CHECK(stage_mark(EDP_STAGE_RANK_CONNECTIVITY, st));
   k_samples<<<blocks(R), kBlock, 0, st>>>(d, d.propagate_ranks ? 1 : 0);
   note_launch();
   EDP_CHECK(stage_mark(EDP_STAGE_RANK_SAMPLES, st));
-  EDP_CHECK(cudaMemsetAsync(d.sample_table, 0xff, sizeof(int) * (int64_t(d.sample_mask) + 1), st));
-  EDP_CHECK(cudaMemsetAsync(d.sample_min, 0x7f, sizeof(int) * (int64_t(d.sample_mask) + 1), st));
   k_group_insert<<<blocks(R), kBlock, 0, st>>>(d);
   note_launch();
   EDP_CHECK(stage_mark(EDP_STAGE_RANK_QUERY_GROUPS, st));
@@ -1482,15 +1498,6 @@ cudaError_t stage_rank(const Dev &d, SortScratch &s, cudaStream_t st) {
   k_groups<<<blocks(R), kBlock, 0, st>>>(d);
   note_launch();
   EDP_CHECK(stage_mark(EDP_STAGE_RANK_CERTIFY, st));
-  {
-    const int64_t cells = int64_t(d.grid_size) * d.grid_size;
-    k_ray_grid_count<<<blocks(d.n), kBlock, 0, st>>>(d);
-    note_launch();
-    EDP_CHECK(scan_exclusive(d.ray_count, d.ray_start, d.sc + kRayGridCells, cells,
-                             d.ray_start + cells, s, st));
-    k_ray_grid_fill<<<blocks(d.n), kBlock, 0, st>>>(d);
-    note_launch();
-  }
   EDP_CHECK(stage_mark(EDP_STAGE_RANK_RAY_GRID, st));
   // Filtered binary64 predicates: the filter-only kernels, then exact passes
   // over what their filters left undecided (same results as form 3 alone).
@@ -1572,7 +1579,6 @@ cudaError_t stage_rank(const Dev &d, SortScratch &s, cudaStream_t st) {
   note_launch();
   EDP_CHECK(stage_mark(EDP_STAGE_RANK_ASSIGN, st));
   if (d.merge_regions) {
-    EDP_CHECK(cudaMemsetAsync(d.merge_choice, 0x7f, sizeof(int) * R, st));
     k_merge_propose<<<blocks(E), kBlock, 0, st>>>(d);
     note_launch();
     k_merge<<<blocks(E), kBlock, 0, st>>>(d);

@@ -25,6 +25,7 @@ struct edp_peeler {
   cudaStream_t stream = nullptr;
   cudaStream_t body_stream = nullptr;
   cudaStream_t round_stream = nullptr;  // records the DevicePeeler's clipping rounds
+  Side side;                            // EventPeeler: the branch beside its subdivision
   SortScratch scratch;
   TreeBuffers source_tree, seg_tree, point_tree;  // seg_tree holds contours for DevicePeeler
   TreeBuffers residual_tree;
@@ -167,12 +168,11 @@ cudaError_t allocate_shared(edp_peeler *p) {
   return cudaSuccess;
 }
 
-cudaError_t allocate_scratch(edp_peeler *p, int64_t largest_sort, int64_t largest_scan) {
-  SortScratch &s = p->scratch;
+cudaError_t allocate_scratch(edp_peeler *p, SortScratch &s, int64_t largest_sort,
+                             int64_t largest_scan) {
   s.tiles = ceil_div(largest_sort, kSortTile);
   s.scan_tiles = ceil_div(largest_scan, kScanTile);
   EDP_CHECK(alloc(p, &s.hist, 256 * kSortPasses));
-  s.scan_tiles = std::max<int64_t>(s.scan_tiles, (int64_t(1) << p->d.order_bits) / kScanTile);
   EDP_CHECK(alloc(p, &s.look_back.words, std::max(256 * s.tiles, s.scan_tiles)));
   EDP_CHECK(alloc(p, &s.look_back.control, 3));
   s.look_back.error = p->d.status + kError;
@@ -283,7 +283,10 @@ cudaError_t allocate_event(edp_peeler *p) {
   int64_t scan = R > E ? R : E;
   scan = S > scan ? S : scan;  // the segment-slot compaction
   scan = std::max(scan, int64_t(d.grid_layers) * d.point_grid * d.point_grid);
-  return allocate_scratch(p, largest, scan);
+  scan = std::max(scan, int64_t(1) << d.order_bits);
+  EDP_CHECK(allocate_scratch(p, p->side.scratch, p->source_tree.leaves_cap,
+                             int64_t(d.grid_size) * d.grid_size));
+  return allocate_scratch(p, p->scratch, largest, scan);
 }
 
 cudaError_t allocate_device(edp_peeler *p) {
@@ -326,15 +329,16 @@ cudaError_t allocate_device(edp_peeler *p) {
   for (int64_t v : {p->point_tree.leaves_cap, p->seg_tree.leaves_cap, p->source_tree.leaves_cap,
                     p->residual_tree.leaves_cap})
     largest = v > largest ? v : largest;
-  return allocate_scratch(p, largest,
-                         std::max({R, E, int64_t(d.grid_layers) * d.point_grid * d.point_grid}));
+  return allocate_scratch(p, p->scratch, largest,
+                          std::max({R, E, int64_t(d.grid_layers) * d.point_grid * d.point_grid,
+                                    int64_t(1) << d.order_bits}));
 }
 
 // Stage sequence of each peeler.  The loop body runs while the device sets
 // the condition: subdivision rounds (EventPeeler) or layer passes
 // (DevicePeeler).
 cudaError_t run_prepare(edp_peeler *p, const Dev &d, cudaStream_t st) {
-  return p->method == 0 ? stage_prepare(d, p->scratch, p->source_tree, p->seg_tree, st)
+  return p->method == 0 ? stage_prepare(d, p->scratch, p->source_tree, p->seg_tree, p->side, st)
                         : stage_device_prepare(d, p->scratch, p->source_tree, p->seg_tree, st);
 }
 cudaError_t run_body(edp_peeler *p, const Dev &d, cudaStream_t st) {
@@ -344,6 +348,7 @@ cudaError_t run_body(edp_peeler *p, const Dev &d, cudaStream_t st) {
 }
 cudaError_t run_finish(edp_peeler *p, const Dev &d, cudaStream_t st) {
   if (p->method == 0) {
+    EDP_CHECK(side_join(d, p->side, st));
     EDP_CHECK(stage_rank(d, p->scratch, st));
   } else {  // its finish is timed as the assignment stage
     EDP_CHECK(stage_mark(EDP_STAGE_RANK_HIT_SORT, st));
@@ -357,8 +362,9 @@ cudaError_t run_finish(edp_peeler *p, const Dev &d, cudaStream_t st) {
 // The whole extraction, recorded on `st`.  With `graph` the loop becomes a
 // conditional WHILE node of the graph being captured on `st`; otherwise the
 // host drives the loop (used by warm-up only).
-int enqueue(edp_peeler *p, cudaStream_t st, bool graph) {
+int enqueue(edp_peeler *p, cudaStream_t st, bool graph, bool own = false) {
   Dev d = p->d;
+  d.use_side = own && p->side.stream ? 1 : 0;
   if (!graph) {
     d.use_handle = 0;
     EDP_TRY(run_prepare(p, d, st));
@@ -501,6 +507,9 @@ int edp_event_create(const double *vertices, int64_t nv, const int32_t *faces, i
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->body_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->round_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) d.aux_stream = p->round_stream;
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->side.stream, cudaStreamNonBlocking);
+  for (cudaEvent_t *ev : {&p->side.forked, &p->side.joined})
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
   if (e == cudaSuccess) e = allocate_event(p);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
@@ -598,7 +607,7 @@ int edp_capture(edp_peeler *p) {
     if (!ev) EDP_TRY(cudaEventCreate(&ev));
   EDP_TRY(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
   set_stage_marks(p->marks);
-  int rc = enqueue(p, p->stream, true);
+  int rc = enqueue(p, p->stream, true, true);
   set_stage_marks(nullptr);
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamEndCapture(p->stream, &g);
@@ -664,6 +673,9 @@ void edp_destroy(edp_peeler *p) {
   for (void *a : p->allocations) cudaFree(a);
   if (p->body_stream) cudaStreamDestroy(p->body_stream);
   if (p->round_stream) cudaStreamDestroy(p->round_stream);
+  if (p->side.stream) cudaStreamDestroy(p->side.stream);
+  for (cudaEvent_t ev : {p->side.forked, p->side.joined})
+    if (ev) cudaEventDestroy(ev);
   for (auto &e : p->stage_exec)
     if (e) cudaGraphExecDestroy(e);
   for (cudaEvent_t ev : p->marks)
