@@ -433,9 +433,32 @@ __device__ __noinline__ unsigned walk_batch(Tree t, int leaves, float4 lo, float
   return walk_next(w, t, leaves, lo, hi, cursor, budget, batch, first, resume) ? batch : 0u;
 }
 
+// Swap frontiers and decide whether another round runs (event_kernels.py:12-25).
+// Patches parked for the exact pass shared the next frontier's slots from the
+// top: together with the pushed ones they must have fit.
+__device__ inline void advance_round(const Dev &d) {
+  volatile int *status = d.status, *sc = d.sc;
+  const int next = status[kNextResidual], deferred = sc[kDeferred];
+  if (int64_t(next) + deferred > d.cap.frontier) set_error(d.status, kErrResidual);
+  d.metrics[kParkedPatches] += deferred;
+  sc[kDeferred] = 0;
+  sc[kDeferredNext] = 0;
+  status[kResidual] = next;
+  status[kNextResidual] = 0;
+  sc[kFrontierNext] = 0;
+  long long rounds = ++d.metrics[kRounds];
+  if (rounds >= d.cap.rounds && next > 0) set_error(d.status, kErrRounds);
+  status[kPeakResidual] = max(status[kPeakResidual], next);
+  *d.parity ^= 1;
+  int c = next > 0 && status[kError] == 0;
+  *d.condition = c;
+  if (d.use_handle) cudaGraphSetConditional(d.cond_handle, unsigned(c));
+}
+
 constexpr int kStack = 8;     // patches a group keeps for itself
 constexpr int kLocalCuts = 6; // cuts of one taken patch whose right parts stay local
 constexpr int kMostCuts = 8;  // cuts of one taken patch before its parts go to the next round
+constexpr int kFewCuts = 3;   // both, when there are fewer patches than groups
 
 // One frontier round (frontier.py:106-223), a patch per group of W lanes.  A
 // patch meets its source's listed segments whose boxes overlap its own, from
@@ -465,10 +488,11 @@ constexpr int kMostCuts = 8;  // cuts of one taken patch before its parts go to 
 // The time is instruction issue on patches of three to six vertices, and at
 // small sizes the chain of one group's steps: a warp per patch left 26 of 32
 // lanes idle, and a round per right-hand part made 14 rounds of the knot.
-// Rounds in all (a warp per patch, then this): knot-65536 3.04 -> 1.05 ms,
-// 720K primitives 11.5 -> 3.4 ms, 2,560-face icospheres 0.60 -> 0.40 ms.  The
+// Rounds in all (a warp per patch, then this): knot-65536 3.04 -> 0.97 ms,
+// 720K primitives 11.5 -> 3.2 ms, 2,560-face icospheres 0.60 -> 0.36 ms.  The
 // cut bounds trade a round's longest chain against the number of rounds:
-// unbounded chains took 1.2, 3.5 and 0.43 ms.  4 blocks of 128 registers per
+// unbounded chains took 1.2, 3.5 and 0.43 ms, and 8 cuts even for few patches
+// 1.04, 3.4 and 0.40.  4 blocks of 128 registers per
 // SM: 5 blocks spill (1.3 ms on the knot), 3 hide less latency (1.13).
 template <int F, int W>
 __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
@@ -494,6 +518,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
                       &d.status[kNextResidual], d.status, d.cap.frontier - parked};
   int visits = 0, tests = 0, splits = 0;  // each group's lane 0
   CutTally tally;
+  // With fewer patches than groups the round lasts as long as one group's chain.
+  const bool few = live <= int(gridDim.x) * kGroups / 2;
+  const int local_cuts = few ? kFewCuts : kLocalCuts, most_cuts = few ? kFewCuts : kMostCuts;
   // The group's patch.
   bool idle = true, drained = false, changed = false;
   int waiting = 0, cut_count = 0, budget = 0;
@@ -585,6 +612,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
           if (meets) {
             id = __ldg(&segs.ids[base + g.lane]);
             code = kDepthOpen;
+            ca = segs.a[id];
+            cb = segs.b[id];
+            cn = segs.near[id];
           }
         }
       } else if (look) {
@@ -599,14 +629,14 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
             const int2 e = d.cand[int64_t(start) + base + g.lane];
             id = e.x;
             code = e.y;
-            meets = overlaps(segs.lo[id], segs.hi[id], box.lo, box.hi);
+            // The segment with its box, not after it: one latency, not two.
+            const float4 lo = segs.lo[id], hi = segs.hi[id];
+            ca = segs.a[id];
+            cb = segs.b[id];
+            cn = segs.near[id];
+            meets = overlaps(lo, hi, box.lo, box.hi);
           }
         }
-      }
-      if (meets) {
-        ca = segs.a[id];
-        cb = segs.b[id];
-        cn = segs.near[id];
       }
       tests += __popc(g.ballot(meets));
       if (!kWide && __any_sync(kFull, meets)) {
@@ -683,7 +713,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
     }
     // The right part: to the stack, or to the next round.
     const int right_size = nr | (generation + 1) << kSizeBits;
-    if (!kWide && keep_right && waiting < kStack && cut_count < kLocalCuts) {
+    if (!kWide && keep_right && waiting < kStack && cut_count < local_cuts) {
       s_stack[slot][waiting][g.lane] = pr;
       if (g.lane == 0) s_waiting[slot][waiting] = make_int2(right_size, base + k + 1);
       ++waiting;
@@ -697,7 +727,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
       changed = true;
       batch = 0;
       cursor = base + k + 1;
-      push = !kWide && cut_count >= kMostCuts;
+      push = !kWide && cut_count >= most_cuts;
     }
     if (kWide && test && !park && n <= 8 && count != kUnlisted) {
       cursor = base + k + 1;  // past its candidate, a group of eight lanes can go on
@@ -726,27 +756,17 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
     tally.segment.flush(d, kPredSegment);
     tally.depth.flush(d, kPredDepth);
   }
-}
-
-// Swap frontiers and decide whether another round runs (event_kernels.py:12-25).
-// Patches parked for the exact pass shared the next frontier's slots from the
-// top: together with the pushed ones they must have fit.
-__global__ void k_advance(Dev d) {
-  int next = d.status[kNextResidual];
-  if (int64_t(next) + d.sc[kDeferred] > d.cap.frontier) set_error(d.status, kErrResidual);
-  d.metrics[kParkedPatches] += d.sc[kDeferred];
-  d.sc[kDeferred] = 0;
-  d.sc[kDeferredNext] = 0;
-  d.status[kResidual] = next;
-  d.status[kNextResidual] = 0;
-  d.sc[kFrontierNext] = 0;
-  long long rounds = ++d.metrics[kRounds];
-  if (rounds >= d.cap.rounds && next > 0) set_error(d.status, kErrRounds);
-  d.status[kPeakResidual] = max(d.status[kPeakResidual], next);
-  *d.parity ^= 1;
-  int c = next > 0 && d.status[kError] == 0;
-  *d.condition = c;
-  if (d.use_handle) cudaGraphSetConditional(d.cond_handle, unsigned(c));
+  if constexpr (kWide) {  // the second pass's last block ends the round
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      if (atomicAdd(&d.sc[kRoundBlocks], 1) == int(gridDim.x) - 1) {
+        __threadfence();
+        d.sc[kRoundBlocks] = 0;
+        advance_round(d);
+      }
+    }
+  }
 }
 
 }  // namespace
@@ -790,8 +810,6 @@ cudaError_t stage_step(const Dev &d, cudaStream_t st) {
     case 2: launch_round<2, 2>(d, g, second, st); break;
     default: launch_round<4, 3>(d, g, second, st); break;
   }
-  k_advance<<<1, 1, 0, st>>>(d);
-  note_launch();
   return cudaGetLastError();
 }
 

@@ -150,7 +150,8 @@ enum Scalar : int {
   kDeepGroups = 31,  // hit groups sorted a warp each (k_group_sort_deep)
   kCandidates = 32,  // entries of the sources' candidate lists
   kOrderLive = 33,   // buckets of the current work order
-  kScalarCount = 34  // k_reset clears them with its first threads
+  kRoundBlocks = 34, // blocks of this round's second pass that are done
+  kScalarCount = 35  // k_reset clears them with its first threads
 };
 
 // Predicate tallies: six classes by three deciding stages (edp_filtered.cuh).
