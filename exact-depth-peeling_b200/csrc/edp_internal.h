@@ -103,7 +103,7 @@ struct Caps {
 };
 
 constexpr int kRayCells = 16;  // most source-grid cells one source is listed in, at least
-constexpr int kSegCells = 4;   // most segment-grid cells one contour segment is listed in
+constexpr int kSegCells = 4;   // most segment-grid cells one segment is listed in, at least
 
 // Device scalars kept between kernels of one extraction.
 enum Scalar : int {
@@ -229,6 +229,7 @@ struct Dev {
   unsigned long long *owners;
   V2 *starts, *ends;
   int *partners, *edge_hash, *parents, *reps;
+  int2 *pairs;  // matched patch edges, smaller index first
   int edge_hash_mask;
   // samples and query groups
   V2 *samples;
@@ -275,8 +276,10 @@ struct Dev {
   float4 *ray_boxes, *ray_edges;  // ray_edges: three binary32 edge functions per source
   int ray_cells;                  // most cells one source is listed in
   // Contour segment grid for the connection test: distinct segments listed in
-  // the cells their box (grown by 1e-6) meets, at most kSegCells each.
+  // the cells their box (grown by 1e-6) meets, at most seg_cells each.
   int *seg_count, *seg_start, *seg_entries, *seg_big;
+  int seg_cells;
+  float4 *seg_boxes;  // per entry: its segment's lo.x, lo.y, hi.x, hi.y
   int *cell_count, *cell_start;
   V2 *grid_pts;
   int *heavy_polygons;  // polygons with many grid candidates, noded a warp each

@@ -90,32 +90,40 @@ __device__ inline uint64_t point_key(V2 x) {
 
 // A bounded open-addressing table pairs each patch edge with the reversed edge
 // of another patch that has the same owner (components.py:330-366).  The key
-// is symmetric in the endpoints so both directions probe the same chain.
+// is symmetric in the endpoints so both directions probe the same chain.  The
+// pairs are listed, by their smaller edge, for the connection test.
 __global__ void k_match_edges(Dev d) {
   const int total = patch_edges(d);
   for (int64_t i = tid(); i < total; i += stride()) {
     if (d.status[kError] != 0) return;
     V2 a = d.starts[i], b = d.ends[i];
-    if (a == b) continue;
-    const unsigned long long owner = d.owners[i];
-    uint64_t key = mix64(owner) ^ point_key(a) ^ point_key(b);
-    uint32_t slot = uint32_t(key) & uint32_t(d.edge_hash_mask);
-    bool placed = false;
-    for (int attempt = 0; attempt < 64; ++attempt) {
-      int other = atomicCAS(&d.edge_hash[slot], -1, int(i));
-      if (other < 0) {
-        placed = true;
-        break;
+    int partner = -1;
+    bool placed = a == b;
+    if (!placed) {
+      const unsigned long long owner = d.owners[i];
+      uint64_t key = mix64(owner) ^ point_key(a) ^ point_key(b);
+      uint32_t slot = uint32_t(key) & uint32_t(d.edge_hash_mask);
+      for (int attempt = 0; attempt < 64; ++attempt) {
+        int other = atomicCAS(&d.edge_hash[slot], -1, int(i));
+        if (other < 0) {
+          placed = true;
+          break;
+        }
+        if (d.owners[other] == owner && d.tasks[i].x != d.tasks[other].x && a == d.ends[other] &&
+            b == d.starts[other]) {
+          partner = other;
+          placed = true;
+          break;
+        }
+        slot = (slot + 1) & uint32_t(d.edge_hash_mask);
       }
-      if (d.owners[other] == owner && d.tasks[i].x != d.tasks[other].x && a == d.ends[other] &&
-          b == d.starts[other]) {
-        d.partners[i] = other;
-        d.partners[other] = int(i);
-        add_metric(d, kMatchedPatchEdges, 1);
-        placed = true;
-        break;
-      }
-      slot = (slot + 1) & uint32_t(d.edge_hash_mask);
+    }
+    // One reservation for the warp, not one per attempt that found a partner.
+    const long long at = reserve(&d.metrics[kMatchedPatchEdges], partner >= 0 ? 1 : 0);
+    if (partner >= 0) {
+      d.partners[i] = partner;
+      d.partners[partner] = int(i);
+      d.pairs[at] = make_int2(min(int(i), partner), max(int(i), partner));
     }
     if (!placed) add_metric(d, kEdgeHashMisses, 1);  // loses only the optimisation
   }
@@ -148,7 +156,7 @@ __device__ inline void uf_unite(int *parents, int a, int b) {
 }
 
 // Contour-segment grid (the same cells as the source grid): each distinct
-// segment whose box, grown by 1e-6, meets at most kSegCells cells is listed
+// segment whose box, grown by 1e-6, meets at most Dev::seg_cells cells is listed
 // in them; longer ones go to a list every query reads.
 __device__ inline int seg_grid_cell(double v, int g) {
   const double c = floor(v * double(g));
@@ -171,7 +179,7 @@ __global__ void k_seg_grid_count(Dev d) {
   for (int64_t c = tid(); c < total; c += stride()) {
     int cx0, cx1, cy0, cy1;
     if (!segment_cells(d, int(c), cx0, cx1, cy0, cy1)) continue;
-    if ((cx1 - cx0 + 1) * (cy1 - cy0 + 1) > kSegCells) {
+    if ((cx1 - cx0 + 1) * (cy1 - cy0 + 1) > d.seg_cells) {
       d.seg_big[reserve(&d.sc[kSegBig], 1)] = int(c);
       continue;
     }
@@ -186,11 +194,15 @@ __global__ void k_seg_grid_fill(Dev d) {
   for (int64_t c = tid(); c < total; c += stride()) {
     int cx0, cx1, cy0, cy1;
     if (!segment_cells(d, int(c), cx0, cx1, cy0, cy1)) continue;
-    if ((cx1 - cx0 + 1) * (cy1 - cy0 + 1) > kSegCells) continue;
+    if ((cx1 - cx0 + 1) * (cy1 - cy0 + 1) > d.seg_cells) continue;
+    const float4 lo = d.seg_lo[c], hi = d.seg_hi[c];
+    const float4 box = make_float4(lo.x, lo.y, hi.x, hi.y);
     for (int cy = cy0; cy <= cy1; ++cy)
       for (int cx = cx0; cx <= cx1; ++cx) {
         const int cell = cy * d.grid_size + cx;
-        d.seg_entries[d.seg_start[cell] + atomicSub(&d.seg_count[cell], 1) - 1] = int(c);
+        const int e = d.seg_start[cell] + atomicSub(&d.seg_count[cell], 1) - 1;
+        d.seg_entries[e] = int(c);
+        d.seg_boxes[e] = box;
       }
   }
 }
@@ -198,16 +210,23 @@ __global__ void k_seg_grid_fill(Dev d) {
 // Matched edges are connected when no nearer-or-equal contour passes through
 // the edge midpoint (components.py:393-450).  Candidate segments are those
 // whose box meets the query box: from the segment grid's cell of the midpoint
-// (every such segment is listed there or among the long ones), else from the
-// contour hierarchy.  Any blocking segment decides, so the order does not
-// matter; the visit counter counts segments met until the first blocker.
+// (every such segment is listed there, with its box, or among the long ones),
+// else from the contour hierarchy.  Any blocking segment decides, so the order
+// does not matter; the visit counter counts segments met until the first
+// blocker.
+//
+// Bound by the latency of the segments' loads.  One thread per matched pair;
+// a thread per patch edge, of which three in ten led a pair, with a square
+// root and a division per candidate, made the matching and this test 0.23 ms
+// longer on the 65,536-face knot (0.88 ms) and 0.46 on the 720K primitives.
 __global__ void k_connect(Dev d) {
-  const int total = patch_edges(d);
+  const int total = int(min((long long)d.metrics[kMatchedPatchEdges], (long long)d.cap.vertices));
   const int leaves = *d.seg_tree.size;
-  for (int64_t i = tid(); i < total; i += stride()) {
+  const bool grid = d.sc[kSegGridOn] != 0;
+  for (int64_t m = tid(); m < total; m += stride()) {
     if (d.status[kError] != 0) return;
-    int other = d.partners[i];
-    if (other <= i) continue;
+    const int2 pair = d.pairs[m];
+    const int i = pair.x, other = pair.y;
     int2 task = d.tasks[i];
     V2 a = d.starts[i], b = d.ends[i];
     if (length(b - a) <= 16.0 * kEps) continue;
@@ -218,14 +237,20 @@ __global__ void k_connect(Dev d) {
     float4 hi = make_float4(upper_f(x.x + 2.0e-7), upper_f(x.y + 2.0e-7), upper_f(z + pad), 0.f);
     int visits = 0;
     bool safe = true;
-    // Does segment c pass through x at or in front of the patch?
+    // Does segment c, whose box meets the query box in x and y, meet it and
+    // pass through x at or in front of the patch?
     auto blocks = [&](int c) {
+      const float front = d.seg_lo[c].z;  // loaded with the ends, in one latency
+      const V2 u = d.seg_a[c], v = d.seg_b[c], dv = v - u;
+      if (!(front <= hi.z)) return false;
       ++visits;
-      V2 u = d.seg_a[c], v = d.seg_b[c], dv = v - u;
-      double len = length(dv);
+      const double off = cross(u, v, x), square = dot(dv, dv);
+      // Off the line by more than the rounding of the test below: most.
+      if (off * off > kEps * kEps * square * (1.0 + 1.0e-9)) return false;
+      const double len = length(dv);
       if (len > 0.0) {
-        double t = dot(x - u, dv) / dot(dv, dv);
-        if (fabs(cross(u, v, x)) <= kEps * len && t >= -kEps / len && t <= 1.0 + kEps / len) {
+        const double t = dot(x - u, dv) / square;
+        if (fabs(off) <= kEps * len && t >= -kEps / len && t <= 1.0 + kEps / len) {
           V2 near = d.seg_near[c];
           double depth = near.x + t * (near.y - near.x);
           if (depth <= z + pad) return true;
@@ -233,13 +258,20 @@ __global__ void k_connect(Dev d) {
       }
       return false;
     };
-    if (d.sc[kSegGridOn]) {
+    if (grid) {
       const int g = d.grid_size;
       const int cell = seg_grid_cell(x.y, g) * g + seg_grid_cell(x.x, g);
       const int begin = d.seg_start[cell], end = d.seg_start[cell + 1], big = d.sc[kSegBig];
       for (int e = begin; e < end + big; ++e) {
-        const int c = e < end ? d.seg_entries[e] : d.seg_big[e - end];
-        if (!overlaps(d.seg_lo[c], d.seg_hi[c], lo, hi)) continue;
+        int c;
+        if (e < end) {
+          const float4 box = d.seg_boxes[e];
+          c = d.seg_entries[e];
+          if (!(box.x <= hi.x && box.y <= hi.y && box.z >= lo.x && box.w >= lo.y)) continue;
+        } else {
+          c = d.seg_big[e - end];
+          if (!overlaps(d.seg_lo[c], d.seg_hi[c], lo, hi)) continue;
+        }
         if (blocks(c)) {
           safe = false;
           break;

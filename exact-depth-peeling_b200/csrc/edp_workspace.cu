@@ -244,7 +244,10 @@ cudaError_t allocate_event(edp_peeler *p) {
     EDP_CHECK(alloc(p, &d.leaf_of, n > 0 ? n : 1));
     EDP_CHECK(alloc(p, &d.seg_count, cells));
     EDP_CHECK(alloc(p, &d.seg_start, cells + 1));
-    EDP_CHECK(alloc(p, &d.seg_entries, int64_t(kSegCells) * S));
+    d.seg_cells = int(std::min(cells, std::max<int64_t>(kSegCells, (int64_t(1) << 20) /
+                                                                       (S > 0 ? S : 1))));
+    EDP_CHECK(alloc(p, &d.seg_entries, int64_t(d.seg_cells) * S));
+    EDP_CHECK(alloc(p, &d.seg_boxes, int64_t(d.seg_cells) * S));
     EDP_CHECK(alloc(p, &d.seg_big, S));
   }
   EDP_CHECK(alloc(p, &d.group_counts, R));
@@ -259,6 +262,7 @@ cudaError_t allocate_event(edp_peeler *p) {
   EDP_CHECK(alloc(p, &d.starts, E));
   EDP_CHECK(alloc(p, &d.ends, E));
   EDP_CHECK(alloc(p, &d.partners, E));
+  EDP_CHECK(alloc(p, &d.pairs, E));
   if (d.merge_regions) {
     EDP_CHECK(alloc(p, &d.merge_choice, R));
     EDP_CHECK(alloc(p, &d.merged_v, R * kMaxVertices));
