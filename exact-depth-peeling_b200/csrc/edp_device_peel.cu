@@ -228,27 +228,63 @@ __device__ inline V2 *piece_at(V2 *base, int64_t slot) { return base + kMaxVerti
 struct PiecePool {
   V2 *v;
   int *n, *target, *cursor;  // cursor: null for the hidden pool
-  int *count, *status;
-  int cap, full;             // full: the error bit of a pool that is full
+  int *count;
+  int cap;
 };
 
-// Appends a piece (one vertex per lane) to a pool; false (and the pool's
-// error) when it is full.
-__device__ __noinline__ bool append_piece(PiecePool f, V2 p, int n, int target, int cursor) {
+// The queue of a clipping launch.  Pieces are appended while other warps take
+// them: `ready` holds the launch's epoch once a slot is written, and `pending`
+// counts the pieces queued or in a warp.  Pieces past the pool's end go to the
+// spill pool, which the next launch takes.
+struct PieceQueue {
+  PiecePool pool, spill;
+  int *ready, *pending, *status;
+  int epoch;
+};
+
+__device__ inline void write_piece(const PiecePool &f, int slot, V2 p, int n, int target,
+                                   int cursor) {
   const int lane = threadIdx.x & 31;
-  int slot = 0;
-  if (lane == 0) slot = atomicAdd(f.count, 1);
-  slot = __shfl_sync(kFull, slot, 0);
-  if (slot >= f.cap) {
-    if (lane == 0) set_error(f.status, f.full);
-    return false;
-  }
   if (lane < n) piece_at(f.v, slot)[lane] = p;
   if (lane == 0) {
     f.n[slot] = n;
     f.target[slot] = target;
     if (f.cursor) f.cursor[slot] = cursor;
   }
+}
+
+// Appends a piece (one vertex per lane) to the hidden pool; false when it is
+// full.
+__device__ __noinline__ bool hide_piece(PiecePool f, V2 p, int n, int target) {
+  int slot = 0;
+  if ((threadIdx.x & 31) == 0) slot = atomicAdd(f.count, 1);
+  slot = __shfl_sync(kFull, slot, 0);
+  if (slot >= f.cap) return false;
+  write_piece(f, slot, p, n, target, 0);
+  return true;
+}
+
+// Queues a piece; false (and the worker-pool error) when both pools are full.
+__device__ __noinline__ bool queue_piece(PieceQueue q, V2 p, int n, int target, int cursor) {
+  const int lane = threadIdx.x & 31;
+  int slot = 0;
+  if (lane == 0) slot = atomicAdd(q.pool.count, 1);
+  slot = __shfl_sync(kFull, slot, 0);
+  if (slot < q.pool.cap) {
+    if (lane == 0) atomicAdd(q.pending, 1);  // before this warp's own piece ends
+    write_piece(q.pool, slot, p, n, target, cursor);
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) *(volatile int *)&q.ready[slot] = q.epoch;
+    return true;
+  }
+  if (lane == 0) slot = atomicAdd(q.spill.count, 1);
+  slot = __shfl_sync(kFull, slot, 0);
+  if (slot >= q.spill.cap) {
+    if (lane == 0) set_error(q.status, kErrWorker);
+    return false;
+  }
+  write_piece(q.spill, slot, p, n, target, cursor);
   return true;
 }
 
@@ -339,7 +375,7 @@ enum CutResult : int { kKept = 0, kCut = 1, kFailed = 2 };
 // shared memory (more than kClipParts of them are split off a second time),
 // so a cut that hides nothing leaves no parts behind.
 template <int F>
-__device__ inline int cut_piece(const Dev &d, const PiecePool &queue, const PiecePool &hidden,
+__device__ inline int cut_piece(const Dev &d, const PieceQueue &queue, const PiecePool &hidden,
                                 V2 &p, V2 &q, int &n, const Occluder &c, const Plane &st,
                                 int source, int target, int cursor,
                                 bool tested, V2 *left, V2 *right, V2 *held, int *held_n,
@@ -377,7 +413,7 @@ __device__ inline int cut_piece(const Dev &d, const PiecePool &queue, const Piec
   V2 keep = nearer;
   int keep_n = 0;
   auto emit = [&](V2 x, int m) {
-    if (keep_n > 0 && !append_piece(queue, keep, keep_n, target, cursor)) return false;
+    if (keep_n > 0 && !queue_piece(queue, keep, keep_n, target, cursor)) return false;
     keep = x;
     keep_n = m;
     return true;
@@ -423,7 +459,7 @@ __device__ inline int cut_piece(const Dev &d, const PiecePool &queue, const Piec
       if (in_n == 0) return kKept;  // nothing covered after all
       if (lane == 0 && atomicAdd(&d.target_hidden[target], 1) >= d.pieces)
         set_error(d.status, kErrWorker);
-      append_piece(hidden, in, in_n, target, 0);
+      if (!hide_piece(hidden, in, in_n, target) && lane == 0) set_error(d.status, kErrResidual);
       if (nearer_n > 0) emit(nearer, nearer_n);
       if (parts <= kClipParts) {
         __syncwarp();
@@ -460,28 +496,57 @@ __global__ void k_clip_begin(Dev d) {
     const int queued = live <= d.work_cap ? live : 0;
     if (live > d.work_cap) set_error(d.status, kErrWorker);
     d.sc[kClipLive] = queued;
-    d.sc[kClipNext] = 0;
+    d.sc[kClipNext] = queued;
+    d.sc[kClipSpill] = 0;
+    d.sc[kClipPending] = queued;
     d.sc[kClipHidden] = 0;
     d.sc[kClipParity] = 0;
     d.sc[kFrontierNext] = 0;
+    ++*d.clip_epoch;
     const int c = queued > 0 && d.status[kError] == 0;
     d.sc[kClipCondition] = c;
     if (d.use_inner) cudaGraphSetConditional(d.inner_handle, unsigned(c));
   }
 }
 
-// One clipping round over the queued pieces, one piece per warp; warps take
-// pieces from a counter.  F is the predicate form.  A leaf batch of the walk
-// holds up to 32 candidates: each lane decides one against the piece as the
-// batch met it (may_hide), and the few left are cut one by one in leaf order
-// with a lane per piece vertex.  A part of a piece that may_hide rejected
-// needs no new test: it lies in the piece.
+// After a launch, by its last block: the spilled pieces become the next
+// launch's queue; stop when there are none.
+__device__ inline void advance_clipping(const Dev &d) {
+  volatile int *sc = d.sc;
+  const int spilled = min(sc[kClipSpill], d.work_cap);
+  sc[kClipLive] = spilled;
+  sc[kClipNext] = spilled;
+  sc[kClipSpill] = 0;
+  sc[kClipPending] = spilled;
+  sc[kFrontierNext] = 0;
+  sc[kClipParity] = sc[kClipParity] ^ 1;
+  ++*d.clip_epoch;
+  const int c = spilled > 0 && *(volatile int *)&d.status[kError] == 0;
+  sc[kClipCondition] = c;
+  if (d.use_inner) cudaGraphSetConditional(d.inner_handle, unsigned(c));
+}
+
+// Clips the queue, one piece per warp, until it is empty.  F is the predicate
+// form.  A leaf batch of the walk holds up to 32 candidates: each lane decides
+// one against the piece as the batch met it (may_hide), and the few left are
+// cut one by one in leaf order with a lane per piece vertex.  A part of a
+// piece that may_hide rejected needs no new test: it lies in the piece.
+//
+// Warps take slots of the queue by ticket and wait for the slot to be written,
+// or for the last piece to end.  A waited-for slot is written by a warp that
+// holds a piece and waits for nothing, so every wait ends; each is bounded all
+// the same (kWaitLimit polls, about a second, without a piece queued or ended),
+// and running out is an error.
 //
 // The bound is the serial chain of cuts of one piece, not throughput: a layer
-// has a few thousand pieces for 148 SMs.  With a thread per piece, local-memory
-// polygons and every cut ending its piece's round, the two nested icospheres
-// (2,560 faces, 12 layers) took 52.2 ms in this loop and a crossing scene of
-// 994 faces 12.3 ms.
+// has a few thousand pieces for 148 SMs.  A thread per piece, with its polygons
+// in local memory and every cut ending the piece's launch, took 59.8 ms per
+// extraction of two nested icospheres (2,560 faces, 12 layers) and 42.6 ms of
+// a crossing scene of 994 faces; a warp per piece with a launch per round of
+// cuts took 10.1 and 7.0, with the queue taken while it grows 5.4 and 3.2.
+// More polls, longer or shorter turns and half the blocks are all within 2%.
+constexpr int kWaitLimit = 1 << 20;
+
 template <int F>
 __global__ void __launch_bounds__(kBlock, 4) k_clip_round(Dev d) {
   __shared__ V2 s_piece[kClipWarps][kMaxVertices];
@@ -495,29 +560,64 @@ __global__ void __launch_bounds__(kBlock, 4) k_clip_round(Dev d) {
   const int rpar = *d.parity;
   const int layer = d.status[kPass];
   const int source_leaves = *d.source_tree.size, residual_leaves = *d.residual_tree.size;
-  const PiecePool queue{d.work_v[next], d.work_n[next], d.work_target[next],
-                        d.work_cursor[next], &d.sc[kClipNext], d.status, d.work_cap, kErrWorker};
+  const PieceQueue queue{
+      {d.work_v[wpar], d.work_n[wpar], d.work_target[wpar], d.work_cursor[wpar],
+       &d.sc[kClipNext], d.work_cap},
+      {d.work_v[next], d.work_n[next], d.work_target[next], d.work_cursor[next],
+       &d.sc[kClipSpill], d.work_cap},
+      d.work_ready[wpar], &d.sc[kClipPending], d.status, *d.clip_epoch};
   const PiecePool hidden{d.hid_v, d.hid_n, d.hid_target, nullptr, &d.sc[kClipHidden],
-                         d.status, d.hidden_cap, kErrResidual};
+                         d.hidden_cap};
   long long tested = 0;  // lane 0's tally
   Tally clip;
   for (;;) {
-    int i = 0, failed = 0;
+    int i = 0;
     if (lane == 0) {
       i = atomicAdd(&d.sc[kFrontierNext], 1);
-      failed = *(volatile int *)&d.status[kError];
+      // Slots below `live` were written before this launch.
+      int seen = 0;
+      for (int polls = 0;; ++polls) {
+        if (*(volatile int *)&d.status[kError] != 0 || i >= d.work_cap) {
+          i = -1;
+          break;
+        }
+        if (i < live || *(volatile int *)&queue.ready[i] == queue.epoch) break;
+        const int pending = *(volatile int *)queue.pending;
+        if (pending <= 0) {  // every piece has ended, so no slot is written any more
+          i = -1;
+          break;
+        }
+        const int progress = pending + *(volatile int *)queue.pool.count;
+        if (progress != seen) polls = 0;
+        seen = progress;
+        if (polls > kWaitLimit) {
+          set_error(d.status, kErrWorker);
+          i = -1;
+          break;
+        }
+        __nanosleep(200);
+      }
+      __threadfence();
     }
     i = __shfl_sync(kFull, i, 0);
-    if (i >= live || __shfl_sync(kFull, failed, 0) != 0) break;
-    int n = d.work_n[wpar][i];
-    if (n < 3) continue;
-    const int target = d.work_target[wpar][i];
-    const int start = d.work_cursor[wpar][i];
-    V2 p = lane < n ? piece_at(d.work_v[wpar], i)[lane] : v2(0.0, 0.0);
+    if (i < 0) break;
+    // Past L1, which may hold these lines from before they were written.
+    int n = __ldcg(&d.work_n[wpar][i]);
+    const int target = __ldcg(&d.work_target[wpar][i]);
+    const int start = __ldcg(&d.work_cursor[wpar][i]);
+    V2 p = v2(0.0, 0.0);
+    if (lane < n) {
+      const double2 x = __ldcg(reinterpret_cast<const double2 *>(piece_at(d.work_v[wpar], i)) + lane);
+      p = v2(x.x, x.y);
+    }
+    if (n < 3) {
+      if (lane == 0) atomicSub(queue.pending, 1);
+      continue;
+    }
     V2 q = Group<32>().shfl(p, lane + 1 < n ? lane + 1 : 0);
     const int source = d.res_src[rpar][target];
     const Plane st = d.scores[source];
-    // At least the steps from the root to a leaf group, so that every round
+    // At least the steps from the root to a leaf group, so that every turn
     // moves the walk on.
     int budget = max(d.clip_budget, 8);
     bool done = false;  // nothing of the piece is left in this warp
@@ -576,17 +676,22 @@ __global__ void __launch_bounds__(kBlock, 4) k_clip_round(Dev d) {
           box.lo.z = -1.0e30f;
         }
       }
-      if (!done && resume < leaves) {  // the budget ran out first
-        append_piece(queue, p, n, target, (tree << kCursorTree) | resume);
+      if (!done && resume < leaves) {  // the budget ran out first: to the queue's end
+        queue_piece(queue, p, n, target, (tree << kCursorTree) | resume);
         done = true;
       }
     }
-    if (done) continue;
+    if (done) {
+      __syncwarp();
+      if (lane == 0) atomicSub(queue.pending, 1);
+      continue;
+    }
     int slot = 0;
     if (lane == 0) {
       if (atomicAdd(&d.target_visible[target], 1) >= d.pieces) set_error(d.status, kErrWorker);
       slot = atomicAdd(&d.status[kPolygons], 1);
       if (slot >= d.cap.regions) set_error(d.status, kErrOutput);
+      atomicSub(queue.pending, 1);
     }
     slot = __shfl_sync(kFull, slot, 0);
     if (slot >= d.cap.regions) continue;
@@ -600,19 +705,15 @@ __global__ void __launch_bounds__(kBlock, 4) k_clip_round(Dev d) {
   }
   if (lane == 0 && layer < d.cap.layers && tested) count_add(&d.stats[3 * int64_t(layer) + 1], tested);
   if constexpr (F == 2) clip.flush(d, kPredClip);
-}
-
-// Between rounds: the appended pieces become the queue; stop when it is
-// empty.
-__global__ void k_clip_advance(Dev d) {
-  const int queued = d.sc[kClipNext];
-  d.sc[kClipLive] = min(queued, d.work_cap);
-  d.sc[kClipNext] = 0;
-  d.sc[kFrontierNext] = 0;
-  d.sc[kClipParity] ^= 1;
-  const int c = queued > 0 && d.status[kError] == 0;
-  d.sc[kClipCondition] = c;
-  if (d.use_inner) cudaGraphSetConditional(d.inner_handle, unsigned(c));
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&d.sc[kRoundBlocks], 1) == int(gridDim.x) - 1) {
+      __threadfence();
+      d.sc[kRoundBlocks] = 0;
+      advance_clipping(d);
+    }
+  }
 }
 
 // After the last round: a target with no visible piece is hidden whole (its
@@ -734,8 +835,6 @@ cudaError_t stage_device_layer(const Dev &layer_dev, SortScratch &s, TreeBuffers
                                             cudaStreamCaptureModeRelaxed));
     EDP_LAUNCH_FORM(d.predicates, k_clip_round, clip_blocks, kBlock, rounds, d);
     note_launch();
-    k_clip_advance<<<1, 1, 0, rounds>>>(d);
-    note_launch();
     cudaError_t launched = cudaGetLastError();
     cudaGraph_t captured = nullptr;
     cudaError_t end = cudaStreamEndCapture(rounds, &captured);
@@ -752,7 +851,6 @@ cudaError_t stage_device_layer(const Dev &layer_dev, SortScratch &s, TreeBuffers
       EDP_CHECK(cudaStreamSynchronize(st));
       if (!more) break;
       EDP_LAUNCH_FORM(d.predicates, k_clip_round, clip_blocks, kBlock, st, d);
-      k_clip_advance<<<1, 1, 0, st>>>(d);
       EDP_CHECK(cudaGetLastError());
     }
   }

@@ -151,7 +151,10 @@ enum Scalar : int {
   kCandidates = 32,  // entries of the sources' candidate lists
   kOrderLive = 33,   // buckets of the current work order
   kRoundBlocks = 34, // blocks of this round's second pass that are done
-  kScalarCount = 35  // k_reset clears them with its first threads
+  // Clipping: pieces spilled for the next launch, and pieces queued or in a warp.
+  kClipSpill = 35,
+  kClipPending = 36,
+  kScalarCount = 37  // k_reset clears them with its first threads
 };
 
 // Predicate tallies: six classes by three deciding stages (edp_filtered.cuh).
@@ -315,6 +318,7 @@ struct Dev {
   // target its visible and hidden piece counts.
   V2 *work_v[2];
   int *work_n[2], *work_target[2], *work_cursor[2];
+  int *work_ready[2], *clip_epoch;  // the epoch in which a slot was written
   int work_cap;
   V2 *hid_v;
   int *hid_n, *hid_target;

@@ -80,6 +80,27 @@ EDP_HD inline int expansion_sign(const double *e, int n) {
 // from every caller.
 EDP_HD inline EDP_COLD int orient2d_exact(double ax, double ay, double bx, double by, double cx,
                                    double cy) {
+  // Twice the working precision first.  The differences are exact as pairs
+  // (d, t) with |t| <= u |d|, and with S = |detleft| + |detright| the terms
+  // left out or rounded below are: two t t products (u^2 S), four d t products
+  // and their sums (at most 10 u^2 S), and the sums of the low parts, of at
+  // most 5 u S in all (at most 20 u^2 S).  A value above 64 u^2 S has its
+  // sign.  This decides nearly every call: a cut point off its line by its own
+  // rounding is 1e-17 away, far above 1e-31.
+  {
+    double adx, adxt, ady, adyt, bdx, bdxt, bdy, bdyt, l, lt, r, rt, d, dt;
+    two_sum(ax, -cx, adx, adxt);
+    two_sum(ay, -cy, ady, adyt);
+    two_sum(bx, -cx, bdx, bdxt);
+    two_sum(by, -cy, bdy, bdyt);
+    two_product(adx, bdy, l, lt);
+    two_product(ady, bdx, r, rt);
+    two_sum(l, -r, d, dt);
+    const double low = (dt + (lt - rt)) + ((adx * bdyt + adxt * bdy) - (ady * bdxt + adyt * bdx));
+    const double det = d + low;
+    const double bound = 64.0 * kU64 * kU64 * (fabs(l) + fabs(r));
+    if (det > bound || -det > bound) return sign_of(det);
+  }
   double e[12];
   int n = 0;
   const double xs[6] = {ax, -ay, bx, -by, cx, -cy};
@@ -191,6 +212,23 @@ EDP_HD inline int orient2d_lean(double ax, double ay, double bx, double by, doub
 // Exact stage of dot_sign: every product as a two-component expansion, all
 // grown into one (out of line, as orient2d_exact).
 EDP_HD inline EDP_COLD int dot_sign_exact(const double *p, const double *q, int n) {
+  // Twice the working precision first (the compensated dot product of Ogita,
+  // Rump and Oishi 2005): the sum s + c is within (n u)^2 S (1 + O(n u)) of the
+  // exact one before its last rounding, S the sum of magnitudes.
+  {
+    double s = 0.0, c = 0.0, magnitude = 0.0;
+    for (int k = 0; k < n; ++k) {
+      double h, l, t, r;
+      two_product(p[k], q[k], h, l);
+      two_sum(s, h, t, r);
+      s = t;
+      c += r + l;
+      magnitude += fabs(h);
+    }
+    const double sum = s + c;
+    const double bound = 4.0 * double(n + 2) * double(n + 2) * kU64 * kU64 * magnitude;
+    if (sum > bound || -sum > bound) return sign_of(sum);
+  }
   double e[16];
   int m = 0;
   for (int k = 0; k < n; ++k) {

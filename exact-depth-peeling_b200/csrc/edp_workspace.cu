@@ -318,7 +318,9 @@ cudaError_t allocate_device(edp_peeler *p) {
     EDP_CHECK(alloc(p, &d.work_n[k], d.work_cap));
     EDP_CHECK(alloc(p, &d.work_target[k], d.work_cap));
     EDP_CHECK(alloc(p, &d.work_cursor[k], d.work_cap));
+    EDP_CHECK(alloc(p, &d.work_ready[k], d.work_cap));
   }
+  EDP_CHECK(alloc(p, &d.clip_epoch, 1));
   EDP_CHECK(alloc(p, &d.hid_v, int64_t(d.hidden_cap) * kMaxVertices));
   EDP_CHECK(alloc(p, &d.hid_n, d.hidden_cap));
   EDP_CHECK(alloc(p, &d.hid_target, d.hidden_cap));

@@ -40,3 +40,27 @@ def test_many_edged_pieces_against_the_oracle(count, budget):
     p.set_tuning(clip_budget=budget)
     p.run()
     parity.check_against_oracle(p, parity.exact_scene_of(*arrays), range(count + 1))
+
+
+@pytest.mark.parametrize("count", [4, 6])
+def test_tight_pools(count):
+    """Pools that just hold the residual and the output: pieces queued past the
+    pool's end spill to the next launch of the layer."""
+    from dataclasses import replace
+
+    from peel_b200 import Capacities, DevicePeeler, scenes
+
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    arrays = rotated_stack(count)
+    device = scenes.to_device(arrays)
+    wide = Capacities(1024, 1024, 8192, 8192)
+    p = DevicePeeler(*device, capacities=wide)
+    p.run()
+    info = p.read_status()
+    tight = replace(wide, residual=info["peak_residual_patches"] + 8,
+                    polygons=info["polygons"] + 8)
+    p = DevicePeeler(*device, capacities=tight)
+    for _ in range(2):
+        p.run()
+        parity.check_against_oracle(p, parity.exact_scene_of(*arrays), range(count + 1))
