@@ -86,8 +86,8 @@ struct TreeBuffers {
   Tree tree() const { return Tree{nodes, ids, size}; }
 };
 
-cudaError_t tree_alloc(TreeBuffers &t, int64_t capacity);
-void tree_free(TreeBuffers &t);
+// Empties a new hierarchy, whose arrays are allocated and zero.
+cudaError_t tree_init(TreeBuffers &t);
 // Build over item boxes [0, *count).  `count_ptr` null means `static_count`.
 // `layered` adds lo.z (a layer number) above the Morton bits (kernels.py:89-90).
 cudaError_t tree_build(TreeBuffers &t, const float4 *lo, const float4 *hi, const int *count_ptr,

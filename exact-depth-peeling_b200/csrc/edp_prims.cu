@@ -503,31 +503,12 @@ cudaError_t tree_refit(TreeBuffers &t, const float4 *lo, const float4 *hi, cudaS
   return cudaGetLastError();
 }
 
-cudaError_t tree_alloc(TreeBuffers &t, int64_t capacity) {
-  t.capacity = capacity > 0 ? capacity : 1;
-  t.leaves_cap = pow2_at_least(t.capacity);
-  EDP_CHECK(cudaMalloc(&t.nodes, sizeof(float4) * 4 * t.leaves_cap));
-  EDP_CHECK(cudaMalloc(&t.ids, sizeof(int) * t.leaves_cap));
-  EDP_CHECK(cudaMalloc(&t.ids_tmp, sizeof(int) * t.leaves_cap));
-  EDP_CHECK(cudaMalloc(&t.keys, sizeof(uint64_t) * t.leaves_cap));
-  EDP_CHECK(cudaMalloc(&t.keys_tmp, sizeof(uint64_t) * t.leaves_cap));
-  EDP_CHECK(cudaMalloc(&t.flags, sizeof(int)));
-  EDP_CHECK(cudaMemset(t.flags, 0, sizeof(int)));
-  EDP_CHECK(cudaMalloc(&t.size, sizeof(int) * 2));
+cudaError_t tree_init(TreeBuffers &t) {
   t.count = t.size + 1;
-  EDP_CHECK(cudaMemset(t.size, 0, sizeof(int) * 2));
   const int64_t count = 2 * t.leaves_cap;
   k_tree_clear<<<grid_for(count, 256) < 4 * 148 ? grid_for(count, 256) : 4 * 148, 256>>>(t.nodes, count);
   note_launch();
-  EDP_CHECK(cudaGetLastError());
-  EDP_CHECK(cudaStreamSynchronize(0));
-  return cudaSuccess;
-}
-
-void tree_free(TreeBuffers &t) {
-  cudaFree(t.nodes); cudaFree(t.ids); cudaFree(t.ids_tmp);
-  cudaFree(t.keys); cudaFree(t.keys_tmp); cudaFree(t.flags); cudaFree(t.size);
-  t = TreeBuffers{};
+  return cudaGetLastError();
 }
 
 cudaError_t tree_build(TreeBuffers &t, const float4 *lo, const float4 *hi, const int *count_ptr,
