@@ -482,7 +482,8 @@ constexpr int kFewCuts = 3;   // both, when there are fewer patches than groups
 // past kStack waiting parts or kLocalCuts cuts, in the next round's frontier,
 // where other groups take it; both have the cursor just past the cutting
 // segment.  After kMostCuts cuts the left part goes to the next round too.  A
-// patch that has met every candidate is final and goes to the output pool.  Groups take patches from a shared counter.
+// patch that has met every candidate is final and goes to the output pool.  Groups take patches from a shared
+// counter.
 //
 // The groups of a warp run one loop in step: take a patch, find its next
 // candidate, test it, split.  Every step is run by the whole warp when any

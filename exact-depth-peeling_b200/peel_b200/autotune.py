@@ -3,12 +3,12 @@
 The knobs (``edp_tuning`` in include/edp.h) decide how work is spread over
 rounds, blocks and warps, never which regions or triangles come out:
 
-* ``step_budget``: subdivision walk steps a patch spends per round (the
-  queue granularity of the subdivision loop);
+* ``step_budget``: chunks of candidates a patch looks through per subdivision
+  round (the queue granularity of the subdivision loop);
 * ``subdivide_blocks``: subdivision blocks of four warps per SM (the tile
   width of the persistent subdivision grid);
 * ``heavy_noding_work``: candidate x edge tests above which a polygon is
-  noded by a warp instead of one thread;
+  noded by a warp instead of eight lanes;
 * ``clip_budget``: DevicePeeler hierarchy walk steps per piece and clipping round.
 
 ``tune`` runs a coordinate search: starting from the defaults, each knob in

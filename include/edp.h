@@ -183,11 +183,12 @@ int edp_predicate_counts(edp_peeler *p, int64_t *counts);
  * times replays under each and keeps the fastest.  No counterpart in the
  * reference, whose kernels fix them (frontier.py:149 and kernels.py:815-908
  * use 32 candidates per round and 4096 persistent workers).
- *   step_budget        subdivision: hierarchy walk steps a patch spends in a
+ *   step_budget        subdivision: chunks of candidates (8 of its source's
+ *                      list, or a walk step's 32) a patch looks through in a
  *                      round before it carries over (default 48)
  *   subdivide_blocks   subdivision: blocks of 4 warps per SM (default 8)
  *   heavy_noding_work  noding: candidate x edge tests above which a polygon
- *                      is noded by a warp instead of a thread (default 1024)
+ *                      is noded by a warp instead of 8 lanes (default 1024)
  *   clip_budget        DevicePeeler: hierarchy walk steps per piece and
  *                      clipping round (default 32, at least 8) */
 typedef struct edp_tuning {
