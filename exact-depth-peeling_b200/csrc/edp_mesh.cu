@@ -406,13 +406,13 @@ __global__ void __launch_bounds__(kBlock, 8) k_mesh_polygons(Dev d, int edge_cap
 // Bound by instruction issue (about 10 of a polygon's 55 cell points lie in
 // its box).  A thread per polygon ran 4.6 of 32 lanes, which waited for the
 // one with the most candidates, and wrote 48- and 72-byte pieces.  Noding and
-// emission together: knot-65536 1.36 -> 0.87 ms, its 9,702-face relative 0.55
-// -> 0.13, 720K primitives 4.0 -> 3.45, 640-face icospheres 0.12 -> 0.035.
+// emission together: knot-65536 1.36 -> 0.88 ms, its 9,702-face relative 0.55
+// -> 0.13, 720K primitives 4.0 -> 3.6, 640-face icospheres 0.12 -> 0.03.
 // Testing each near point by all edges at once instead of eight at a time took
 // 1.01 ms on the knot.  6 blocks of 80 registers per SM: 4 and 5 hide less
 // latency (0.97 and 0.91 ms), 7 spill (1.22).  The line to the warp kernel at
-// 1024 tests: 512 takes 0.94 and 2048 takes 1.01 ms on the knot, 3.8 and 3.3
-// on the 720K primitives.
+// 1024 tests takes 0.79 ms on the knot and 3.6 on the 720K primitives: 512
+// takes 0.86 and 3.9, 2048 takes 0.85 and 3.5.
 constexpr int kLanes = 8;
 constexpr int kMeshGroups = kBlock / kLanes;
 constexpr int kEdgeSplits = 8;
@@ -660,14 +660,22 @@ struct NodeEdge {
 constexpr int kHeavyWarps = kBlock / 32;
 
 // Noding and emission of the polygons k_mesh_groups queued as heavy, one
-// polygon per warp.  Lanes take the polygon's grid candidates 32 at a time
-// and test each against every edge with the thread kernel's expressions, so
-// the split points are the same.  Each split point is placed by its edge and
-// its rank along the edge, and the fan is written with a lane per edge.
+// polygon per warp.  The warp reads the points of 32 grid rows together, 32
+// at a time; those in the polygon's box wait until there are 32 to test, a
+// point per lane, against every edge with k_mesh_groups' expressions, so the
+// split points are the same.  Each split point is placed by its edge and its
+// rank along the edge, and the fan is written with a lane per piece of edge.
+//
+// Bound by instruction issue.  Row by row, with the fan a lane per edge, 11
+// of 32 lanes were busy: on the 65,536-face knot (14 thousand polygons) noding
+// and emission took 0.91 instead of 0.79 ms, on the 9,702-face knot 0.13
+// instead of 0.11, on the 50,000-face overlapping primitives 0.29 instead of
+// 0.27; on the 720K primitives it makes no difference.
 __global__ void __launch_bounds__(kBlock, 5) k_mesh_heavy(Dev d, int edge_capacity) {
   __shared__ NodeEdge s_edge[kHeavyWarps][kMaxVertices];
   __shared__ double s_t[kHeavyWarps][kPolygonSplits], s_sorted_t[kHeavyWarps][kPolygonSplits];
   __shared__ unsigned char s_e[kHeavyWarps][kPolygonSplits];
+  __shared__ V2 s_near[kHeavyWarps][64];
   __shared__ int s_count[kHeavyWarps], s_per_edge[kHeavyWarps][kMaxVertices];
   constexpr unsigned kFull = 0xffffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -675,6 +683,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_mesh_heavy(Dev d, int edge_capaci
   if (tid() == 0) d.metrics[kHeavyNodedPolygons] = heavy;
   const int g = d.point_grid;
   NodeEdge *edges = s_edge[warp];
+  V2 *waiting = s_near[warp];
   int *per_edge = s_per_edge[warp];
   double *split_t = s_t[warp], *sorted_t = s_sorted_t[warp];
   unsigned char *split_edge = s_e[warp];
@@ -686,18 +695,20 @@ __global__ void __launch_bounds__(kBlock, 5) k_mesh_heavy(Dev d, int edge_capaci
     const V2 *p = d.out_v + int64_t(kMaxVertices) * i;
     const int n = d.out_n[i];
     const int layer = d.out_layer[i], source = d.out_src[i];
-    // Box and centroid in the thread kernel's order (every lane alike).
-    double lx = 1.0e30, ly = 1.0e30, hx = -1.0e30, hy = -1.0e30;
-    V2 center = v2(0.0, 0.0);
-    for (int j = 0; j < n; ++j) {
-      const V2 x = p[j];
-      lx = fmin(lx, x.x); ly = fmin(ly, x.y);
-      hx = fmax(hx, x.x); hy = fmax(hy, x.y);
-      center = center + x / double(n);
+    // Box, and the centroid summed in vertex order.
+    const V2 own = lane < n ? p[lane] : v2(0.0, 0.0);
+    double lx = lane < n ? own.x : 1.0e30, ly = lane < n ? own.y : 1.0e30;
+    double hx = lane < n ? own.x : -1.0e30, hy = lane < n ? own.y : -1.0e30;
+    for (int off = 16; off > 0; off >>= 1) {
+      lx = smaller(lx, __shfl_xor_sync(kFull, lx, off));
+      ly = smaller(ly, __shfl_xor_sync(kFull, ly, off));
+      hx = larger(hx, __shfl_xor_sync(kFull, hx, off));
+      hy = larger(hy, __shfl_xor_sync(kFull, hy, off));
     }
+    waiting[lane] = own / double(n);
     if (lane < n) {
       NodeEdge e;
-      e.a = p[lane];
+      e.a = own;
       e.b = p[(lane + 1) % n];
       e.dir = e.b - e.a;
       e.length2 = dot(e.dir, e.dir);
@@ -708,32 +719,76 @@ __global__ void __launch_bounds__(kBlock, 5) k_mesh_heavy(Dev d, int edge_capaci
     }
     if (lane == 0) s_count[warp] = 0;
     __syncwarp();
+    V2 center = v2(0.0, 0.0);
+    for (int j = 0; j < n; ++j) center = center + waiting[j];
+    __syncwarp();
     const double qlx = lx - 1.0e-9, qly = ly - 1.0e-9, qhx = hx + 1.0e-9, qhy = hy + 1.0e-9;
     const int cx0 = grid_cell(qlx, g), cx1 = grid_cell(qhx, g);
     const int cy0 = grid_cell(qly, g), cy1 = grid_cell(qhy, g);
-    for (int cy = cy0; cy <= cy1; ++cy) {
-      const int64_t row = (int64_t(layer) * g + cy) * g;
-      const int begin = d.cell_start[row + cx0], end = d.cell_start[row + cx1 + 1];
-      for (int j = begin + lane; j < end; j += 32) {
-        const V2 x = d.grid_pts[j];
-        if (x.x < qlx || x.x > qhx || x.y < qly || x.y > qhy) continue;
-        for (int e = 0; e < n; ++e) {
-          const NodeEdge &E = edges[e];
-          if (x == E.a || x == E.b) continue;
-          if (!(E.length2 > 0.0)) continue;
-          const double off = cross(E.a, E.b, x);
-          if (off * off > E.slack) continue;
-          const double tt = dot(x - E.a, E.dir) / E.length2;
-          if (tt > kEps && tt < 1.0 - kEps && fabs(off) <= E.tol) {
-            const int at = atomicAdd(&s_count[warp], 1);
-            atomicAdd(&per_edge[e], 1);
-            if (at < kPolygonSplits) {
-              split_t[at] = tt;
-              split_edge[at] = (unsigned char)e;
+    int near_n = 0;
+    for (int row0 = cy0; row0 <= cy1; row0 += 32) {
+      const bool last_rows = row0 + 32 > cy1;
+      // 32 rows, one per lane, and the scan of their point counts.
+      int begin = 0, points = 0;
+      if (row0 + lane <= cy1) {
+        const int64_t row = (int64_t(layer) * g + row0 + lane) * g;
+        begin = d.cell_start[row + cx0];
+        points = d.cell_start[row + cx1 + 1] - begin;
+      }
+      int before = points;
+      for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(kFull, before, off);
+        if (lane >= off) before += y;
+      }
+      const int total = __shfl_sync(kFull, before, 31);
+      before -= points;
+      int t0 = 0;
+      do {
+        const int t = t0 + lane;
+        int r = 0;  // the row that holds the t-th point: the last one that begins at or before t
+        for (int off = 16; off > 0; off >>= 1)
+          if (__shfl_sync(kFull, before, r + off) <= t) r += off;
+        const int at = __shfl_sync(kFull, begin, r) + t - __shfl_sync(kFull, before, r);
+        V2 y = v2(0.0, 0.0);
+        bool near = t < total;
+        if (near) {
+          y = d.grid_pts[at];
+          near = !(y.x < qlx || y.x > qhx || y.y < qly || y.y > qhy);
+        }
+        const unsigned nears = __ballot_sync(kFull, near);
+        if (near) waiting[near_n + __popc(nears & ((1u << lane) - 1u))] = y;
+        near_n += __popc(nears);
+        t0 += 32;
+        __syncwarp();
+        // 32 waiting points at a time, a point per lane, against every edge.
+        const int need = last_rows && t0 >= total ? 1 : 32;
+        while (near_n >= need) {
+          const V2 x = waiting[lane];
+          if (lane < near_n) {
+            for (int e = 0; e < n; ++e) {
+              const NodeEdge &E = edges[e];
+              const double off = cross(E.a, E.b, x);
+              if (off * off > E.slack) continue;
+              if (x == E.a || x == E.b) continue;
+              if (!(E.length2 > 0.0)) continue;
+              const double tt = dot(x - E.a, E.dir) / E.length2;
+              if (tt > kEps && tt < 1.0 - kEps && fabs(off) <= E.tol) {
+                const int place = atomicAdd(&s_count[warp], 1);
+                atomicAdd(&per_edge[e], 1);
+                if (place < kPolygonSplits) {
+                  split_t[place] = tt;
+                  split_edge[place] = (unsigned char)e;
+                }
+              }
             }
           }
+          const V2 rest = waiting[32 + lane];
+          __syncwarp();
+          waiting[lane] = rest;
+          near_n = max(near_n - 32, 0);
+          __syncwarp();
         }
-      }
+      } while (t0 < total);
     }
     __syncwarp();
     // The thread kernel's overflow rule on the totals: more split points
@@ -769,35 +824,47 @@ __global__ void __launch_bounds__(kBlock, 5) k_mesh_heavy(Dev d, int edge_capaci
       sorted_t[rank] = t;
     }
     __syncwarp();
-    // The fan of emit_fan() with a lane per edge: lane e walks its edge's
-    // split points, and the lanes' triangle counts are scanned in edge order,
-    // so the triangles and their order within the polygon are emit_fan()'s.
-    V2 a = v2(0.0, 0.0), dir = a;
-    int emitted = 0;
+    // The fan of emit_fan(): a lane per edge keeps the split points that are
+    // more than kEps past the one before, then a lane per piece of edge emits
+    // its triangle, in the same order.
+    int kept = 0;
+    bool ends = false;
     if (lane < n) {
-      a = edges[lane].a;
-      dir = edges[lane].dir;
       double previous = 0.0;
-      V2 cursor = a;
-      for (int k = first;;) {
-        const bool last = k == first + mine;
-        const double following = last ? 1.0 : sorted_t[k++];
-        if (following > previous + kEps) {
-          const V2 next = a + following * dir;
-          if (cross(center, cursor, next) > kEps * kEps) ++emitted;
-          cursor = next;
-          previous = following;
+      for (int k = 0; k < mine; ++k) {
+        const double t = sorted_t[first + k];
+        if (t > previous + kEps) {
+          sorted_t[first + kept++] = t;
+          previous = t;
         }
-        if (last) break;
       }
+      ends = 1.0 > previous + kEps;
     }
-    int offset = emitted;
+    const int pieces = kept + int(ends);
+    int before = pieces;
     for (int off = 1; off < 32; off <<= 1) {
-      const int y = __shfl_up_sync(kFull, offset, off);
-      if (lane >= off) offset += y;
+      const int y = __shfl_up_sync(kFull, before, off);
+      if (lane >= off) before += y;
     }
-    const int total = __shfl_sync(kFull, offset, 31);
-    offset -= emitted;
+    const int all = __shfl_sync(kFull, before, 31);
+    before -= pieces;
+    __syncwarp();
+    // Piece s runs from `from` to `to`; `fan` says whether it has a triangle.
+    V2 from = center, to = center;
+    auto piece = [&](int s) {
+      int e = 0;  // its edge: the last one that begins at or before s
+      for (int off = 16; off > 0; off >>= 1)
+        if (__shfl_sync(kFull, before, e + off) <= s) e += off;
+      const int j = s - __shfl_sync(kFull, before, e), points = __shfl_sync(kFull, kept, e);
+      const double *t = sorted_t + __shfl_sync(kFull, first, e);
+      if (s >= all) return false;
+      const V2 start = edges[e].a, dir = edges[e].dir;
+      from = j == 0 ? start : start + t[j - 1] * dir;
+      to = start + (j == points ? 1.0 : t[j]) * dir;
+      return cross(center, from, to) > kEps * kEps;
+    };
+    int total = 0;
+    for (int s0 = 0; s0 < all; s0 += 32) total += __popc(__ballot_sync(kFull, piece(s0 + lane)));
     int base = 0;
     if (lane == 0 && total) base = atomicAdd(&d.status[kTriangles], total);
     base = __shfl_sync(kFull, base, 0);
@@ -806,43 +873,31 @@ __global__ void __launch_bounds__(kBlock, 5) k_mesh_heavy(Dev d, int edge_capaci
       __syncwarp();
       continue;
     }
-    if (lane < n) {
-      const Plane sc = d.scores[source];
-      double w_center[3];
-      lift(d, center, sc, w_center);
-      int slot = base + offset;
-      double previous = 0.0;
-      V2 cursor = a;
-      double w_cursor[3];
-      lift(d, cursor, sc, w_cursor);
-      for (int k = first;;) {
-        const bool last = k == first + mine;
-        const double following = last ? 1.0 : sorted_t[k++];
-        if (following > previous + kEps) {
-          const V2 next = a + following * dir;
-          double w_next[3];
-          lift(d, next, sc, w_next);
-          if (cross(center, cursor, next) > kEps * kEps) {
-            V2 *uv = d.tri_uv + 3 * int64_t(slot);
-            double *w = d.tri_world + 9 * int64_t(slot);
-            uv[0] = center;
-            uv[1] = cursor;
-            uv[2] = next;
-            for (int c = 0; c < 3; ++c) {
-              w[c] = w_center[c];
-              w[3 + c] = w_cursor[c];
-              w[6 + c] = w_next[c];
-            }
-            d.tri_src[slot] = source;
-            d.tri_layer[slot] = layer;
-            ++slot;
-          }
-          cursor = next;
-          for (int c = 0; c < 3; ++c) w_cursor[c] = w_next[c];
-          previous = following;
+    const Plane sc = d.scores[source];
+    double w_center[3];
+    lift(d, center, sc, w_center);
+    for (int s0 = 0; s0 < all; s0 += 32) {
+      const bool fan = piece(s0 + lane);
+      const unsigned fans = __ballot_sync(kFull, fan);
+      if (fan) {
+        const int64_t at = base + __popc(fans & ((1u << lane) - 1u));
+        double w_from[3], w_to[3];
+        lift(d, from, sc, w_from);
+        lift(d, to, sc, w_to);
+        V2 *uv = d.tri_uv + 3 * at;
+        double *w = d.tri_world + 9 * at;
+        uv[0] = center;
+        uv[1] = from;
+        uv[2] = to;
+        for (int c = 0; c < 3; ++c) {
+          w[c] = w_center[c];
+          w[3 + c] = w_from[c];
+          w[6 + c] = w_to[c];
         }
-        if (last) break;
+        d.tri_src[at] = source;
+        d.tri_layer[at] = layer;
       }
+      base += __popc(fans);
     }
     __syncwarp();
   }

@@ -49,3 +49,22 @@ def test_split_points_per_lane(m):
     parity.check_against_oracle(p, parity.exact_scene_of(*arrays), range(len(arrays[1])))
     sources = p.triangle_sources[: info["triangles"]].cpu().numpy()
     assert (sources == len(arrays[1]) - 1).sum() == 3 * m
+
+
+@pytest.mark.parametrize("m", [2, 10, 11, 32])
+def test_warp_kernel_fan(m):
+    """Every polygon noded by a warp, whose lanes take 32 points and 32 pieces
+    of edge at a time: 3 m pieces, of 3 (m - 1) points."""
+    from peel_b200 import EventPeeler, scenes
+
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    arrays = noded_triangle(m)
+    p = EventPeeler(*scenes.to_device(arrays))
+    p.set_tuning(heavy_noding_work=1)
+    p.run()
+    info = p.read_status()
+    assert info["heavy_noded_polygons"] > 0
+    parity.check_against_oracle(p, parity.exact_scene_of(*arrays), range(len(arrays[1])))
+    sources = p.triangle_sources[: info["triangles"]].cpu().numpy()
+    assert (sources == len(arrays[1]) - 1).sum() == 3 * m
