@@ -147,7 +147,7 @@ def hbm_peak():
         return FALLBACK_HBM_GBS, "fallback"
 
 
-def ncu_traffic(config, kernel="k_mesh_polygons"):
+def ncu_traffic(config, kernel="k_mesh_groups"):
     """DRAM bytes (read + write) of one noding stage on this workload (the
     launch of `kernel` plus that of k_mesh_heavy after it), as recorded from an
     ncu capture in profiles/<kernel>_<config>.md, or None."""
@@ -550,11 +550,11 @@ def measure_config(config, args, rank, world, local_rank, steps, e2e_steps, cpu_
     emit_ms = float(stage_ms["mesh_emit"])
     roofline = {
         "bound": "hbm",
-        "kernel": "k_mesh_polygons + k_mesh_heavy (noding, fan emission, world lift)",
+        "kernel": "k_mesh_groups + k_mesh_heavy (noding, fan emission, world lift)",
         "achieved": emit_bytes / (emit_ms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
         "frac": emit_bytes / (emit_ms * 1e-3) / 1e9 / peak,
         "traffic": ncu_traffic(config),
-        "traffic_source": f"ncu capture recorded in profiles/k_mesh_polygons_{config}.md",
+        "traffic_source": f"ncu capture recorded in profiles/k_mesh_groups_{config}.md",
         "peak_source": f"{peak_kind} copy bandwidth", "algorithmic_bytes": emit_bytes,
         "launch_ms": emit_ms,
         "pipeline": {"bytes_per_mesh": mesh_bytes,
