@@ -374,6 +374,24 @@ __device__ inline double atomic_max_double(double *addr, double v) {
 
 __device__ inline void set_error(int *status, int bit) { atomicOr(&status[kError], bit); }
 
+// Claims `count` consecutive entries of a pool of `capacity`, and returns the
+// first one, or -1 when they do not fit.  The counter only grows: what is
+// granted is never granted again, whatever claims are refused beside it.
+// (Giving a refused claim back would lower the counter under the claims
+// granted in the meantime.)  A pool that is full is left alone, so the counter
+// passes the capacity by at most one claim per caller.
+__host__ __device__ inline int64_t claim_entries(unsigned long long *counter, int64_t count,
+                                                 int64_t capacity) {
+  if (int64_t(*static_cast<volatile unsigned long long *>(counter)) + count > capacity) return -1;
+#ifdef __CUDA_ARCH__
+  const int64_t at = int64_t(atomicAdd(counter, (unsigned long long)count));
+#else
+  const int64_t at = int64_t(__atomic_fetch_add(counter, (unsigned long long)count,
+                                                __ATOMIC_RELAXED));
+#endif
+  return at + count <= capacity ? at : -1;
+}
+
 // Reserve `count` consecutive slots of an append counter for this thread,
 // with a single atomic per group of converged threads (the group's scan gives
 // each thread its offset).  Avoids serialising millions of appends on one

@@ -223,11 +223,12 @@ __global__ void __launch_bounds__(kBlock, 8) k_candidates(Dev d) {
       if (pass == 1) break;
       total = at;
       if (total == 0) break;
-      if (lane == 0) start = atomicAdd(&d.sc[kCandidates], total);
+      if (lane == 0)
+        start = int(claim_entries(reinterpret_cast<unsigned long long *>(&d.sc[kCandidates]),
+                                  total, d.cand_cap));
       start = __shfl_sync(kFull, start, 0);
-      if (start < 0 || int64_t(start) + total > d.cand_cap) {
+      if (start < 0) {
         total = kUnlisted;
-        if (lane == 0) atomicAdd(&d.sc[kCandidates], -at);
         break;
       }
       if (total <= kListBuffer) {

@@ -148,14 +148,15 @@ enum Scalar : int {
   kSortDeferred = 29,
   kAssignDeferred = 30,
   kDeepGroups = 31,  // hit groups sorted a warp each (k_group_sort_deep)
-  kCandidates = 32,  // entries of the sources' candidate lists
-  kOrderLive = 33,   // buckets of the current work order
-  kRoundBlocks = 34, // blocks of this round's second pass that are done
+  kCandidates = 32,  // entries claimed for the sources' candidate lists (64 bits: two slots)
+  kOrderLive = 34,   // buckets of the current work order
+  kRoundBlocks = 35, // blocks of this round's second pass that are done
   // Clipping: pieces spilled for the next launch, and pieces queued or in a warp.
-  kClipSpill = 35,
-  kClipPending = 36,
-  kScalarCount = 37  // k_reset clears them with its first threads
+  kClipSpill = 36,
+  kClipPending = 37,
+  kScalarCount = 38  // k_reset clears them with its first threads
 };
+static_assert(kCandidates % 2 == 0, "a 64-bit counter");
 
 // Predicate tallies: six classes by three deciding stages (edp_filtered.cuh).
 constexpr int kPredCounters = 18;

@@ -91,3 +91,78 @@ def test_long_lists_and_sources_without_one(side, sheets, form):
         assert abs(areas[(k + 1, s)] - covered) <= 1e-9
         assert abs(whole - areas[(0, n - sheets)] - areas[(1, n - sheets)]) <= 1e-9
         assert {key for key in areas if key[1] == s} == {(k, s), (k + 1, s)}
+
+
+def clipped_area(subject, triangle):
+    """Area of a convex polygon inside a counter-clockwise triangle."""
+    for j in range(3):
+        a, b = triangle[j], triangle[(j + 1) % 3]
+        side = (b[0] - a[0]) * (subject[:, 1] - a[1]) - (b[1] - a[1]) * (subject[:, 0] - a[0])
+        out = []
+        for k in range(len(subject)):
+            m = (k + 1) % len(subject)
+            if side[k] >= 0.0:
+                out.append(subject[k])
+            if side[k] * side[m] < 0.0:
+                t = side[k] / (side[k] - side[m])
+                out.append(subject[k] + t * (subject[m] - subject[k]))
+        if len(out) < 3:
+            return 0.0
+        subject = np.array(out)
+    x, y = (subject - subject[0]).T
+    return 0.5 * float(np.sum(x * np.roll(y, -1) - np.roll(x, -1) * y))
+
+
+@pytest.mark.parametrize("form", ["filtered64", "binary64"])
+def test_long_and_short_lists_past_the_pool(form):
+    """Lists of very different lengths that together exceed the pool: no two
+    sources share entries, so every region is the one the faces' order gives.
+    Disjoint tiles in front of disjoint cards of a few tiles each, in front of
+    sheets that fill the window."""
+    from peel_b200 import EventCapacities, EventPeeler, scenes
+
+    side, sheets, cards = 20, 24, 18
+    v, f, camera, settings = tiles_over_sheets(side, sheets)
+    rng = np.random.default_rng(2)
+    i, j = np.meshgrid(np.arange(cards), np.arange(cards), indexing="ij")
+    corner = np.array([[0.02, 0.05], [0.93, 0.11], [0.17, 0.95]])
+    xy = -0.5 + (np.stack([i, j], -1)[:, :, None, :] + corner
+                 + rng.uniform(-0.02, 0.02, size=(cards, cards, 3, 2))) / cards
+    xy = xy.reshape(-1, 3, 2)
+    front = np.concatenate([xy, np.full((len(xy), 3, 1), 1.5)], -1).reshape(-1, 3)
+    v = np.concatenate([v, front])
+    f = np.arange(len(v), dtype=np.int32).reshape(-1, 3)
+    tiles = v.reshape(-1, 3, 3)[: side * side, :, :2] * 0.5
+    short = xy * 0.5
+    area = {}
+
+    def doubled(t):
+        return ((t[:, 1, 0] - t[:, 0, 0]) * (t[:, 2, 1] - t[:, 0, 1])
+                - (t[:, 1, 1] - t[:, 0, 1]) * (t[:, 2, 0] - t[:, 0, 0]))
+
+    tile_areas, card_areas = 0.5 * doubled(tiles), 0.5 * doubled(short)
+    for s, a in enumerate(tile_areas):
+        area[(0, s)] = a
+    covered = 0.0
+    for c, (t, a) in enumerate(zip(short, card_areas)):
+        near = tiles[np.abs(tiles.mean(1) - t.mean(0)).max(1) < 1.5 / side]
+        under = sum(clipped_area(x, t) for x in near)
+        area[(0, side * side + sheets + c)] = a - under
+        area[(1, side * side + sheets + c)] = under
+        covered += under
+    single = float(tile_areas.sum() + card_areas.sum()) - 2.0 * covered
+    for k in range(sheets):
+        s = side * side + k
+        area[(k + 2, s)] = covered
+        area[(k + 1, s)] = single
+        area[(k, s)] = 1.0 - covered - single
+    n = len(f)
+    capacities = EventCapacities(400 * n, 800 * n, 8000 * n, 4000 * n, 4000 * n, layers=64)
+    p = EventPeeler(*scenes.to_device((v, f, camera, settings)), predicates=form,
+                    capacities=capacities)
+    for _ in range(4):
+        p.run()
+        assert p.read_status()["layers"] == sheets + 2
+        parity.assert_areas({key: a for key, a in parity.gpu_areas(parity.polygons(p),
+                                                                   range(n)).items() if a},
+                            {key: a for key, a in area.items() if a})
