@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_candidates(Dev d) {
         __syncwarp();
         queue[lane] = rest;
         queued = max(0, queued - 32);
+        __syncwarp();  // the next batch is written over the places past the rest
       };
       while (walk_next(w, d.seg_tree, leaves, lo, hi, 0, budget, batch, first, resume)) {
         if ((batch >> lane) & 1u)
