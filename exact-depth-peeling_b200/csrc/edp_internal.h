@@ -110,7 +110,7 @@ enum Scalar : int {
   kLivePolygons = 0,   // min(status[2], regions)
   kPatchEdges = 1,     // patch edges of all live polygons
   kLiveHits = 2,       // min(metrics[5], hits)
-  kLiveVertices = 3,   // min(status[6], vertices)
+  kLiveVertices = 3,   // boundary vertices: past the capacity only beside its error
   kSourceCount = 4,    // n (constant)
   kSegmentCount = 5,   // distinct contour segments (the hierarchy's items)
   kFrontierLive = 6,   // min(status[0], frontier)

@@ -30,7 +30,8 @@ __device__ inline int grid_cell(double v, int g) {
 // hierarchy does.
 __global__ void k_scatter(Dev d) {
   const int live = d.sc[kLivePolygons];
-  const int total = d.sc[kLiveVertices];  // or the capacity, once clamped below
+  // No block of this launch writes the count, so all of them take it alike.
+  const int total = d.sc[kLiveVertices];
   const bool fits = int64_t(total) <= d.cap.vertices;
   fill_words(d.point_table, ceil_div(int64_t(d.point_mask) + 1, 4), 0xffffffffu, tid(), stride());
   if (tid() == 0) {
@@ -39,10 +40,7 @@ __global__ void k_scatter(Dev d) {
     d.sc[kGridOn] = on ? 1 : 0;
     d.sc[kGridCells] = on ? int(int64_t(layers) * d.point_grid * d.point_grid) : 0;
     d.status[kBoundaryVertices] = total;
-    if (!fits) {
-      set_error(d.status, kErrVertices);
-      d.sc[kLiveVertices] = int(d.cap.vertices);
-    }
+    if (!fits) set_error(d.status, kErrVertices);
   }
   if (!fits) return;
   for (int64_t k = tid(); k < live; k += stride()) {
@@ -51,7 +49,7 @@ __global__ void k_scatter(Dev d) {
     const V2 *p = d.out_v + int64_t(kMaxVertices) * i;
     const int layer = d.out_layer[i];
     const int64_t base = d.offsets[k];
-    const int n = d.out_n[i];
+    const int n = int(min(int64_t(d.out_n[i]), d.cap.vertices - base));
     for (int j = 0; j < n; ++j) {
       d.bverts[base + j] = p[j];
       d.blayers[base + j] = layer;
