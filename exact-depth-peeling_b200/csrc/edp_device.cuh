@@ -33,7 +33,8 @@ enum StatusSlot : int {
 enum ErrorBit : int {
   kErrPolygon = 1, kErrWorker = 2, kErrResidual = 4, kErrOutput = 8, kErrVertices = 16,
   kErrTriangles = 32, kErrLayers = 64, kErrEdgeNoding = 128, kErrInput = 256,
-  kErrHits = 1024, kErrRounds = 2048
+  kErrHits = 1024, kErrRounds = 2048,
+  kErrWait = 4096  // a bounded wait between blocks or warps ran out
 };
 // EventPeeler counters (warp_peel/events.py:816-844).
 enum Metric : int {

@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_clip_round(Dev d) {
         if (progress != seen) polls = 0;
         seen = progress;
         if (polls > kWaitLimit) {
-          set_error(d.status, kErrWorker);
+          set_error(d.status, kErrWait);
           i = -1;
           break;
         }

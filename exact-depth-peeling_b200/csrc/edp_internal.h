@@ -53,7 +53,9 @@ struct LookBack {
   unsigned long long *words;
   int *control;
   int *error;  // where a wait that runs out sets its error bit
+  int polls;   // of a word before a wait runs out
 };
+constexpr int kPollLimit = 1 << 22;
 
 constexpr int kSortPasses = 8;
 

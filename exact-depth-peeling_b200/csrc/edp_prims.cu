@@ -54,20 +54,20 @@ __device__ inline int block_exclusive(int v, int *smem, int &total) {
 // subdivision loop became 97.  Replays: icospheres-640 0.81 -> 0.72 ms,
 // knot-9702 1.14 -> 1.03, a batch of 16 small scenes 3.44 -> 3.03.
 enum Published : unsigned { kNothing = 0, kSum = 1, kPrefix = 2 };
-constexpr int kPollLimit = 1 << 22;
 
 __device__ inline unsigned long long publish_word(unsigned epoch, unsigned state, int value) {
   return (unsigned long long)(epoch << 2 | state) << 32 | unsigned(value);
 }
 
-// The word at `p` once it is of this epoch.
+// The word at `p` once it is of this epoch.  A wait that runs out sets the
+// error and goes on as if nothing came before: every index stays in range.
 __device__ inline unsigned long long await_word(const unsigned long long *p, unsigned epoch,
-                                                int *error) {
+                                                const LookBack &s) {
   const volatile unsigned long long *v = p;
   unsigned long long w = *v;
   for (int polls = 0; unsigned(w >> 34) != epoch || (unsigned(w >> 32) & 3u) == kNothing; w = *v) {
-    if (++polls > kPollLimit) {
-      if (error) atomicOr(error, int(kErrOutput));
+    if (++polls > s.polls) {
+      atomicOr(s.error, int(kErrWait));
       return publish_word(epoch, kPrefix, 0);
     }
   }
@@ -141,7 +141,7 @@ k_scan(int *in, int *out, const int *count, LookBack s, int *total_out, int clea
       if (lane == 0) *(volatile unsigned long long *)&s.words[tile] = publish_word(epoch, kSum, total);
       for (int look = tile - 1;; look -= 32) {
         const int at = look - lane;
-        const unsigned long long w = at >= 0 ? await_word(s.words + at, epoch, s.error)
+        const unsigned long long w = at >= 0 ? await_word(s.words + at, epoch, s)
                                              : publish_word(epoch, kPrefix, 0);
         const unsigned full = __ballot_sync(0xffffffffu, (unsigned(w >> 32) & 3u) == kPrefix);
         const int last = full ? __ffs(int(full)) - 1 : 31;
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(kSortBlock) k_radix_pass(
         for (int c = 0; c < kWindow; ++c) {
           if (done) continue;
           if (unsigned(w[c] >> 34) != epoch || (unsigned(w[c] >> 32) & 3u) == kNothing)
-            w[c] = await_word(words + 256 * int64_t(look - c), epoch, s.error);
+            w[c] = await_word(words + 256 * int64_t(look - c), epoch, s);
           before += int(unsigned(w[c]));
           done = (unsigned(w[c] >> 32) & 3u) == kPrefix;
         }
@@ -287,8 +287,10 @@ __global__ void __launch_bounds__(kSortBlock) k_radix_pass(
     if (d[r] < 256) {
       int pos = wcount[warp][d[r]] + __popc(peers & lt);
       int64_t i = run + r * 32 + lane;
-      keys_out[pos] = k[r];
-      vals_out[pos] = vals[i];
+      if (pos < n) {  // always, unless a wait ran out and left older keys in an earlier pass
+        keys_out[pos] = k[r];
+        vals_out[pos] = vals[i];
+      }
     }
     __syncwarp();
     if (d[r] < 256 && lane == __ffs(peers) - 1) wcount[warp][d[r]] += __popc(peers);

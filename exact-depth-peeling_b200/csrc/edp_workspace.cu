@@ -99,7 +99,10 @@ cudaError_t commit(edp_peeler *p) {
   p->requests.clear();
   for (TreeBuffers *t : {&p->source_tree, &p->seg_tree, &p->point_tree, &p->residual_tree})
     if (t->nodes) EDP_CHECK(tree_init(*t));
-  for (SortScratch *s : {&p->scratch, &p->side.scratch}) s->look_back.error = p->d.status + kError;
+  for (SortScratch *s : {&p->scratch, &p->side.scratch}) {
+    s->look_back.error = p->d.status + kError;
+    s->look_back.polls = kPollLimit;
+  }
   Dev &d = p->d;
   d.source_tree = p->source_tree.tree();
   d.point_tree = p->point_tree.tree();

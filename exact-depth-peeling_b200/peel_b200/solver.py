@@ -24,6 +24,7 @@ _ERROR_LABELS = {
     64: "layer limit",
     128: "edge noding capacity",
     256: "invalid input",
+    4096: "device wait ran out",
 }
 
 

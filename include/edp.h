@@ -57,7 +57,10 @@ enum {
   EDP_ERR_BIT_EDGE_NODING = 128,
   EDP_ERR_BIT_INPUT = 256,
   EDP_ERR_BIT_HITS = 1024,
-  EDP_ERR_BIT_ROUNDS = 2048
+  EDP_ERR_BIT_ROUNDS = 2048,
+  /* A bounded wait of one block or warp for another ran out: a fault of the
+   * library or the device, which no capacity mends. */
+  EDP_ERR_BIT_WAIT = 4096
 };
 
 /* warp_peel/events.py:19-33 (EventCapacities). */
