@@ -51,6 +51,7 @@ inline unsigned grid_for(int64_t n, int block) {
 // one after another (one stream).
 struct LookBack {
   unsigned long long *words;
+  int64_t size;  // of words
   int *control;
   int *error;  // where a wait that runs out sets its error bit
   int polls;   // of a word before a wait runs out

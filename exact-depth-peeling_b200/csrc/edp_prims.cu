@@ -46,7 +46,8 @@ __device__ inline int block_exclusive(int v, int *smem, int &total) {
 // is bounded all the same, and running out sets an error.
 //
 // A published word holds the sum, a state and the launch's epoch, so the words
-// need no clearing between launches.  The last block to finish gives the
+// need no clearing between launches (but once in 2^30, when the epochs start
+// over: a few hours of replays of a small scene).  The last block to finish gives the
 // ticket back and starts the next epoch.
 //
 // Three launches per scan and per pass (counts, their scan, the scatter) cost
@@ -54,6 +55,7 @@ __device__ inline int block_exclusive(int v, int *smem, int &total) {
 // subdivision loop became 97.  Replays: icospheres-640 0.81 -> 0.72 ms,
 // knot-9702 1.14 -> 1.03, a batch of 16 small scenes 3.44 -> 3.03.
 enum Published : unsigned { kNothing = 0, kSum = 1, kPrefix = 2 };
+constexpr unsigned kEpochMask = 0x3fffffffu;
 
 __device__ inline unsigned long long publish_word(unsigned epoch, unsigned state, int value) {
   return (unsigned long long)(epoch << 2 | state) << 32 | unsigned(value);
@@ -77,7 +79,7 @@ __device__ inline unsigned long long await_word(const unsigned long long *p, uns
 // This block's tile (shared by all its threads) and the launch's epoch.
 __device__ inline int take_tile(LookBack s, int *shared, unsigned &epoch) {
   if (threadIdx.x == 0) shared[0] = atomicAdd(&s.control[0], 1);
-  epoch = *(volatile unsigned *)&s.control[2] & 0x3fffffffu;
+  epoch = *(volatile unsigned *)&s.control[2] & kEpochMask;
   __syncthreads();
   return shared[0];
 }
@@ -91,7 +93,12 @@ __device__ inline bool finish_tile(LookBack s, int tiles) {
   if (atomicAdd(&s.control[1], 1) != tiles - 1) return false;
   s.control[0] = 0;
   s.control[1] = 0;
-  s.control[2] = s.control[2] + 1;
+  const unsigned next = unsigned(s.control[2]) + 1u;
+  // The words' 30 epoch bits start over: a word that was last written 2^30
+  // launches ago would look like this epoch's.
+  if ((next & kEpochMask) == 0)
+    for (int64_t w = 0; w < s.size; ++w) s.words[w] = 0;
+  s.control[2] = int(next);
   return true;
 }
 

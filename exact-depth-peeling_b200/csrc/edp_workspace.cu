@@ -208,7 +208,8 @@ cudaError_t allocate_scratch(edp_peeler *p, SortScratch &s, int64_t largest_sort
   s.tiles = ceil_div(largest_sort, kSortTile);
   s.scan_tiles = ceil_div(largest_scan, kScanTile);
   EDP_CHECK(alloc(p, &s.hist, 256 * kSortPasses));
-  EDP_CHECK(alloc(p, &s.look_back.words, std::max(256 * s.tiles, s.scan_tiles)));
+  s.look_back.size = std::max(256 * s.tiles, s.scan_tiles);
+  EDP_CHECK(alloc(p, &s.look_back.words, s.look_back.size));
   EDP_CHECK(alloc(p, &s.look_back.control, 3));
   return cudaSuccess;
 }

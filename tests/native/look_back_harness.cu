@@ -20,11 +20,16 @@ T *device_copy(const T *host, int64_t count) {
 
 // Words and control for `tiles` tiles of `per` words each, with room for the
 // tickets past the last tile that skipped ones push blocks to.
-edp::SortScratch scratch(int64_t tiles, int per, int polls, int missing, int *error) {
+// At the last epoch the words hold sums of an old launch with the next one.
+edp::SortScratch scratch(int64_t tiles, int per, int polls, int missing, unsigned epoch,
+                         int *error) {
   edp::SortScratch s;
   s.tiles = s.scan_tiles = tiles;
-  const int control[3] = {missing, 0, 0};
-  s.look_back.words = device_copy<unsigned long long>(nullptr, (tiles + missing) * per);
+  const int control[3] = {missing, 0, int(epoch)};
+  s.look_back.size = (tiles + missing) * per;
+  const std::vector<unsigned long long> old(s.look_back.size,
+                                            epoch ? 2ull << 32 | 12345ull : 0ull);
+  s.look_back.words = device_copy(old.data(), s.look_back.size);
   s.look_back.control = device_copy(control, 3);
   s.look_back.error = error;
   s.look_back.polls = polls;
@@ -35,13 +40,13 @@ edp::SortScratch scratch(int64_t tiles, int per, int polls, int missing, int *er
 
 // Scans `values` twice with one state; errors[k] is the error word after the
 // k-th.  Returns the CUDA error.
-extern "C" int look_back_scan(const int *values, int n, int polls, int missing, int *out,
-                              int *errors) {
+extern "C" int look_back_scan(const int *values, int n, int polls, int missing,
+                              unsigned epoch, int *out, int *errors) {
   const int64_t tiles = edp::ceil_div(n, edp::kScanTile);
   int *in = device_copy(values, n), *scanned = device_copy<int>(nullptr, n);
   int *count = device_copy(&n, 1), *total = device_copy<int>(nullptr, 1);
   int *error = device_copy<int>(nullptr, 1);
-  edp::SortScratch s = scratch(tiles, 1, polls, missing, error);
+  edp::SortScratch s = scratch(tiles, 1, polls, missing, epoch, error);
   for (int k = 0; k < 2; ++k) {
     edp::scan_exclusive(in, scanned, count, n, total, s, nullptr);
     cudaMemcpy(errors + k, error, sizeof(int), cudaMemcpyDeviceToHost);
@@ -56,15 +61,15 @@ extern "C" int look_back_scan(const int *values, int n, int polls, int missing, 
 }
 
 // Sorts 16-bit `keys` twice with one state, the positions beside them.
-extern "C" int look_back_sort(const uint64_t *keys, int n, int polls, int missing, uint64_t *out,
-                              int *positions, int *errors) {
+extern "C" int look_back_sort(const uint64_t *keys, int n, int polls, int missing,
+                              unsigned epoch, uint64_t *out, int *positions, int *errors) {
   const int64_t tiles = edp::ceil_div(n, edp::kSortTile);
   std::vector<int> index(n);
   for (int i = 0; i < n; ++i) index[i] = i;
   uint64_t *k = device_copy(keys, n), *k_tmp = device_copy<uint64_t>(nullptr, n);
   int *v = device_copy(index.data(), n), *v_tmp = device_copy<int>(nullptr, n);
   int *count = device_copy(&n, 1), *error = device_copy<int>(nullptr, 1);
-  edp::SortScratch s = scratch(tiles, 256, polls, missing, error);
+  edp::SortScratch s = scratch(tiles, 256, polls, missing, epoch, error);
   for (int round = 0; round < 2; ++round) {
     cudaMemcpy(k, keys, sizeof(uint64_t) * n, cudaMemcpyHostToDevice);
     cudaMemcpy(v, index.data(), sizeof(int) * n, cudaMemcpyHostToDevice);

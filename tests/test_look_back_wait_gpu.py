@@ -1,6 +1,8 @@
-"""A look-back wait that runs out (csrc/edp_prims.cu): the kernel returns, its
-own error bit is set and named by no capacity, nothing is left behind for the
-next launch.  The tiles waited for are tickets that no block takes."""
+"""The ends of the look-back state (csrc/edp_prims.cu).  A wait that runs out:
+the kernel returns, its own error bit is set and named by no capacity, nothing
+is left behind for the next launch (the tiles waited for are tickets that no
+block takes).  And the epochs' start over after 2^30 launches, over words that
+an old launch left."""
 
 import ctypes
 import shutil
@@ -14,6 +16,7 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 WAIT = 4096  # EDP_ERR_BIT_WAIT
+LAST_EPOCH = (1 << 30) - 1
 
 
 @pytest.fixture(scope="module")
@@ -29,25 +32,25 @@ def lib(tmp_path_factory):
 
 
 # Tiles: 4,096 elements of a scan, 2,048 keys of a radix pass.
-@pytest.mark.parametrize("missing", [0, 1, 3])
+@pytest.mark.parametrize("missing,epoch", [(0, 0), (1, 0), (3, 0), (0, LAST_EPOCH)])
 @pytest.mark.parametrize("n", [4097, 8192, 100_001])
-def test_scan(lib, n, missing):
+def test_scan(lib, n, missing, epoch):
     values = np.random.default_rng(n).integers(0, 9, size=n).astype(np.int32)
     out, errors = np.zeros(n + 1, dtype=np.int32), np.zeros(2, dtype=np.int32)
-    assert lib.look_back_scan(values.ctypes.data_as(ctypes.c_void_p), n, 1000, missing,
+    assert lib.look_back_scan(values.ctypes.data_as(ctypes.c_void_p), n, 1000, missing, epoch,
                               out.ctypes.data_as(ctypes.c_void_p),
                               errors.ctypes.data_as(ctypes.c_void_p)) == 0
     assert errors[0] == (WAIT if missing else 0) and errors[1] == 0
     np.testing.assert_array_equal(out, np.concatenate([[0], np.cumsum(values)]))
 
 
-@pytest.mark.parametrize("missing", [0, 1, 3])
+@pytest.mark.parametrize("missing,epoch", [(0, 0), (1, 0), (3, 0), (0, LAST_EPOCH)])
 @pytest.mark.parametrize("n", [2049, 4096, 50_001])
-def test_sort(lib, n, missing):
+def test_sort(lib, n, missing, epoch):
     keys = np.random.default_rng(n).integers(0, 1 << 16, size=n).astype(np.uint64)
     out, positions = np.zeros(n, dtype=np.uint64), np.zeros(n, dtype=np.int32)
     errors = np.zeros(2, dtype=np.int32)
-    assert lib.look_back_sort(keys.ctypes.data_as(ctypes.c_void_p), n, 1000, missing,
+    assert lib.look_back_sort(keys.ctypes.data_as(ctypes.c_void_p), n, 1000, missing, epoch,
                               out.ctypes.data_as(ctypes.c_void_p),
                               positions.ctypes.data_as(ctypes.c_void_p),
                               errors.ctypes.data_as(ctypes.c_void_p)) == 0
