@@ -347,7 +347,7 @@ def run_batched(args, rank, world, local_rank):
         outside = np.zeros(2, dtype=np.int64)
         _lib.check(lib.edp_graph_kernels(p._ws.handle, outside.ctypes.data,
                                          outside.ctypes.data + 8), "graph kernels")
-        launches += int(outside[0] + outside[1] * i["rounds"])
+        launches += int(outside[0] + outside[1] * i["subdivision_loops"])
     cpu = None
     if world == 1 and not args.quick:
         from oracle import fastpeel
@@ -511,7 +511,7 @@ def measure_config(config, args, rank, world, local_rank, steps, e2e_steps, cpu_
     outside = np.zeros(2, dtype=np.int64)
     _lib.check(lib.edp_graph_kernels(p._ws.handle, outside.ctypes.data, outside.ctypes.data + 8),
                "graph kernels")
-    launches = int(outside[0] + outside[1] * check["rounds"])
+    launches = int(outside[0] + outside[1] * check["subdivision_loops"])
     report = None
     if audit_samples and rank == 0:
         from peel_b200.audit import peeler_vertex_audit
@@ -575,7 +575,7 @@ def measure_config(config, args, rank, world, local_rank, steps, e2e_steps, cpu_
                 "serial_value": e2e_serial_ms if e2e_steps else None},
         "gpu_launches": int(steps * launches),
         "kernels_per_replay": {"outside_loop": int(outside[0]), "per_round": int(outside[1]),
-                               "rounds": check["rounds"]},
+                               "rounds": check["subdivision_loops"]},
         "clocks": clocks.summary(),
         "stages_ms": stage_ms,
         "tuning": {"knobs": knobs, "default_ms": default_ms, "tuned_ms": tuned_ms,

@@ -27,6 +27,7 @@ constexpr int kCandidatesPerPass = 32;
 enum StatusSlot : int {
   kResidual = 0, kNextResidual = 1, kPolygons = 2, kTriangles = 3, kLayers = 4,
   kPass = 5, kBoundaryVertices = 6, kDepthTies = 8, kError = 9, kMaxHidden = 10,
+  kLoops = 11,  // of this build: iterations of the subdivision loop, clipping launches
   kPeakResidual = 12, kStatusSlots = 16
 };
 // Error bits (kernels.py:20-21, warp_peel/EVENTS.md:203-207).

@@ -272,7 +272,9 @@ __global__ void __launch_bounds__(kBlock, 8) k_candidates(Dev d) {
 }
 
 __global__ void k_loop_condition(Dev d) {
+  const bool fits = int64_t(d.n) <= d.cap.frontier;
   d.status[kPeakResidual] = d.status[kResidual];
+  d.metrics[kRounds] = fits && d.n > 0 && d.status[kError] == 0 ? 1 : 0;
   int c = d.status[kResidual] > 0 && d.status[kError] == 0;
   *d.condition = c;
   if (d.use_handle) cudaGraphSetConditional(d.cond_handle, unsigned(c));
@@ -402,7 +404,11 @@ __device__ inline int cuts(const Group<W> &g, V2 p, V2 q, int n, const Plane &sc
 
 // A frontier's patch pool.  `n` holds the vertex count and, above it, the
 // patch's generation: how many right-hand parts lie on its way from the
-// source.  A generation at Dev::cap.rounds is the round-capacity error.
+// source.  Generations are the reference's rounds (frontier.py:106-223, each
+// round's right-hand parts make up the next one's frontier): the counter is one
+// above the last generation, and a generation at Dev::cap.rounds is the
+// round-capacity error.  How many iterations of the loop they take here depends
+// on how the work is handed on, and is bounded by nothing but the candidates.
 constexpr int kSizeBits = 6;
 constexpr int kSizeMask = (1 << kSizeBits) - 1;
 
@@ -462,8 +468,9 @@ __device__ inline void advance_round(const Dev &d) {
   status[kResidual] = next;
   status[kNextResidual] = 0;
   sc[kFrontierNext] = 0;
-  long long rounds = ++d.metrics[kRounds];
-  if (rounds >= d.cap.rounds && next > 0) set_error(d.status, kErrRounds);
+  // Each iteration takes every patch past a candidate of its own at least.
+  const int loops = ++status[kLoops];
+  if (loops > sc[kSegmentCount] + 2 && next > 0) set_error(d.status, kErrWait);
   status[kPeakResidual] = max(status[kPeakResidual], next);
   *d.parity ^= 1;
   int c = next > 0 && status[kError] == 0;
@@ -533,7 +540,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
   const Segments segs = segments_of(d);
   const Frontier next{d.fv[par ^ 1], d.fn[par ^ 1], d.fsrc[par ^ 1], d.fcur[par ^ 1],
                       &d.status[kNextResidual], d.status, d.cap.frontier - parked};
-  int visits = 0, tests = 0, splits = 0;  // each group's lane 0
+  int visits = 0, tests = 0, splits = 0, deepest = 0;  // each group's lane 0
   CutTally tally;
   // With fewer patches than groups the round lasts as long as one group's chain.
   const bool few = live <= int(gridDim.x) * kGroups / 2;
@@ -725,6 +732,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
         keep_right = moved = true;
         p = pl;
         n = nl;
+        deepest = max(deepest, generation + 1);
         if (generation + 1 >= d.cap.rounds && g.lane == 0) set_error(d.status, kErrRounds);
       }
     }
@@ -767,6 +775,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
     count_add(&d.metrics[kTargetVisits], visits);
     count_add(&d.metrics[kContourTests], tests);
     count_add(&d.metrics[kSplits], splits);
+    if (deepest > 0) atomicMax(&d.metrics[kRounds], (long long)deepest + 1);
   }
   if constexpr (F == 2) {
     tally.side.flush(d, kPredSide);

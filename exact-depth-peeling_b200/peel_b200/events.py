@@ -119,4 +119,5 @@ class EventPeeler(_Peeler):
         for name in ("peeling_passes", "max_hidden_pieces"):
             info.pop(name)
         info.update(zip(METRIC_NAMES, map(int, metrics)))
+        info["subdivision_loops"] = int(status[11])
         return info

@@ -86,7 +86,10 @@ typedef struct edp_device_capacities {
 } edp_device_capacities;
 
 /* Device pointers of the workspace's buffers.  Counts live in status:
- * status[2] polygons, status[3] triangles, status[6] boundary vertices. */
+ * status[2] polygons, status[3] triangles, status[6] boundary vertices;
+ * status[11] iterations of the subdivision loop (metrics[6], what the rounds
+ * capacity bounds, counts generations of right-hand parts), or launches of the
+ * DevicePeeler's clipping. */
 typedef struct edp_outputs {
   int32_t *status;          /* [16] */
   int64_t *metrics;         /* [20] */
@@ -233,7 +236,7 @@ int edp_stage_times(edp_peeler *p, float *ms);
 
 /* Kernel nodes of the captured graph (the workspace's own, or the caller's
  * graph that edp_enqueue recorded it into): outside the subdivision loop, and
- * per loop iteration (a replay launches outside + per_round * rounds
+ * per loop iteration (a replay launches outside + per_round * status[11]
  * kernels). */
 int edp_graph_kernels(edp_peeler *p, int64_t *outside_loop, int64_t *per_round);
 
