@@ -272,8 +272,9 @@ __global__ void __launch_bounds__(kBlock, 8) k_candidates(Dev d) {
 }
 
 __global__ void k_loop_condition(Dev d) {
+  // The frontier must have room for every source, listed or not.
   const bool fits = int64_t(d.n) <= d.cap.frontier;
-  d.status[kPeakResidual] = d.status[kResidual];
+  d.status[kPeakResidual] = fits ? d.n : 0;
   d.metrics[kRounds] = fits && d.n > 0 && d.status[kError] == 0 ? 1 : 0;
   int c = d.status[kResidual] > 0 && d.status[kError] == 0;
   *d.condition = c;
@@ -471,7 +472,7 @@ __device__ inline void advance_round(const Dev &d) {
   // Each iteration takes every patch past a candidate of its own at least.
   const int loops = ++status[kLoops];
   if (loops > sc[kSegmentCount] + 2 && next > 0) set_error(d.status, kErrWait);
-  status[kPeakResidual] = max(status[kPeakResidual], next);
+  status[kPeakResidual] = max(status[kPeakResidual], next + deferred);
   *d.parity ^= 1;
   int c = next > 0 && status[kError] == 0;
   *d.condition = c;

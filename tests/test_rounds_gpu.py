@@ -1,5 +1,6 @@
 """The rounds' capacity counts generations of right-hand parts, as the
-reference's rounds do, however the loop hands the work on."""
+reference's rounds do, however the loop hands the work on; and a workspace
+sized by the usage that another one reports is large enough."""
 
 from dataclasses import replace
 
@@ -63,3 +64,36 @@ def test_a_long_chain_takes_no_rounds(count, form):
         else:
             with pytest.raises(RuntimeError, match="subdivision round"):
                 q.read_status()
+
+
+@pytest.mark.parametrize("scene", ["strips", "icospheres", "knot"])
+def test_pools_of_the_reported_usage_suffice(scene):
+    from peel_b200 import EventCapacities, EventPeeler, scenes
+
+    arrays = {"strips": lambda: strips(50), "knot": lambda: scenes.knot_tube(48, 24, seed=3),
+              "icospheres": icospheres}[scene]()
+    device = scenes.to_device(arrays)
+    wide = EventCapacities.for_mesh(64 * len(arrays[1]))
+    p = EventPeeler(*device, capacities=wide)
+    p.run()
+    info = p.read_status()
+    tight = replace(wide, frontier=info["peak_residual_patches"], rounds=info["rounds"],
+                    regions=info["polygons"])
+    q = EventPeeler(*device, capacities=tight)
+    for _ in range(2):
+        q.run()
+        again = q.read_status()
+        assert {k: again[k] for k in ("polygons", "layers", "rounds", "splits")} == \
+            {k: info[k] for k in ("polygons", "layers", "rounds", "splits")}
+
+
+def icospheres():
+    from peel_b200 import scenes
+
+    v, f = scenes.icosphere(2)
+    rng = np.random.default_rng(1)
+    outer = v * (1 + rng.uniform(-0.15, 0.15, size=(len(v), 1)))
+    inner = 0.5 * v * (1 + rng.uniform(-0.15, 0.15, size=(len(v), 1)))
+    return (np.concatenate([outer, inner]),
+            np.concatenate([f, f + len(v)]).astype(np.int32), np.diag([1.0, 1.0, -1.0, 1.0]),
+            np.array([-1.3, -1.3, 1.3, 1.3, 0.0, 0.01]))
