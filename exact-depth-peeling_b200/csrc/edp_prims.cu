@@ -86,17 +86,17 @@ __device__ inline int take_tile(LookBack s, int *shared, unsigned &epoch) {
 
 // Counts the block as finished; true in thread 0 of the launch's last block,
 // after the state is ready for the next launch.
-__device__ inline bool finish_tile(LookBack s, int tiles) {
+__device__ inline bool finish_tile(LookBack s, int tiles, unsigned epoch) {
   __syncthreads();
   if (threadIdx.x != 0) return false;
   __threadfence();
   if (atomicAdd(&s.control[1], 1) != tiles - 1) return false;
   s.control[0] = 0;
   s.control[1] = 0;
-  const unsigned next = unsigned(s.control[2]) + 1u;
+  const unsigned next = (epoch + 1u) & kEpochMask;
   // The words' 30 epoch bits start over: a word that was last written 2^30
   // launches ago would look like this epoch's.
-  if ((next & kEpochMask) == 0)
+  if (next == 0)
     for (int64_t w = 0; w < s.size; ++w) s.words[w] = 0;
   s.control[2] = int(next);
   return true;
@@ -179,7 +179,7 @@ k_scan(int *in, int *out, const int *count, LookBack s, int *total_out, int clea
     }
   }
   if (threadIdx.x == 0 && total_out && tile == tiles - 1) *total_out = s_before + total;
-  finish_tile(s, tiles);
+  finish_tile(s, tiles, epoch);
 }
 
 // ---------------------------------------------------------------- radix sort
@@ -292,18 +292,17 @@ __global__ void __launch_bounds__(kSortBlock) k_radix_pass(
   for (int r = 0; r < kSortItems; ++r) {
     unsigned peers = __match_any_sync(0xffffffffu, d[r]);
     if (d[r] < 256) {
-      int pos = wcount[warp][d[r]] + __popc(peers & lt);
+      // Below n, unless a wait ran out and left older keys in an earlier pass.
+      int pos = min(wcount[warp][d[r]] + __popc(peers & lt), n - 1);
       int64_t i = run + r * 32 + lane;
-      if (pos < n) {  // always, unless a wait ran out and left older keys in an earlier pass
-        keys_out[pos] = k[r];
-        vals_out[pos] = vals[i];
-      }
+      keys_out[pos] = k[r];
+      vals_out[pos] = vals[i];
     }
     __syncwarp();
     if (d[r] < 256 && lane == __ffs(peers) - 1) wcount[warp][d[r]] += __popc(peers);
     __syncwarp();
   }
-  const bool last = finish_tile(s, tiles);
+  const bool last = finish_tile(s, tiles, epoch);
   if (pass == passes - 1) {  // every block has read the digit counts
     if (threadIdx.x == 0) s_tile[0] = last;
     __syncthreads();
