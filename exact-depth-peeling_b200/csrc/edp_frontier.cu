@@ -110,7 +110,8 @@ struct CutTally {
 // the order of the hierarchy walk, and takes the same cuts.
 constexpr double kSideMargin = 1.0e-12;
 constexpr double kOutsideMargin = 1.0e-7;
-constexpr int kListBuffer = 192;  // entries a warp holds before it writes a list
+constexpr int kListMost = 192;    // entries of a list, held in shared memory until it is written
+constexpr int kScreenMost = 2048; // candidates screened for one list
 constexpr int kUnlisted = -1;     // Dev::cand_count of a source without a list
 
 // Can segment c cut a patch of the source v[0..n)?  `code` receives its depth
@@ -145,9 +146,14 @@ __device__ inline bool may_cut(const Segments &g, int c, const V2 *v, int n, con
 
 // One warp per source: its candidate list, and its first patch.  The warp
 // walks the contour hierarchy once with the source's box, and screens the
-// candidates 32 at a time, one per lane.  A source with an empty list is a final polygon as it is; any other
-// joins the frontier.  A source whose list does not fit the pool is left
-// without one, and its patches walk the hierarchy themselves.
+// candidates 32 at a time, one per lane.  A source with an empty list is a
+// final polygon as it is; any other joins the frontier.  A source with more
+// than kListMost entries or kScreenMost candidates, or whose list does not fit
+// the pool, is left without a list, and its patches search the hierarchy
+// themselves, in the second pass of each iteration.  A large triangle behind a fine mesh is such a
+// source: one warp would list its thousands of segments while the rest of the
+// GPU waits (1.5 ms for a floor behind the 65,536-face knot), and each of its
+// patches would look through all of them.
 // Bound by the latency of the walk's 4 to 5 dependent steps: 8 blocks per SM
 // with the candidates screened together, against 6 with each leaf group's few
 // by themselves, took the preparation of the 720K primitives from 2.92 to 2.55
@@ -157,7 +163,7 @@ __device__ inline bool may_cut(const Segments &g, int c, const V2 *v, int n, con
 // and 3.7M candidate tests against 65K walks, 0.19 ms here.
 template <int F>
 __global__ void __launch_bounds__(kBlock, 8) k_candidates(Dev d) {
-  __shared__ int2 s_list[kWarps][kListBuffer];
+  __shared__ int2 s_list[kWarps][kListMost];
   __shared__ int s_queue[kWarps][64];
   __shared__ V2 s_source[kWarps][kSourceVertices];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -187,12 +193,10 @@ __global__ void __launch_bounds__(kBlock, 8) k_candidates(Dev d) {
     const float4 hi = d.src_hi[s];
     lo.z = -1.0e30f;
     int total = 0, start = 0;
-    // The first walk lists up to kListBuffer entries; a longer list is written
-    // straight to its place by a second one.
-    for (int pass = 0; pass < 2; ++pass) {
+    {
       WarpWalk w;
       walk_begin(w, d.seg_tree, leaves, lo, hi, 0);
-      int budget = 0x7fffffff, first, resume, at = 0, queued = 0;
+      int budget = 0x7fffffff, first, resume, queued = 0, screened = 0;
       unsigned batch;
       // Screens the first 32 queued candidates, one per lane.
       auto screen = [&]() {
@@ -201,46 +205,44 @@ __global__ void __launch_bounds__(kBlock, 8) k_candidates(Dev d) {
         int code = 0;
         const bool keep = lane < queued && may_cut<F>(segs, c, v, n, sc, s, code, tally);
         const unsigned kept = __ballot_sync(kFull, keep);
-        const int slot = at + __popc(kept & below);
-        if (keep) {
-          if (pass == 1)
-            d.cand[int64_t(start) + slot] = make_int2(c, code);
-          else if (slot < kListBuffer)
-            list[slot] = make_int2(c, code);
-        }
-        at += __popc(kept);
+        const int slot = total + __popc(kept & below);
+        if (keep && slot < kListMost) list[slot] = make_int2(c, code);
+        total += __popc(kept);
+        screened += 32;
         __syncwarp();
         queue[lane] = rest;
         queued = max(0, queued - 32);
         __syncwarp();  // the next batch is written over the places past the rest
       };
-      while (walk_next(w, d.seg_tree, leaves, lo, hi, 0, budget, batch, first, resume)) {
+      while (total <= kListMost && screened <= kScreenMost &&
+             walk_next(w, d.seg_tree, leaves, lo, hi, 0, budget, batch, first, resume)) {
         if ((batch >> lane) & 1u)
           queue[queued + __popc(batch & below)] = __ldg(&segs.ids[first + lane]);
         queued += __popc(batch);
         if (queued >= 32) screen();
       }
-      if (queued > 0) screen();
-      if (pass == 1) break;
-      total = at;
-      if (total == 0) break;
+      if (queued > 0 && total <= kListMost && screened <= kScreenMost) screen();
+      if (total > kListMost || screened > kScreenMost) total = kUnlisted;
+    }
+    if (total > 0) {
       if (lane == 0)
         start = int(claim_entries(reinterpret_cast<unsigned long long *>(&d.sc[kCandidates]),
                                   total, d.cand_cap));
       start = __shfl_sync(kFull, start, 0);
       if (start < 0) {
         total = kUnlisted;
-        break;
-      }
-      if (total <= kListBuffer) {
+      } else {
         __syncwarp();
         for (int k = lane; k < total; k += 32) d.cand[int64_t(start) + k] = list[k];
         __syncwarp();
-        break;
       }
     }
     int slot = 0;
-    if (lane == 0) slot = atomicAdd(total == 0 ? &d.status[kPolygons] : &d.status[kResidual], 1);
+    if (lane == 0)
+      slot = atomicAdd(total == 0           ? &d.status[kPolygons]
+                       : total == kUnlisted ? &d.sc[kTopLive]
+                                            : &d.status[kResidual],
+                       1);
     slot = __shfl_sync(kFull, slot, 0);
     if (total == 0) {
       if (slot >= d.cap.regions) {
@@ -255,7 +257,8 @@ __global__ void __launch_bounds__(kBlock, 8) k_candidates(Dev d) {
       }
       continue;
     }
-    // slot < n <= frontier capacity
+    // The slots of both ends: at most n <= frontier capacity of them.
+    if (total == kUnlisted) slot = int(d.cap.frontier) - 1 - slot;
     if (lane < n) d.fv[0][int64_t(kMaxVertices) * slot + lane] = p;
     if (lane == 0) {
       d.fn[0][slot] = n;
@@ -276,7 +279,7 @@ __global__ void k_loop_condition(Dev d) {
   const bool fits = int64_t(d.n) <= d.cap.frontier;
   d.status[kPeakResidual] = fits ? d.n : 0;
   d.metrics[kRounds] = fits && d.n > 0 && d.status[kError] == 0 ? 1 : 0;
-  int c = d.status[kResidual] > 0 && d.status[kError] == 0;
+  int c = (d.status[kResidual] > 0 || d.sc[kTopLive] > 0) && d.status[kError] == 0;
   *d.condition = c;
   if (d.use_handle) cudaGraphSetConditional(d.cond_handle, unsigned(c));
 }
@@ -444,37 +447,73 @@ __device__ __noinline__ int64_t push_patch(Frontier f, int *count, bool top, boo
   return slot;
 }
 
-// The first leaf batch of the contour hierarchy at or after leaf `cursor`
-// whose leaves meet the box, for a source without a list (a walk from the
-// root each time: no walk state stays live in the caller).
-__device__ __noinline__ unsigned walk_batch(Tree t, int leaves, float4 lo, float4 hi, int cursor,
-                                            int &first) {
-  WarpWalk w;
-  walk_begin(w, t, leaves, lo, hi, cursor);
-  int budget = 0x7fffffff, resume;
-  unsigned batch;
-  return walk_next(w, t, leaves, lo, hi, cursor, budget, batch, first, resume) ? batch : 0u;
+// The first leaves of the contour hierarchy from leaf `cursor` on, up to 32
+// together, of which some meet the box: true for the lanes whose leaf does
+// (segment `id`), `base` the first one's number.  Moves the cursor past them;
+// no lane's answer is true at the end.  The hierarchy's descendants five levels
+// below a node are 32 consecutive nodes: a step tests them, a node per lane,
+// goes down to the first that meets the box, or on and up when none does.
+__device__ inline bool next_leaves(const Tree &t, int leaves, const Box &box, int &cursor,
+                                   int &base, int &id) {
+  const int lane = threadIdx.x & 31;
+  for (int level = 0; cursor < leaves;) {
+    const int nodes = leaves >> level, first = (cursor >> level) & ~31, node = first + lane;
+    const bool in = node >= cursor >> level && node < nodes;
+    int leaf_id = 0;
+    if (in && level == 0) leaf_id = __ldg(&t.ids[node]);  // in one latency with its box
+    const bool meets = in && overlaps(__ldg(&t.nodes[2 * (nodes + node)]),
+                                      __ldg(&t.nodes[2 * (nodes + node) + 1]), box.lo, box.hi);
+    const unsigned met = __ballot_sync(kFull, meets);
+    if (met && level > 0) {
+      cursor = max(cursor, (first + __ffs(int(met)) - 1) << level);
+      level -= 5;
+      continue;
+    }
+    cursor = first + 32 < nodes ? (first + 32) << level : leaves;
+    if (met) {
+      base = first;
+      id = leaf_id;
+      return meets;
+    }
+    if (leaves >> (level + 5) > 0) level += 5;
+  }
+  return false;
 }
 
-// Swap frontiers and decide whether another round runs (event_kernels.py:12-25).
-// Patches parked for the exact pass shared the next frontier's slots from the
-// top: together with the pushed ones they must have fit.
+// Swap frontiers and decide whether another iteration runs
+// (event_kernels.py:12-25).  The patches at the next frontier's top (parked for
+// the second pass, then those without a list) share its slots with the others:
+// together they must have fit.
 __device__ inline void advance_round(const Dev &d) {
-  volatile int *status = d.status, *sc = d.sc;
-  const int next = status[kNextResidual], deferred = sc[kDeferred];
-  if (int64_t(next) + deferred > d.cap.frontier) set_error(d.status, kErrResidual);
-  d.metrics[kParkedPatches] += deferred;
-  sc[kDeferred] = 0;
-  sc[kDeferredNext] = 0;
-  status[kResidual] = next;
-  status[kNextResidual] = 0;
-  sc[kFrontierNext] = 0;
+  // Loads past L1, of one latency together.
+  const int next = __ldcg(&d.status[kNextResidual]), deferred = __ldcg(&d.sc[kDeferred]);
+  const int pushed = __ldcg(&d.sc[kTopPushed]);
+  const int loops = __ldcg(&d.status[kLoops]) + 1, segments = __ldcg(&d.sc[kSegmentCount]);
+  const int peak = __ldcg(&d.status[kPeakResidual]), parity = __ldcg(d.parity);
+  const long long parked = __ldcg(&d.metrics[kParkedPatches]);
+  bool failed = __ldcg(&d.status[kError]) != 0;
+  if (int64_t(next) + deferred + pushed > d.cap.frontier) {
+    set_error(d.status, kErrResidual);
+    failed = true;
+  }
   // Each iteration takes every patch past a candidate of its own at least.
-  const int loops = ++status[kLoops];
-  if (loops > sc[kSegmentCount] + 2 && next > 0) set_error(d.status, kErrWait);
-  status[kPeakResidual] = max(status[kPeakResidual], next + deferred);
-  *d.parity ^= 1;
-  int c = next > 0 && status[kError] == 0;
+  if (loops > segments + 2 && next + pushed > 0) {
+    set_error(d.status, kErrWait);
+    failed = true;
+  }
+  d.metrics[kParkedPatches] = parked + deferred;
+  d.sc[kDeferred] = 0;
+  d.sc[kDeferredNext] = 0;
+  d.sc[kTopPushed] = 0;
+  d.sc[kFrontierNext] = 0;
+  d.sc[kTopFirst] = deferred;
+  d.sc[kTopLive] = pushed;
+  d.status[kResidual] = next;
+  d.status[kNextResidual] = 0;
+  d.status[kLoops] = loops;
+  d.status[kPeakResidual] = max(peak, next + deferred + pushed);
+  *d.parity = parity ^ 1;
+  const int c = next + pushed > 0 && !failed;
   *d.condition = c;
   if (d.use_handle) cudaGraphSetConditional(d.cond_handle, unsigned(c));
 }
@@ -492,8 +531,8 @@ constexpr int kFewCuts = 3;   // both, when there are fewer patches than groups
 // past kStack waiting parts or kLocalCuts cuts, in the next round's frontier,
 // where other groups take it; both have the cursor just past the cutting
 // segment.  After kMostCuts cuts the left part goes to the next round too.  A
-// patch that has met every candidate is final and goes to the output pool.  Groups take patches from a shared
-// counter.
+// patch that has met every candidate is final and goes to the output pool.
+// Groups take patches from a shared counter.
 //
 // The groups of a warp run one loop in step: take a patch, find its next
 // candidate, test it, split.  Every step is run by the whole warp when any
@@ -502,13 +541,21 @@ constexpr int kFewCuts = 3;   // both, when there are fewer patches than groups
 // W = 8 is the first pass of a round, with the filter-only form (F = 4) under
 // filtered binary64 predicates (no exact stage, so fewer registers and less
 // code).  It parks a patch at the top of the next frontier, with its cursor
-// at the candidate it stopped at, when its filters cannot decide, when a part
-// would have more than 8 vertices, or when its source has no list.  W = 32 is
-// the second pass, with the exact stages, over the parked patches: it takes
-// each one past the candidate that stopped it and hands it, or its two parts,
-// to the next round (a patch that no group of eight lanes can take goes on).
-// Each patch meets the same tests in the same order as in one exact pass, so
-// the output is the same.
+// at the candidate it stopped at, when its filters cannot decide, or when a
+// part would have more than 8 vertices.  W = 32 is the second pass, with the
+// exact stages.  It takes each parked patch past the candidate that stopped it
+// and hands it, or its two parts, to the next round (a patch that no group of
+// eight lanes can take goes on).  Then it takes the patches whose source has no
+// list, which lie at the frontier's top: they search the contour hierarchy for
+// the leaves from their cursor on that meet their box (next_leaves), the same
+// segments in the same order.  Each patch meets the same tests in the same
+// order as in one exact pass, so the output is the same.
+//
+// Reading a list of any length from end to end for every patch took 109 ms for
+// 2,000 strips in front of one triangle, 53 for 10,000 tiles and 43 for a floor
+// behind 200,000 faces of primitives; the search takes 27, 17 and 23.  In the
+// first pass's loop, even only called from there, it costs the listed patches
+// 10 to 15%.
 //
 // The time is instruction issue on patches of three to six vertices, and at
 // small sizes the chain of one group's steps: a warp per patch left 26 of 32
@@ -517,8 +564,7 @@ constexpr int kFewCuts = 3;   // both, when there are fewer patches than groups
 // 720K primitives 11.5 -> 3.2 ms, 2,560-face icospheres 0.60 -> 0.36 ms.  The
 // cut bounds trade a round's longest chain against the number of rounds:
 // unbounded chains took 1.2, 3.5 and 0.43 ms, and 8 cuts even for few patches
-// 1.04, 3.4 and 0.40.  4 blocks of 128 registers per
-// SM: 5 blocks spill (1.3 ms on the knot), 3 hide less latency (1.13).
+// 1.04, 3.4 and 0.40.  4 blocks of 128 registers per SM: 5 blocks spill (1.3 ms on the knot), 3 hide less latency (1.13).
 template <int F, int W>
 __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
   constexpr int kGroups = kBlock / W;
@@ -532,16 +578,15 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
   const int slot = threadIdx.x / W, lane = threadIdx.x & 31;
   V2 *left_part = s_parts[slot][0], *right_part = s_parts[slot][1];
   const int par = *d.parity;
-  const int from = kWide ? par ^ 1 : par;
-  const V2 *fv = d.fv[from];
-  const int *fn = d.fn[from], *fsrc = d.fsrc[from], *fcur = d.fcur[from];
+  // Parked in this iteration: at the next frontier's top.
   const int parked = kWide ? int(min(int64_t(d.sc[kDeferred]), d.cap.frontier)) : 0;
-  const int live = kWide ? parked : int(min(int64_t(d.status[kResidual]), d.cap.frontier));
+  const int live = kWide ? parked + d.sc[kTopLive]
+                         : int(min(int64_t(d.status[kResidual]), d.cap.frontier));
   int *taken = kWide ? &d.sc[kDeferredNext] : &d.sc[kFrontierNext];
   const Segments segs = segments_of(d);
   const Frontier next{d.fv[par ^ 1], d.fn[par ^ 1], d.fsrc[par ^ 1], d.fcur[par ^ 1],
                       &d.status[kNextResidual], d.status, d.cap.frontier - parked};
-  int visits = 0, tests = 0, splits = 0, deepest = 0;  // each group's lane 0
+  int visits = 0, tests = 0, splits = 0;  // each group's lane 0
   CutTally tally;
   // With fewer patches than groups the round lasts as long as one group's chain.
   const bool few = live <= int(gridDim.x) * kGroups / 2;
@@ -557,6 +602,14 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
   unsigned batch = 0;
   int base = 0, id = 0, code = 0;
   V2 ca = p, cb = p, cn = p;
+  // To the next frontier: to its top when the source has no list.
+  auto push_part = [&](bool want, V2 x, int size, int from) {
+    const bool up = kWide && want && count == kUnlisted;
+    if (!kWide || __any_sync(kFull, want && !up))
+      push_patch<W>(next, next.count, false, want && !up, x, size, source, from);
+    if (kWide && __any_sync(kFull, up))
+      push_patch<W>(next, &d.sc[kTopPushed], true, up, x, size, source, from);
+  };
   for (;;) {
     // Take a patch: from the group's stack, else from the frontier.
     bool fresh = false, park = false, final = false, push = false;
@@ -574,15 +627,21 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
       const int failed = __shfl_sync(kFull, *(volatile int *)&d.status[kError], 0);
       if (want && (at >= live || failed != 0)) drained = true;
       const bool take = want && !drained;
-      const int i = kWide ? int(d.cap.frontier) - 1 - at : at;  // parked from the top down
-      int size = 0;
+      int from = par, i = at, size = 0;
+      if (kWide) {  // from the top downwards: the parked ones, then those without a list
+        if (at < parked)
+          from = par ^ 1;
+        else
+          i += d.sc[kTopFirst] - parked;
+        i = int(d.cap.frontier) - 1 - i;
+      }
       if (take) {
-        size = fn[i];
+        size = d.fn[from][i];
         n = size & kSizeMask;
         generation = size >> kSizeBits;
-        source = fsrc[i];
-        cursor = fcur[i];
-        p = g.lane < n ? fv[int64_t(kMaxVertices) * i + g.lane] : v2(0.0, 0.0);
+        source = d.fsrc[from][i];
+        cursor = d.fcur[from][i];
+        p = g.lane < n ? d.fv[from][int64_t(kMaxVertices) * i + g.lane] : v2(0.0, 0.0);
         sc = d.scores[source];
         start = d.cand_start[source];
         count = d.cand_count[source];
@@ -591,14 +650,15 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
       }
       if (!kWide) {
         // A patch too large for a group (left by the second pass of an earlier
-        // round), or one without a list: to this round's second pass.
-        const bool wide = take && (n > W || count == kUnlisted);
+        // round): to this round's second pass.
+        const bool wide = take && n > W;
         if (__any_sync(kFull, wide)) {
           const int64_t to =
               push_patch<W>(next, &d.sc[kDeferred], true, wide, p, size, source, cursor);
           if (to >= 0)
             for (int j = W + g.lane; j < n; j += W)
-              next.v[int64_t(kMaxVertices) * to + j] = fv[int64_t(kMaxVertices) * i + j];
+              next.v[int64_t(kMaxVertices) * to + j] =
+                  d.fv[par][int64_t(kMaxVertices) * i + j];
           fresh = fresh && !wide;
         }
       }
@@ -619,35 +679,21 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
       changed = false;
       __syncwarp();
     }
-    // Find the next chunk with a candidate.
+    // Find the next chunk with a candidate: of the source's list, or (second
+    // pass, no list) of the contour hierarchy's leaves.
     const int most = W == 8 ? __reduce_max_sync(kFull, n) : n;
     for (;;) {
       bool look = !idle && !push && !final && batch == 0;
       if (!__any_sync(kFull, look)) break;
+      const bool search = kWide && count == kUnlisted;
+      const int entries = search ? *d.seg_tree.size : count;
       bool meets = false;
-      if (kWide && count == kUnlisted) {
-        const int leaves = *d.seg_tree.size;
-        int first = 0;
-        const unsigned found = walk_batch(d.seg_tree, leaves, box.lo, box.hi, cursor, first);
-        final = found == 0;
-        if (!final) {
-          base = first;
-          cursor = base + W;
-          meets = (found >> g.lane) & 1u;
-          if (meets) {
-            id = __ldg(&segs.ids[base + g.lane]);
-            code = kDepthOpen;
-            ca = segs.a[id];
-            cb = segs.b[id];
-            cn = segs.near[id];
-          }
-        }
-      } else if (look) {
-        if (cursor >= count) {
+      if (look) {
+        if (cursor >= entries) {
           final = true;
         } else if (--budget < 0) {
           push = true;  // a long walk carries over, so that one patch does not hold a round
-        } else {
+        } else if (!search) {
           base = cursor;
           cursor += W;
           if (base + g.lane < count) {
@@ -663,8 +709,17 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
           }
         }
       }
+      if (search && !final && !push) {  // the patch of the whole warp
+        meets = next_leaves(d.seg_tree, entries, box, cursor, base, id);
+        if (meets) {
+          code = kDepthOpen;
+          ca = segs.a[id];
+          cb = segs.b[id];
+          cn = segs.near[id];
+        }
+      }
       tests += __popc(g.ballot(meets));
-      if (!kWide && __any_sync(kFull, meets)) {
+      if ((!kWide || search) && __any_sync(kFull, meets)) {
         const bool missed = certainly_missed<F>(s_patch[slot], n, most, ca, cb, meets);
         meets = meets && !missed;
       }
@@ -682,7 +737,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
           if (g.lane == 0) {
             d.out_n[out] = n;
             d.out_src[out] = source;
-            d.out_layer[out] = 0;
+            d.out_layer[out] = generation;  // until the ranks are there (k_order_count)
           }
         }
       }
@@ -733,7 +788,6 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
         keep_right = moved = true;
         p = pl;
         n = nl;
-        deepest = max(deepest, generation + 1);
         if (generation + 1 >= d.cap.rounds && g.lane == 0) set_error(d.status, kErrRounds);
       }
     }
@@ -746,7 +800,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
       keep_right = false;
     }
     if (__any_sync(kFull, keep_right))
-      push_patch<W>(next, next.count, false, keep_right, pr, right_size, source, base + k + 1);
+      push_part(keep_right, pr, right_size, base + k + 1);
     // The rest of the chunk is met again by the left part: a segment that ends
     // on an edge of the patch may cut a part by a rounding of that edge.
     if (moved) {
@@ -761,8 +815,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
     }
     // Patches that leave the group: back to the frontier, or from the undecided
     // candidate on to the second pass.
-    if (__any_sync(kFull, push))
-      push_patch<W>(next, next.count, false, push, p, n | generation << kSizeBits, source, cursor);
+    if (__any_sync(kFull, push)) push_part(push, p, n | generation << kSizeBits, cursor);
     if (!kWide && __any_sync(kFull, park))
       push_patch<W>(next, &d.sc[kDeferred], true, park, p, n | generation << kSizeBits, source,
                     base + k);
@@ -776,14 +829,13 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
     count_add(&d.metrics[kTargetVisits], visits);
     count_add(&d.metrics[kContourTests], tests);
     count_add(&d.metrics[kSplits], splits);
-    if (deepest > 0) atomicMax(&d.metrics[kRounds], (long long)deepest + 1);
   }
   if constexpr (F == 2) {
     tally.side.flush(d, kPredSide);
     tally.segment.flush(d, kPredSegment);
     tally.depth.flush(d, kPredDepth);
   }
-  if constexpr (kWide) {  // the second pass's last block ends the round
+  if constexpr (kWide) {  // the second pass's last block ends the iteration
     __syncthreads();
     if (threadIdx.x == 0) {
       __threadfence();

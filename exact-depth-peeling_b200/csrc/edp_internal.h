@@ -157,7 +157,13 @@ enum Scalar : int {
   // Clipping: pieces spilled for the next launch, and pieces queued or in a warp.
   kClipSpill = 36,
   kClipPending = 37,
-  kScalarCount = 38  // k_reset clears them with its first threads
+  // Patches of sources without a candidate list, at the frontier's top: how
+  // many, the slots above them (of patches that are done), and those pushed for
+  // the next frontier.
+  kTopLive = 38,
+  kTopFirst = 39,
+  kTopPushed = 40,
+  kScalarCount = 41  // k_reset clears them with its first threads
 };
 static_assert(kCandidates % 2 == 0, "a 64-bit counter");
 

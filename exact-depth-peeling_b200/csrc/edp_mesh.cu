@@ -201,13 +201,24 @@ __device__ inline int live_outputs(const Dev &d) {
   return int(min(int64_t(d.status[kPolygons]), d.cap.regions));
 }
 
+// The rounds that a subdivision made: one above the generations, which the
+// polygons carry in place of their layers until they are ranked.
+__device__ inline void count_rounds(const Dev &d, int generation) {
+  generation = __reduce_max_sync(kFull, generation);
+  if ((threadIdx.x & 31) == 0 && generation >= *(volatile long long *)&d.metrics[kRounds])
+    atomicMax(&d.metrics[kRounds], (long long)generation + 1);
+}
+
 __global__ void k_order_keys(Dev d) {
   const int live = live_outputs(d);
+  int generation = 0;
   if (tid() == 0) d.sc[kLivePolygons] = live;
   for (int64_t i = tid(); i < live; i += stride()) {
     d.order_keys[i] = morton_of(d, i);
     d.order[i] = int(i);
+    generation = max(generation, d.out_layer[i]);
   }
+  count_rounds(d, generation);
 }
 
 // The same order by a counting sort: buckets of the leading Morton bits, below
@@ -237,6 +248,7 @@ __global__ void k_order_count(Dev d, int layered) {
     d.sc[kLivePolygons] = live;
     d.sc[kOrderLive] = 1 << (layer_bits + morton_bits);
   }
+  int generation = 0;
   for (int64_t i = tid(); i < live; i += stride()) {
     int bucket = int(morton_of(d, i) >> (24 - morton_bits));
     if (layered) {
@@ -244,8 +256,10 @@ __global__ void k_order_count(Dev d, int layered) {
       const int layer = min(max(d.out_layer[i], 0) >> layer_shift, (1 << layer_bits) - 1);
       bucket |= layer << morton_bits;
     }
+    if (!layered) generation = max(generation, d.out_layer[i]);
     d.order_keys[i] = uint64_t(bucket) << 32 | unsigned(atomicAdd(&d.order_count[bucket], 1));
   }
+  if (!layered) count_rounds(d, generation);
 }
 
 // Places the polygons, and lays out what the stage scans next: each polygon's

@@ -166,3 +166,25 @@ def test_long_and_short_lists_past_the_pool(form):
         parity.assert_areas({key: a for key, a in parity.gpu_areas(parity.polygons(p),
                                                                    range(n)).items() if a},
                             {key: a for key, a in area.items() if a})
+
+
+# 3 side^2 + 4 segments: hierarchies of 2^10, 2^12 and 2^14 leaves.
+@pytest.mark.parametrize("form", ["filtered64", "filtered", "binary64"])
+@pytest.mark.parametrize("side", [17, 30, 60])
+def test_a_frontier_of_the_sources_suffices(side, form):
+    """One sheet behind many tiles, whose patches search the hierarchy, cut
+    into several times as many patches as there are faces, with a frontier that
+    just holds the faces."""
+    from peel_b200 import EventCapacities, EventPeeler, scenes
+
+    arrays = tiles_over_sheets(side, 1)
+    n = len(arrays[1])
+    capacities = replace(EventCapacities.for_mesh(32 * n), frontier=n, layers=8)
+    p = EventPeeler(*scenes.to_device(arrays), predicates=form, capacities=capacities)
+    p.run()
+    info = p.read_status()
+    assert info["polygons"] > 5 * n and info["peak_residual_patches"] <= n
+    areas = parity.gpu_areas(parity.polygons(p), range(n))
+    covered = sum(areas[(0, s)] for s in range(n - 1))
+    assert abs(areas[(1, n - 1)] - covered) <= 1e-9
+    assert abs(areas[(0, n - 1)] + covered - 1.0) <= 1e-9
