@@ -110,7 +110,10 @@ struct CutTally {
 // the order of the hierarchy walk, and takes the same cuts.
 constexpr double kSideMargin = 1.0e-12;
 constexpr double kOutsideMargin = 1.0e-7;
-constexpr int kListMost = 192;    // entries of a list, held in shared memory until it is written
+// Entries of a list, held in shared memory until it is written.  One sheet
+// behind 100 tiles has 304: 0.89 ms with its list, 1.00 with the search; behind
+// 400 tiles, with 1,204, 2.9 ms with the list and 2.5 with the search.
+constexpr int kListMost = 384;
 constexpr int kScreenMost = 2048; // candidates screened for one list
 constexpr int kUnlisted = -1;     // Dev::cand_count of a source without a list
 
