@@ -19,6 +19,11 @@ constexpr int kHeavyBlock = 256;
 constexpr int kHeavyBlocks = 148 * 8;
 constexpr int kCells = 1024;         // 32 x 32 image buckets (beams.py:18-22)
 
+unsigned blocks(int64_t n) {
+  int64_t g = ceil_div(n > 0 ? n : 1, kBlock);
+  return unsigned(g < 148 * 16 ? g : 148 * 16);
+}
+
 __device__ inline int64_t tid() { return blockIdx.x * int64_t(blockDim.x) + threadIdx.x; }
 __device__ inline int64_t stride() { return int64_t(gridDim.x) * blockDim.x; }
 __device__ inline void add_metric(const Dev &d, int m, long long v) { count_add(&d.metrics[m], v); }
@@ -226,36 +231,72 @@ __device__ inline bool segment_cells(const Dev &d, int c, int &cx0, int &cx1, in
   return true;
 }
 
-__global__ void k_seg_grid_count(Dev d) {
-  const int total = d.sc[kSegmentCount];
-  for (int64_t c = tid(); c < total; c += stride()) {
-    int cx0, cx1, cy0, cy1;
-    if (!segment_cells(d, int(c), cx0, cx1, cy0, cy1)) continue;
-    if ((cx1 - cx0 + 1) * (cy1 - cy0 + 1) > d.seg_cells) {
-      d.seg_big[reserve(&d.sc[kSegBig], 1)] = int(c);
-      continue;
-    }
+// The cells of a range by L lanes together, this one `lane`.
+//
+// A large triangle of a small scene is listed in up to all 1,024 cells.  One
+// thread took an atomic after the other, each of whose results it needs: 165 us
+// for the few sources of a smallest scene and 78 for their segments; a warp
+// takes 11 and 8 (two triangles that fill the view: 0.44 -> 0.26 ms in all).  A
+// warp per item while the grid has one for each, eight lanes while listings
+// (of `cells` cells at most) are long enough to share, else a thread: 20,000
+// and more faces take the same time either way.
+template <int L, class F>
+__device__ inline void each_cell(int lane, int cx0, int cx1, int cy0, int cy1, F &&f) {
+  if constexpr (L == 1) {
     for (int cy = cy0; cy <= cy1; ++cy)
-      for (int cx = cx0; cx <= cx1; ++cx) atomicAdd(&d.seg_count[cy * d.grid_size + cx], 1);
+      for (int cx = cx0; cx <= cx1; ++cx) f(cx, cy);
+  } else {
+    const int width = cx1 - cx0 + 1, cells = width * (cy1 - cy0 + 1);
+#pragma unroll 4
+    for (int k = lane; k < cells; k += L) f(cx0 + k % width, cy0 + k / width);
   }
 }
 
+constexpr int kWarpItems = 148 * 16 * (kBlock / 32);  // warps of a full grid
+
+inline int grid_lanes(int64_t items, int cells) {
+  return items <= kWarpItems ? 32 : cells > kRayCells ? 8 : 1;
+}
+
+#define EDP_LAUNCH_LANES(lanes, kernel, items, stream, dev)                               \
+  do {                                                                                    \
+    if ((lanes) == 32) kernel<32><<<blocks(32 * (items)), kBlock, 0, stream>>>(dev);      \
+    else if ((lanes) == 8) kernel<8><<<blocks(8 * (items)), kBlock, 0, stream>>>(dev);    \
+    else kernel<1><<<blocks(items), kBlock, 0, stream>>>(dev);                            \
+    note_launch();                                                                        \
+  } while (0)
+
+template <int L>
+__global__ void k_seg_grid_count(Dev d) {
+  const int total = d.sc[kSegmentCount], lane = int(threadIdx.x % L);
+  for (int64_t c = tid() / L; c < total; c += stride() / L) {
+    int cx0, cx1, cy0, cy1;
+    if (!segment_cells(d, int(c), cx0, cx1, cy0, cy1)) continue;
+    if ((cx1 - cx0 + 1) * (cy1 - cy0 + 1) > d.seg_cells) {
+      if (lane == 0) d.seg_big[reserve(&d.sc[kSegBig], 1)] = int(c);
+      continue;
+    }
+    each_cell<L>(lane, cx0, cx1, cy0, cy1,
+                 [&](int cx, int cy) { atomicAdd(&d.seg_count[cy * d.grid_size + cx], 1); });
+  }
+}
+
+template <int L>
 __global__ void k_seg_grid_fill(Dev d) {
   if (tid() == 0) d.sc[kSegGridOn] = d.sc[kSegBig] <= 64 ? 1 : 0;
-  const int total = d.sc[kSegmentCount];
-  for (int64_t c = tid(); c < total; c += stride()) {
+  const int total = d.sc[kSegmentCount], lane = int(threadIdx.x % L);
+  for (int64_t c = tid() / L; c < total; c += stride() / L) {
     int cx0, cx1, cy0, cy1;
     if (!segment_cells(d, int(c), cx0, cx1, cy0, cy1)) continue;
     if ((cx1 - cx0 + 1) * (cy1 - cy0 + 1) > d.seg_cells) continue;
     const float4 lo = d.seg_lo[c], hi = d.seg_hi[c];
     const float4 box = make_float4(lo.x, lo.y, hi.x, hi.y);
-    for (int cy = cy0; cy <= cy1; ++cy)
-      for (int cx = cx0; cx <= cx1; ++cx) {
-        const int cell = cy * d.grid_size + cx;
-        const int e = d.seg_start[cell] + atomicSub(&d.seg_count[cell], 1) - 1;
-        d.seg_entries[e] = int(c);
-        d.seg_boxes[e] = box;
-      }
+    each_cell<L>(lane, cx0, cx1, cy0, cy1, [&](int cx, int cy) {
+      const int cell = cy * d.grid_size + cx;
+      const int e = d.seg_start[cell] + atomicSub(&d.seg_count[cell], 1) - 1;
+      d.seg_entries[e] = int(c);
+      d.seg_boxes[e] = box;
+    });
   }
 }
 
@@ -661,6 +702,7 @@ __device__ inline bool edges_exclude(const Dev &d, int s, float x, float y) {
          c.x * x + c.y * y + c.z < c.w;
 }
 
+template <int L>
 __global__ void k_ray_grid_count(Dev d) {
   // Each source's leaf in the source hierarchy (the order of its binary walk).
   const int leaves = *d.source_tree.size;
@@ -668,36 +710,38 @@ __global__ void k_ray_grid_count(Dev d) {
     const int s = d.source_tree.ids[leaf];
     if (s < d.n) d.leaf_of[s] = int(leaf);
   }
-  for (int64_t s = tid(); s < d.n; s += stride()) {
-    edge_functions(d, s);
+  const int lane = int(threadIdx.x % L);
+  for (int64_t s = tid() / L; s < d.n; s += stride() / L) {
+    if (lane == 0) edge_functions(d, s);
     int cx0, cx1, cy0, cy1;
     if (!source_cells(d, int(s), cx0, cx1, cy0, cy1)) continue;
     if ((cx1 - cx0 + 1) * (cy1 - cy0 + 1) > d.ray_cells) {
-      d.ray_big[reserve(&d.sc[kRayBig], 1)] = int(s);
+      if (lane == 0) d.ray_big[reserve(&d.sc[kRayBig], 1)] = int(s);
       continue;
     }
-    for (int cy = cy0; cy <= cy1; ++cy)
-      for (int cx = cx0; cx <= cx1; ++cx) atomicAdd(&d.ray_count[cy * d.grid_size + cx], 1);
+    each_cell<L>(lane, cx0, cx1, cy0, cy1,
+                 [&](int cx, int cy) { atomicAdd(&d.ray_count[cy * d.grid_size + cx], 1); });
   }
 }
 
 // Counting sort: ray_start is the scan of the counts; each listing takes a
 // slot of its cell.  The grid serves the rays when few sources are big.
+template <int L>
 __global__ void k_ray_grid_fill(Dev d) {
   if (tid() == 0) d.sc[kRayGridOn] = d.sc[kRayBig] <= 64 ? 1 : 0;
-  for (int64_t s = tid(); s < d.n; s += stride()) {
+  const int lane = int(threadIdx.x % L);
+  for (int64_t s = tid() / L; s < d.n; s += stride() / L) {
     int cx0, cx1, cy0, cy1;
     if (!source_cells(d, int(s), cx0, cx1, cy0, cy1)) continue;
     if ((cx1 - cx0 + 1) * (cy1 - cy0 + 1) > d.ray_cells) continue;
     const float4 lo = d.src_lo[s], hi = d.src_hi[s];
     const float4 box = make_float4(lo.x, lo.y, hi.x, hi.y);
-    for (int cy = cy0; cy <= cy1; ++cy)
-      for (int cx = cx0; cx <= cx1; ++cx) {
-        const int c = cy * d.grid_size + cx;
-        const int e = d.ray_start[c] + atomicSub(&d.ray_count[c], 1) - 1;
-        d.ray_entries[e] = int(s);
-        d.ray_boxes[e] = box;
-      }
+    each_cell<L>(lane, cx0, cx1, cy0, cy1, [&](int cx, int cy) {
+      const int c = cy * d.grid_size + cx;
+      const int e = d.ray_start[c] + atomicSub(&d.ray_count[c], 1) - 1;
+      d.ray_entries[e] = int(s);
+      d.ray_boxes[e] = box;
+    });
   }
 }
 
@@ -1535,11 +1579,6 @@ __global__ void k_merge_finish(Dev d) {
   d.sc[kLivePolygons] = d.sc[kMergedLive];
 }
 
-unsigned blocks(int64_t n) {
-  int64_t g = ceil_div(n > 0 ? n : 1, kBlock);
-  return unsigned(g < 148 * 16 ? g : 148 * 16);
-}
-
 int bits_for(int64_t n) {
   int b = 1;
   while ((int64_t(1) << b) < n + 1) ++b;
@@ -1550,23 +1589,22 @@ int bits_for(int64_t n) {
 
 cudaError_t stage_ray_grid(const Dev &d, SortScratch &s, cudaStream_t st) {
   const int64_t cells = int64_t(d.grid_size) * d.grid_size;
-  k_ray_grid_count<<<blocks(d.n), kBlock, 0, st>>>(d);
-  note_launch();
+  const int lanes = grid_lanes(d.n, d.ray_cells);
+  EDP_LAUNCH_LANES(lanes, k_ray_grid_count, int64_t(d.n), st, d);
   EDP_CHECK(scan_exclusive(d.ray_count, d.ray_start, d.sc + kRayGridCells, cells,
                            d.ray_start + cells, s, st));
-  k_ray_grid_fill<<<blocks(d.n), kBlock, 0, st>>>(d);
-  note_launch();
+  EDP_LAUNCH_LANES(lanes, k_ray_grid_fill, int64_t(d.n), st, d);
   return cudaGetLastError();
 }
 
 cudaError_t stage_segment_grid(const Dev &d, SortScratch &s, cudaStream_t st) {
   const int64_t cells = int64_t(d.grid_size) * d.grid_size;
-  k_seg_grid_count<<<blocks(kSourceVertices * int64_t(d.n)), kBlock, 0, st>>>(d);
-  note_launch();
+  // Up to kSourceVertices segments a source, mostly less than one.
+  const int lanes = grid_lanes(kSourceVertices / 2 * int64_t(d.n), d.seg_cells);
+  EDP_LAUNCH_LANES(lanes, k_seg_grid_count, kSourceVertices * int64_t(d.n), st, d);
   EDP_CHECK(scan_exclusive(d.seg_count, d.seg_start, d.sc + kRayGridCells, cells,
                            d.seg_start + cells, s, st));
-  k_seg_grid_fill<<<blocks(kSourceVertices * int64_t(d.n)), kBlock, 0, st>>>(d);
-  note_launch();
+  EDP_LAUNCH_LANES(lanes, k_seg_grid_fill, kSourceVertices * int64_t(d.n), st, d);
   return cudaGetLastError();
 }
 
