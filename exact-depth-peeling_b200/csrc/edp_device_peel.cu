@@ -201,15 +201,15 @@ __global__ void k_active_bounds(Dev d) {
 // from the source hierarchy, then the other residual patches from the
 // residual hierarchy (src/peel_common.h:169-199).  The work is a queue of
 // pieces: a piece is a convex part of a target with the position of its
-// candidate walk (which hierarchy, and the first leaf it has not met).  Each
-// clipping round runs every queued piece, a warp each, against the candidates
-// of up to Dev::clip_budget hierarchy steps.  A candidate that cuts a piece
+// candidate walk (which hierarchy, and the first leaf it has not met).  A
+// clipping launch runs every queued piece, a warp each, against all of its
+// candidates.  A candidate that cuts a piece
 // splits off the parts of the piece outside the candidate (or nearer than
 // it), and the part the candidate hides goes to the layer's hidden pool; one
-// of the parts goes on in the same warp, the others are queued for the next
-// round with the walk position past the candidate.  A piece that meets no
-// more candidates is visible in this layer.  Rounds repeat (a conditional
-// WHILE node inside the layer loop) until the queue is empty; then a target
+// of the parts goes on in the same warp, the others are queued with the walk
+// position past the candidate.  A piece that meets no more candidates is
+// visible in this layer.  Launches repeat (a conditional WHILE node inside the
+// layer loop) until no piece is left over; then a target
 // none of whose pieces stayed visible is hidden whole, as the exact route
 // restores it (src/bvh_peel.cpp:141-199), and the hidden pieces form the next
 // layer's residual.  The work and hidden pools are shared by all targets and
@@ -499,6 +499,7 @@ __global__ void k_clip_begin(Dev d) {
     d.sc[kClipNext] = queued;
     d.sc[kClipSpill] = 0;
     d.sc[kClipPending] = queued;
+    d.sc[kClipTurns] = 0;
     d.sc[kClipHidden] = 0;
     d.sc[kClipParity] = 0;
     d.sc[kFrontierNext] = 0;
@@ -520,6 +521,7 @@ __device__ inline void advance_clipping(const Dev &d) {
   sc[kClipPending] = spilled;
   sc[kFrontierNext] = 0;
   sc[kClipParity] = sc[kClipParity] ^ 1;
+  d.status[kLoops] = *(volatile int *)&d.status[kLoops] + 1;
   ++*d.clip_epoch;
   const int c = spilled > 0 && *(volatile int *)&d.status[kError] == 0;
   sc[kClipCondition] = c;
@@ -535,8 +537,13 @@ __device__ inline void advance_clipping(const Dev &d) {
 // Warps take slots of the queue by ticket and wait for the slot to be written,
 // or for the last piece to end.  A waited-for slot is written by a warp that
 // holds a piece and waits for nothing, so every wait ends; each is bounded all
-// the same (kWaitLimit polls, about a second, without a piece queued or ended),
-// and running out is an error.
+// the same (kWaitLimit polls, about a second, without a piece queued or ended
+// or a turn of Dev::clip_budget walk steps), and running out is an error.
+//
+// A walk is not put back into the queue between its turns: the queue's slots
+// are written once per launch, so that they are as many as the pieces (a target
+// or an uncovered part each, which ends as a visible or a hidden piece, or
+// several), however long their walks are.
 //
 // The bound is the serial chain of cuts of one piece, not throughput: a layer
 // has a few thousand pieces for 148 SMs.  A thread per piece, with its polygons
@@ -546,6 +553,7 @@ __device__ inline void advance_clipping(const Dev &d) {
 // cuts took 10.1 and 7.0, with the queue taken while it grows 5.4 and 3.2.
 // More polls, longer or shorter turns and half the blocks are all within 2%.
 constexpr int kWaitLimit = 1 << 20;
+constexpr int kMostSteps = 1024;  // of a turn, far less than a wait's limit takes
 
 template <int F>
 __global__ void __launch_bounds__(kBlock, 4) k_clip_round(Dev d) {
@@ -574,28 +582,35 @@ __global__ void __launch_bounds__(kBlock, 4) k_clip_round(Dev d) {
     int i = 0;
     if (lane == 0) {
       i = atomicAdd(&d.sc[kFrontierNext], 1);
-      // Slots below `live` were written before this launch.
+      if (i >= d.work_cap) i = -1;
       int seen = 0;
-      for (int polls = 0;; ++polls) {
-        if (*(volatile int *)&d.status[kError] != 0 || i >= d.work_cap) {
+      for (int polls = 0; i >= 0; ++polls) {
+        // Loaded together, for one latency per poll.
+        const int failed = *(volatile int *)&d.status[kError];
+        const int ready = *(volatile int *)&queue.ready[i];
+        const int pending = *(volatile int *)queue.pending;
+        if (failed != 0) {
           i = -1;
           break;
         }
-        if (i < live || *(volatile int *)&queue.ready[i] == queue.epoch) break;
-        const int pending = *(volatile int *)queue.pending;
+        // Slots below `live` were written before this launch.
+        if (i < live || ready == queue.epoch) break;
         if (pending <= 0) {  // every piece has ended, so no slot is written any more
           i = -1;
           break;
         }
-        const int progress = pending + *(volatile int *)queue.pool.count;
-        if (progress != seen) polls = 0;
-        seen = progress;
+        if ((polls & 63) == 63) {
+          const int progress = pending + *(volatile int *)queue.pool.count +
+                               *(volatile int *)&d.sc[kClipTurns];
+          if (progress != seen) polls = 0;
+          seen = progress;
+        }
         if (polls > kWaitLimit) {
           set_error(d.status, kErrWait);
           i = -1;
           break;
         }
-        __nanosleep(200);
+        __nanosleep(400);
       }
       __threadfence();
     }
@@ -617,22 +632,29 @@ __global__ void __launch_bounds__(kBlock, 4) k_clip_round(Dev d) {
     V2 q = Group<32>().shfl(p, lane + 1 < n ? lane + 1 : 0);
     const int source = d.res_src[rpar][target];
     const Plane st = d.scores[source];
-    // At least the steps from the root to a leaf group, so that every turn
-    // moves the walk on.
-    int budget = max(d.clip_budget, 8);
+    const int turn = min(max(d.clip_budget, 8), kMostSteps);
+    int budget = turn;
     bool done = false;  // nothing of the piece is left in this warp
     for (int tree = start >> kCursorTree; tree < 2 && !done; ++tree) {
       const Tree &t = tree == 0 ? d.source_tree : d.residual_tree;
       const int leaves = tree == 0 ? source_leaves : residual_leaves;
-      const int cursor = tree == start >> kCursorTree ? start & kCursorLeaf : 0;
+      int cursor = tree == start >> kCursorTree ? start & kCursorLeaf : 0;
       Box box = group_bounds<32>(p, n, st);
       box.lo.z = -1.0e30f;
       WarpWalk w;
       walk_begin(w, t, leaves, box.lo, box.hi, cursor);
       unsigned batch;
       int first, resume = leaves;
-      while (!done &&
-             walk_next(w, t, leaves, box.lo, box.hi, cursor, budget, batch, first, resume)) {
+      while (!done) {
+        if (!walk_next(w, t, leaves, box.lo, box.hi, cursor, budget, batch, first, resume)) {
+          if (resume >= leaves) break;
+          if (lane == 0) atomicAdd(&d.sc[kClipTurns], 1);
+          done = __shfl_sync(kFull, *(volatile int *)&d.status[kError], 0) != 0;
+          budget = turn;
+          cursor = resume;
+          walk_begin(w, t, leaves, box.lo, box.hi, cursor);  // with the box it has by now
+          continue;
+        }
         // Each lane's candidate of the batch.
         Occluder mine{nullptr, 0, -1};
         if ((batch >> lane) & 1u) {
@@ -675,10 +697,6 @@ __global__ void __launch_bounds__(kBlock, 4) k_clip_round(Dev d) {
           box = group_bounds<32>(p, n, st);
           box.lo.z = -1.0e30f;
         }
-      }
-      if (!done && resume < leaves) {  // the budget ran out first: to the queue's end
-        queue_piece(queue, p, n, target, (tree << kCursorTree) | resume);
-        done = true;
       }
     }
     if (done) {

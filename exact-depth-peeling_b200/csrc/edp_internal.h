@@ -163,7 +163,8 @@ enum Scalar : int {
   kTopLive = 38,
   kTopFirst = 39,
   kTopPushed = 40,
-  kScalarCount = 41  // k_reset clears them with its first threads
+  kClipTurns = 41,  // clipping: turns of walks under way, for the warps that wait
+  kScalarCount = 42  // k_reset clears them with its first threads
 };
 static_assert(kCandidates % 2 == 0, "a 64-bit counter");
 

@@ -330,10 +330,11 @@ cudaError_t allocate_event(edp_peeler *p) {
 cudaError_t allocate_device(edp_peeler *p) {
   Dev &d = p->d;
   const int64_t n = d.n, F = d.cap.frontier, R = d.cap.regions, E = d.cap.vertices;
-  // Live clipping pieces end as visible (at most R) or hidden pieces, so
-  // R + F slots hold every round's queue.  The hidden pool also holds the
-  // pieces of targets that end up hidden whole (dropped when the layer
-  // finishes), so it takes R + F slots too.
+  // The hidden pool also holds the pieces of targets that end up hidden whole
+  // (dropped when the layer finishes), so it takes R + F slots.  A layer's
+  // targets and queued parts each end as at least one visible piece (at most R)
+  // or one hidden piece, so two queues of R + F slots hold them all: a launch
+  // takes one, and what does not fit spills to the other for the next launch.
   d.work_cap = int(std::min<int64_t>(R + F, (int64_t(1) << 31) - 1));
   d.hidden_cap = d.work_cap;
   EDP_CHECK(allocate_shared(p));

@@ -9,7 +9,8 @@ rounds, blocks and warps, never which regions or triangles come out:
   width of the persistent subdivision grid);
 * ``heavy_noding_work``: candidate x edge tests above which a polygon is
   noded by a warp instead of eight lanes;
-* ``clip_budget``: DevicePeeler hierarchy walk steps per piece and clipping round.
+* ``clip_budget``: DevicePeeler hierarchy walk steps of a clipped piece between
+  two reports to the warps that wait for work.
 
 ``tune`` runs a coordinate search: starting from the defaults, each knob in
 turn takes each of its values with the others fixed, and the value with the

@@ -195,8 +195,9 @@ int edp_predicate_counts(edp_peeler *p, int64_t *counts);
  *   subdivide_blocks   subdivision: blocks of 4 warps per SM (default 8)
  *   heavy_noding_work  noding: candidate x edge tests above which a polygon
  *                      is noded by a warp instead of 8 lanes (default 1024)
- *   clip_budget        DevicePeeler: hierarchy walk steps per piece and
- *                      clipping round (default 32, at least 8) */
+ *   clip_budget        DevicePeeler: hierarchy walk steps of a clipped piece
+ *                      between two reports to the warps that wait for work
+ *                      (default 32, 8 to 1024) */
 typedef struct edp_tuning {
   int32_t step_budget, subdivide_blocks, heavy_noding_work, clip_budget;
 } edp_tuning;
