@@ -805,6 +805,13 @@ int edp_get_tuning(edp_peeler *p, edp_tuning *t) {
   return EDP_OK;
 }
 
+int edp_set_clip_queue(edp_peeler *p, int64_t slots) {
+  if (!p || p->method != 1 || slots < 0 || slots > p->d.hidden_cap) return EDP_ERR_ARGUMENT;
+  if (p->exec) return EDP_ERR_STATE;
+  p->d.work_cap = slots ? int(slots) : p->d.hidden_cap;
+  return EDP_OK;
+}
+
 int edp_predicate_counts(edp_peeler *p, int64_t *counts) {
   if (!p || !counts) return EDP_ERR_ARGUMENT;
   EDP_TRY(cudaStreamSynchronize(p->stream));

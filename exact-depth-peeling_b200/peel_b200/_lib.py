@@ -53,6 +53,7 @@ EXPORTS = (
     "edp_last_error_site", "edp_weld_noalloc", "edp_stage_times", "edp_set_predicates",
     "edp_predicate_counts", "edp_workspace_bytes", "edp_tile_features", "edp_mlp_infer",
     "edp_mlp_grad", "edp_adam_step", "edp_set_tuning", "edp_get_tuning",
+    "edp_set_clip_queue",
 )
 
 # enum edp_predicates and enum edp_predicate_class in include/edp.h.
@@ -106,6 +107,7 @@ def load():
     lib.edp_workspace_bytes.argtypes = [P, P]
     lib.edp_set_tuning.argtypes = [P, ctypes.POINTER(TuningC)]
     lib.edp_get_tuning.argtypes = [P, ctypes.POINTER(TuningC)]
+    lib.edp_set_clip_queue.argtypes = [P, I64]
     lib.edp_tile_features.argtypes = [P, I64, P, I64, P, P, P, P, P]
     lib.edp_mlp_infer.argtypes = [P, P, I64, P, P]
     lib.edp_mlp_grad.argtypes = [P, P, P, P, I64, ctypes.c_float, P, P, P]

@@ -203,6 +203,13 @@ typedef struct edp_tuning {
 } edp_tuning;
 int edp_set_tuning(edp_peeler *p, const edp_tuning *t);
 int edp_get_tuning(edp_peeler *p, edp_tuning *t);
+/* Limits a DevicePeeler's clipping queue to `slots` pieces, at most the
+ * polygons + residual that it was made for (0: all of them), for the next
+ * capture or warm-up; EDP_ERR_STATE once the workspace's own graph exists.
+ * Pieces past the queue's end wait for another launch of the layer, as many
+ * again at most.  No result depends on it; the tests use it to reach that
+ * path. */
+int edp_set_clip_queue(edp_peeler *p, int64_t slots);
 
 /* Stages timed by edp_stage_times, in extraction order: the reference
  * profiler's phases (scripts/profile_events.py:35-56) with its rank and mesh
