@@ -4,11 +4,10 @@
 // Each layer pass: sources whose whole-face rank is below the current layer
 // retire from the source hierarchy (a refit, no re-sort), the residual
 // hierarchy is rebuilt over the patches still unresolved, and a queue of
-// pieces is clipped round by round against every candidate that can be in
-// front of its target (below).  Pieces that stay visible are output for this
-// layer; hidden pieces form the next pass's residual.  The layer loop is the
-// graph's conditional WHILE node, the clipping rounds a WHILE node nested in
-// its body.
+// pieces is clipped against every candidate that can be in front of its target
+// (below).  Pieces that stay visible are output for this layer; hidden pieces
+// form the next pass's residual.  The layer loop is the graph's conditional
+// WHILE node, the clipping launches a WHILE node nested in its body.
 #include "../../include/edp.h"
 #include "edp_filtered.cuh"
 #include "edp_internal.h"

@@ -183,9 +183,9 @@ struct Dev {
   // and counted into pred_counts ([class][stage], edp_filtered.cuh).
   int predicates;
   unsigned long long *pred_counts;
-  // Tuning knobs (edp_tuning): subdivision walk steps per patch and round,
+  // Tuning knobs (edp_tuning): chunks of candidates per patch and round,
   // subdivision blocks per SM, candidate x edge tests above which a polygon
-  // is noded by a warp, clipping walk steps per piece and round.  None
+  // is noded by a warp, walk steps between a clipped piece's reports.  None
   // changes a result, only how the work is spread.
   int step_budget, subdivide_blocks, heavy_noding_work, clip_budget;
   Caps cap;
@@ -227,7 +227,7 @@ struct Dev {
   int seg_mask;
   Tree source_tree, seg_tree, point_tree;
   // Candidate lists of the subdivision: per source, its entries (segment,
-  // depth code) in leaf order, or a count of -1 where the pool had no room.
+  // depth code) in leaf order, or a count of -1 where there are too many.
   int2 *cand;
   int *cand_start, *cand_count;
   int64_t cand_cap;
@@ -336,7 +336,7 @@ struct Dev {
   int hidden_cap;
   int *target_visible, *target_hidden;
   long long *stats;                 // [layers][3]: targets, candidate tests, restored whole
-  int workers, pieces;              // clipping threads; pieces one target may hold
+  int workers, pieces;  // workers: kept for the interface; pieces one target may hold
   unsigned long long inner_handle;  // cudaGraphConditionalHandle of the clipping rounds
   int use_inner;
   // Host-side: a second stream of the workspace, on which conditional node
@@ -399,9 +399,8 @@ cudaError_t stage_segment_grid(const Dev &d, SortScratch &s, cudaStream_t st);
 cudaError_t stage_lists(const Dev &d, cudaStream_t st);
 cudaError_t stage_step(const Dev &d, cudaStream_t st);
 cudaError_t stage_rank(const Dev &d, SortScratch &s, cudaStream_t st);
-cudaError_t stage_mesh(const Dev &d, SortScratch &s, TreeBuffers &point_tree, cudaStream_t st);
-// The two halves of stage_mesh: boundary vertices and point hierarchy, then
-// the noding / emission / lifting kernel.
+// The mesh stage in two halves: boundary vertices and point hierarchy, then the
+// noding / emission / lifting kernels.
 cudaError_t stage_mesh_index(const Dev &d, SortScratch &s, TreeBuffers &point_tree,
                              cudaStream_t st);
 cudaError_t stage_mesh_emit(const Dev &d, cudaStream_t st);

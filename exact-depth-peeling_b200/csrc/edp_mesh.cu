@@ -1049,9 +1049,4 @@ cudaError_t stage_mesh_emit(const Dev &d, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t stage_mesh(const Dev &d, SortScratch &s, TreeBuffers &point_tree, cudaStream_t st) {
-  EDP_CHECK(stage_mesh_index(d, s, point_tree, st));
-  return stage_mesh_emit(d, st);
-}
-
 }  // namespace edp

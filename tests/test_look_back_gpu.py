@@ -27,3 +27,9 @@ def test_stack_over_tile_edges(n):
         sources = p.output_sources[:n].cpu().numpy()
         np.testing.assert_array_equal(layers, sources)
         np.testing.assert_array_equal(np.sort(layers), np.arange(n))
+
+
+@pytest.mark.parametrize("n", [1365, 1366, 4095, 4096, 4097])
+def test_stack_over_scan_tile_edges(n):
+    """A scan's tiles hold 4,096 elements (a radix pass's 2,048)."""
+    test_stack_over_tile_edges(n)

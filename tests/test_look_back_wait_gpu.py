@@ -33,7 +33,7 @@ def lib(tmp_path_factory):
 
 # Tiles: 4,096 elements of a scan, 2,048 keys of a radix pass.
 @pytest.mark.parametrize("missing,epoch", [(0, 0), (1, 0), (3, 0), (0, LAST_EPOCH)])
-@pytest.mark.parametrize("n", [4097, 8192, 100_001])
+@pytest.mark.parametrize("n", [4095, 4096, 4097, 8192, 100_001])
 def test_scan(lib, n, missing, epoch):
     values = np.random.default_rng(n).integers(0, 9, size=n).astype(np.int32)
     out, errors = np.zeros(n + 1, dtype=np.int32), np.zeros(2, dtype=np.int32)
