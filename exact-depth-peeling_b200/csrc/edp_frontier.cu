@@ -586,6 +586,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
   const int live = kWide ? parked + d.sc[kTopLive]
                          : int(min(int64_t(d.status[kResidual]), d.cap.frontier));
   int *taken = kWide ? &d.sc[kDeferredNext] : &d.sc[kFrontierNext];
+  const V2 *fv = d.fv[par];
+  const int *fn = d.fn[par], *fsrc = d.fsrc[par], *fcur = d.fcur[par];
   const Segments segs = segments_of(d);
   const Frontier next{d.fv[par ^ 1], d.fn[par ^ 1], d.fsrc[par ^ 1], d.fcur[par ^ 1],
                       &d.status[kNextResidual], d.status, d.cap.frontier - parked};
@@ -630,21 +632,23 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
       const int failed = __shfl_sync(kFull, *(volatile int *)&d.status[kError], 0);
       if (want && (at >= live || failed != 0)) drained = true;
       const bool take = want && !drained;
-      int from = par, i = at, size = 0;
+      int i = at, size = 0;
       if (kWide) {  // from the top downwards: the parked ones, then those without a list
-        if (at < parked)
-          from = par ^ 1;
-        else
-          i += d.sc[kTopFirst] - parked;
+        const int from = at < parked ? par ^ 1 : par;
+        if (at >= parked) i += d.sc[kTopFirst] - parked;
         i = int(d.cap.frontier) - 1 - i;
+        fv = d.fv[from];
+        fn = d.fn[from];
+        fsrc = d.fsrc[from];
+        fcur = d.fcur[from];
       }
       if (take) {
-        size = d.fn[from][i];
+        size = fn[i];
         n = size & kSizeMask;
         generation = size >> kSizeBits;
-        source = d.fsrc[from][i];
-        cursor = d.fcur[from][i];
-        p = g.lane < n ? d.fv[from][int64_t(kMaxVertices) * i + g.lane] : v2(0.0, 0.0);
+        source = fsrc[i];
+        cursor = fcur[i];
+        p = g.lane < n ? fv[int64_t(kMaxVertices) * i + g.lane] : v2(0.0, 0.0);
         sc = d.scores[source];
         start = d.cand_start[source];
         count = d.cand_count[source];
@@ -660,8 +664,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
               push_patch<W>(next, &d.sc[kDeferred], true, wide, p, size, source, cursor);
           if (to >= 0)
             for (int j = W + g.lane; j < n; j += W)
-              next.v[int64_t(kMaxVertices) * to + j] =
-                  d.fv[par][int64_t(kMaxVertices) * i + j];
+              next.v[int64_t(kMaxVertices) * to + j] = fv[int64_t(kMaxVertices) * i + j];
           fresh = fresh && !wide;
         }
       }
