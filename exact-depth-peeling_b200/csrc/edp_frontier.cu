@@ -556,7 +556,7 @@ constexpr int kFewCuts = 3;   // both, when there are fewer patches than groups
 //
 // Reading a list of any length from end to end for every patch took 109 ms for
 // 2,000 strips in front of one triangle, 53 for 10,000 tiles and 43 for a floor
-// behind 200,000 faces of primitives; the search takes 27, 17 and 23.  In the
+// behind 200,000 faces of primitives; the search takes 27, 15 and 20.  In the
 // first pass's loop, even only called from there, it costs the listed patches
 // 10 to 15%.
 //
