@@ -153,10 +153,10 @@ __device__ inline bool may_cut(const Segments &g, int c, const V2 *v, int n, con
 // final polygon as it is; any other joins the frontier.  A source with more
 // than kListMost entries or kScreenMost candidates, or whose list does not fit
 // the pool, is left without a list, and its patches search the hierarchy
-// themselves, in the second pass of each iteration.  A large triangle behind a fine mesh is such a
-// source: one warp would list its thousands of segments while the rest of the
-// GPU waits (1.5 ms for a floor behind the 65,536-face knot), and each of its
-// patches would look through all of them.
+// themselves, in the second pass of each iteration.  A large triangle behind a
+// fine mesh is such a source: one warp would list its thousands of segments
+// while the rest of the GPU waits (1.5 ms for a floor behind the 65,536-face
+// knot), and each of its patches would look through all of them.
 // Bound by the latency of the walk's 4 to 5 dependent steps: 8 blocks per SM
 // with the candidates screened together, against 6 with each leaf group's few
 // by themselves, took the preparation of the 720K primitives from 2.92 to 2.55
