@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_candidates(Dev d) {
       continue;
     }
     // The slots of both ends: at most n <= frontier capacity of them.
-    if (total == kUnlisted) slot = int(d.cap.frontier) - 1 - slot;
+    if (total == kUnlisted) slot = d.frontier_room - 1 - slot;
     if (lane < n) d.fv[0][int64_t(kMaxVertices) * slot + lane] = p;
     if (lane == 0) {
       d.fn[0][slot] = n;
@@ -495,7 +495,7 @@ __device__ inline void advance_round(const Dev &d) {
   const int peak = __ldcg(&d.status[kPeakResidual]), parity = __ldcg(d.parity);
   const long long parked = __ldcg(&d.metrics[kParkedPatches]);
   bool failed = __ldcg(&d.status[kError]) != 0;
-  if (int64_t(next) + deferred + pushed > d.cap.frontier) {
+  if (int64_t(next) + deferred + pushed > d.frontier_room) {
     set_error(d.status, kErrResidual);
     failed = true;
   }
@@ -582,15 +582,15 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
   V2 *left_part = s_parts[slot][0], *right_part = s_parts[slot][1];
   const int par = *d.parity;
   // Parked in this iteration: at the next frontier's top.
-  const int parked = kWide ? int(min(int64_t(d.sc[kDeferred]), d.cap.frontier)) : 0;
+  const int parked = kWide ? int(min(int64_t(d.sc[kDeferred]), int64_t(d.frontier_room))) : 0;
   const int live = kWide ? parked + d.sc[kTopLive]
-                         : int(min(int64_t(d.status[kResidual]), d.cap.frontier));
+                         : int(min(int64_t(d.status[kResidual]), int64_t(d.frontier_room)));
   int *taken = kWide ? &d.sc[kDeferredNext] : &d.sc[kFrontierNext];
   const V2 *fv = d.fv[par];
   const int *fn = d.fn[par], *fsrc = d.fsrc[par], *fcur = d.fcur[par];
   const Segments segs = segments_of(d);
   const Frontier next{d.fv[par ^ 1], d.fn[par ^ 1], d.fsrc[par ^ 1], d.fcur[par ^ 1],
-                      &d.status[kNextResidual], d.status, d.cap.frontier - parked};
+                      &d.status[kNextResidual], d.status, int64_t(d.frontier_room) - parked};
   int visits = 0, tests = 0, splits = 0;  // each group's lane 0
   CutTally tally;
   // With fewer patches than groups the round lasts as long as one group's chain.
@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_subdivide(Dev d) {
       if (kWide) {  // from the top downwards: the parked ones, then those without a list
         const int from = at < parked ? par ^ 1 : par;
         if (at >= parked) i += d.sc[kTopFirst] - parked;
-        i = int(d.cap.frontier) - 1 - i;
+        i = d.frontier_room - 1 - i;
         fv = d.fv[from];
         fn = d.fn[from];
         fsrc = d.fsrc[from];

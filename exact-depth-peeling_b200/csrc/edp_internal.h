@@ -231,7 +231,9 @@ struct Dev {
   int2 *cand;
   int *cand_start, *cand_count;
   int64_t cand_cap;
-  // frontier ping-pong; fn holds the vertex count and the generation
+  // frontier ping-pong, `frontier_room` slots each; fn holds the vertex count
+  // and the generation
+  int frontier_room;
   V2 *fv[2];
   int *fn[2], *fsrc[2], *fcur[2];
   // output polygons

@@ -97,3 +97,24 @@ def icospheres():
     return (np.concatenate([outer, inner]),
             np.concatenate([f, f + len(v)]).astype(np.int32), np.diag([1.0, 1.0, -1.0, 1.0]),
             np.array([-1.3, -1.3, 1.3, 1.3, 0.0, 0.01]))
+
+
+@pytest.mark.parametrize("form", ["filtered64", "binary64"])
+def test_the_frontier_has_room_beside_a_generation(form):
+    """The capacity is for a generation of right-hand parts; the patches that an
+    iteration holds besides have room of their own."""
+    from peel_b200 import EventCapacities, EventPeeler, scenes
+
+    arrays = scenes.knot_tube(117, 60, seed=5)
+    device = scenes.to_device(arrays)
+    wide = EventCapacities.for_mesh(8 * len(arrays[1]))
+    p = EventPeeler(*device, capacities=wide, predicates=form)
+    p.run()
+    info = p.read_status()
+    frontier = max(len(arrays[1]), int(info["peak_residual_patches"] / 1.2))
+    assert frontier < info["peak_residual_patches"]
+    q = EventPeeler(*device, capacities=replace(wide, frontier=frontier), predicates=form)
+    q.run()
+    again = q.read_status()
+    assert {k: again[k] for k in ("polygons", "layers", "rounds", "splits")} == \
+        {k: info[k] for k in ("polygons", "layers", "rounds", "splits")}
