@@ -188,3 +188,54 @@ def test_a_frontier_of_the_sources_suffices(side, form):
     covered = sum(areas[(0, s)] for s in range(n - 1))
     assert abs(areas[(1, n - 1)] - covered) <= 1e-9
     assert abs(areas[(0, n - 1)] + covered - 1.0) <= 1e-9
+
+
+@pytest.mark.parametrize("form", ["filtered64", "binary64"])
+@pytest.mark.parametrize("count", [127, 128, 129])
+def test_lists_at_their_longest(count, form):
+    """A sheet behind ``count`` tiles, three segments each, where a list holds
+    384 of them."""
+    from peel_b200 import EventCapacities, EventPeeler, scenes
+
+    v, f, camera, settings = tiles_over_sheets(12, 1)
+    v = np.concatenate([v[:3 * count], v[-3:]])
+    f = np.arange(len(v), dtype=np.int32).reshape(-1, 3)
+    p = EventPeeler(*scenes.to_device((v, f, camera, settings)), predicates=form,
+                    capacities=replace(EventCapacities.for_mesh(32 * len(f)), layers=8))
+    p.run()
+    assert p.read_status()["unique_contours"] >= 3 * count
+    areas = parity.gpu_areas(parity.polygons(p), range(len(f)))
+    covered = sum(areas[(0, s)] for s in range(count))
+    assert abs(areas[(1, count)] - covered) <= 1e-9
+    assert abs(areas[(0, count)] + covered - 1.0) <= 1e-9
+
+
+@pytest.mark.parametrize("form", ["filtered64", "binary64"])
+@pytest.mark.parametrize("gap", [0.5, -0.5])
+def test_many_candidates(gap, form):
+    """A slanted sheet half a unit in front of (or behind) 1,600 tiles of its
+    own slant: every tile's edges are candidates of the sheet, none (or all) of
+    which cut it."""
+    from peel_b200 import EventCapacities, EventPeeler, scenes
+
+    side = 40
+    v, f, camera, settings = tiles_over_sheets(side, 1)
+    v[:, 2] = 10.0 + 4.0 * v[:, 0]
+    v[:-3, 2] += gap
+    n = len(f)
+    p = EventPeeler(*scenes.to_device((v, f, camera, settings)), predicates=form,
+                    capacities=replace(EventCapacities.for_mesh(32 * n), layers=8))
+    p.run()
+    assert p.read_status()["layers"] == 2
+    areas = parity.gpu_areas(parity.polygons(p), range(n))
+    tiles, sheet = (1, 0) if gap > 0.0 else (0, 1)
+    covered = sum(areas[(tiles, s)] for s in range(n - 1))
+    if gap > 0.0:
+        assert len(areas) == n and abs(areas[(0, n - 1)] - 1.0) <= 1e-9
+    else:
+        assert abs(areas[(sheet, n - 1)] - covered) <= 1e-9
+        assert abs(areas[(0, n - 1)] + covered - 1.0) <= 1e-9
+    corners = v[f][:, :, :2] * 0.5
+    u, w = corners[:, 1] - corners[:, 0], corners[:, 2] - corners[:, 0]
+    whole = 0.5 * (u[:, 0] * w[:, 1] - u[:, 1] * w[:, 0])[:-1]
+    assert abs(covered - whole.sum()) <= 1e-9
