@@ -200,6 +200,7 @@ struct Dev {
   // welding
   int *canonical, *weld_table, *weld_min, *weld_slot;
   int weld_mask;
+  int frontier_room;  // slots of the frontier's arrays (below)
   // projected sources, at most kSourceVertices vertices each
   V2 *src_v;
   int *src_n;
@@ -233,7 +234,6 @@ struct Dev {
   int64_t cand_cap;
   // frontier ping-pong, `frontier_room` slots each; fn holds the vertex count
   // and the generation
-  int frontier_room;
   V2 *fv[2];
   int *fn[2], *fsrc[2], *fcur[2];
   // output polygons
